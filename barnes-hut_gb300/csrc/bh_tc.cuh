@@ -38,10 +38,22 @@ __device__ __forceinline__ uint64_t kdesc(uint32_t saddr, int kc, int j) {
     return sdesc(saddr + 256u * (uint32_t)j, 128u, 128u * (uint32_t)kc);
 }
 
+// descriptor of K-step j of the same tile used as its transpose: the tile's rows are the K
+// dimension (16 of them a step) and its columns the M or N dimension (MN-major, no swizzle: the
+// leading-dimension offset leads to the next 8 rows, the stride offset to the next 8 columns)
+__device__ __forceinline__ uint64_t tdesc(uint32_t saddr, int kc, int j) {
+    return sdesc(saddr + 256u * (uint32_t)(kc * j), 128u * (uint32_t)kc, 128u);
+}
+
 // instruction descriptor, kind::f16: BF16 A and B (K-major), FP32 D, shape M x N
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
            ((uint32_t)(M >> 4) << 24);
+}
+
+// the same with both operands MN-major (the transposes of K-major tiles, tdesc)
+__host__ __device__ constexpr uint32_t idesc_bf16_t(int M, int N) {
+    return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t ncols) {
@@ -134,6 +146,13 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float *v) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+// the same for two columns
+__device__ __forceinline__ void ld2(uint32_t taddr, float *v) {
+    uint32_t r[2];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
+    v[0] = __uint_as_float(r[0]);
+    v[1] = __uint_as_float(r[1]);
+}
 __device__ __forceinline__ void ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -146,14 +165,11 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 constexpr float GELU_C0 = 0.7978845608028654f;  // sqrt(2 / pi)
 constexpr float GELU_C1 = 0.044715f;
-__device__ __forceinline__ float gelu(float x) {
-    float t = tanh_approx(GELU_C0 * (x + GELU_C1 * x * x * x));
+// gelu(x), and its derivative in g
+__device__ __forceinline__ float gelu_and_grad(float x, float &g) {
+    const float t = tanh_approx(GELU_C0 * (x + GELU_C1 * x * x * x));
+    g = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * GELU_C0 * (1.f + 3.f * GELU_C1 * x * x);
     return 0.5f * x * (1.f + t);
-}
-__device__ __forceinline__ float gelu_grad(float x) {
-    float u = GELU_C0 * (x + GELU_C1 * x * x * x);
-    float t = tanh_approx(u);
-    return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * GELU_C0 * (1.f + 3.f * GELU_C1 * x * x);
 }
 
 }  // namespace tc
