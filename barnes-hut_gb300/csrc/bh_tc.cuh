@@ -165,6 +165,10 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 constexpr float GELU_C0 = 0.7978845608028654f;  // sqrt(2 / pi)
 constexpr float GELU_C1 = 0.044715f;
+__device__ __forceinline__ float gelu(float x) {
+    float t = tanh_approx(GELU_C0 * (x + GELU_C1 * x * x * x));
+    return 0.5f * x * (1.f + t);
+}
 // gelu(x), and its derivative in g
 __device__ __forceinline__ float gelu_and_grad(float x, float &g) {
     const float t = tanh_approx(GELU_C0 * (x + GELU_C1 * x * x * x));
