@@ -205,7 +205,7 @@ extern "C" int bh_plan_create(bh_plan **out, int nsys, const long long *n, const
     for (int s = 0; s < nsys; s++) maxG = std::max(maxG, p->sys[s].G);
     p->stream = !flat && pr.precision != BH_PREC_FP64 && pr.cutoff_r2 == 0.0 && pr.softening > 0.0 &&
                 !(pr.flags & BH_FLAG_WALK) && maxG <= LIST_MAX_G;
-    p->chunk = p->stream ? STREAM_CHUNK : TARGET_CHUNK;
+    p->chunk = p->stream ? STREAM_CHUNK : pr.precision == BH_PREC_FP64 ? TARGET_CHUNK64 : TARGET_CHUNK;
     if (pr.dense_min < 0) return bad("dense_min < 0");
     p->dense_min = pr.dense_min > 0 ? pr.dense_min : BH_STREAM_DENSE_MIN;
     p->quad_min = pr.quad_min > 0 ? pr.quad_min : (pr.quad_min == 0 ? BH_STREAM_QUAD_MIN : 0);
@@ -731,7 +731,8 @@ extern "C" int bh_direct_sample(bh_plan *p, int sys, const long long *targets, l
     if (r) return r;
     if (sys < 0 || sys >= p->nsys) return fail(p, BH_ERR_INVALID, "system %d out of range", sys);
     if (nt < 0 || (nt > 0 && (!targets || !ax || !ay))) return fail(p, BH_ERR_INVALID, "bad targets");
-    CK(p, launch_direct(p->dev, sys, targets, nt, ax, ay, (cudaStream_t)stream), "direct sample");
+    CK(p, launch_direct(p->dev, sys, p->sys[sys].poff, p->sys[sys].n, targets, nt, ax, ay, (cudaStream_t)stream),
+       "direct sample");
     return BH_OK;
 }
 

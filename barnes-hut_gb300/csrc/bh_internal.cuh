@@ -39,6 +39,10 @@ constexpr int MAX_LEVELS = 16;  // G <= 32768
 constexpr int FORCE_THREADS = 128;
 constexpr int FORCE_R = 4;                                   // targets per thread (FP32)
 constexpr int TARGET_CHUNK = FORCE_THREADS * FORCE_R;        // targets per work item
+// FP64 pairs cost 16 FP32 ones or more, so their items are small: a CTA's share of the FP64 pipe
+// turns an item of 512 targets of a dense box into tens of milliseconds (65,536 clustered particles
+// on 32 x 32 boxes, the step: 512 targets 32.9 ms, 64: 8.1, 32: 7.1, 16: 6.6)
+constexpr int TARGET_CHUNK64 = 16;
 constexpr int FRONTIER_CAP = 512;                            // traversal frontier per level
 constexpr int SCAN_TILE = 4096;   // counts per tile of the single-pass scans (256 threads x 16)
 constexpr int MAX_TG = 8;          // largest target group (boxes per side)
@@ -152,7 +156,7 @@ struct DevPlan {
     int nsm;     // streaming multiprocessors of the plan's device (queried at bh_bind): sizes the
                  // persistent and grid-stride launches
     int stream;  // 1: lists are built by k_lists and streamed by k_fstream
-    int chunk;   // targets per work item (TARGET_CHUNK, or STREAM_CHUNK when stream)
+    int chunk;   // targets per work item (TARGET_CHUNK, TARGET_CHUNK64, or STREAM_CHUNK when stream)
     // parameters
     double gconst, dt, eps2, cutoff;
     float theta2_f, eps2_f, cut_f;
@@ -384,8 +388,8 @@ cudaError_t launch_load(const DevPlan &d, const double *x, const double *y, cons
                         cudaStream_t st);
 cudaError_t launch_store(const DevPlan &d, int has_tree, bool has_acc, double *rec, double *x, double *y, double *vx,
                          double *vy, double *ax, double *ay, cudaStream_t st);
-cudaError_t launch_direct(const DevPlan &d, int sys, const long long *targets, long long nt,
-                          double *ax, double *ay, cudaStream_t st);
+cudaError_t launch_direct(const DevPlan &d, int sys, long long poff, long long n, const long long *targets,
+                          long long nt, double *ax, double *ay, cudaStream_t st);
 cudaError_t launch_diag(const DevPlan &d, int sys, int want_pot, double *out, cudaStream_t st);
 cudaError_t launch_box_com(const DevPlan &d, int sys, double *out, cudaStream_t st);
 // record a failure of a call without a plan (read by bh_last_error(NULL)); returns code

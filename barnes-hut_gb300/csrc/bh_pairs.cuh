@@ -17,6 +17,20 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
+// 1 / x in FP64: the hardware's approximation and one step of the cubic iteration y + y (e + e^2),
+// e = 1 - x y (Householder's method of order 2), 3 FP64 operations; the last is a fused one, so the
+// result is within rounding of the quotient.  Arguments near the ends of the exponent range, zeros,
+// infinities and NaN take the division.
+__device__ __forceinline__ double rcp64(double x) {
+    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+    if (e - 24u > 2000u) return 1.0 / x;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double r = __fma_rn(-x, y, 1.0);
+    r = __fma_rn(r, r, r);
+    return __fma_rn(y, r, y);
+}
+
 // Packed FP32 pairs (sm_100-family f32x2 instructions): two lanes of work per instruction.
 typedef unsigned long long f2_t;
 __device__ __forceinline__ f2_t f2_pack(float a, float b) {

@@ -74,7 +74,7 @@ def test_network_gradient_rows_and_alignment(n, width, shift):
 # walk): the same groups, so the same band cells and the same network outputs in another tiling.
 # Its sums are FP32 (2^-24 relative a term, some hundred terms) and are read off as the difference
 # of two accelerations some ten times larger: 1e-4 relative RMS.
-@pytest.mark.parametrize("n,grid,group", [(700, 8, 2), (5003, 16, 4), (20011, 24, 8)])
+@pytest.mark.parametrize("n,grid,group", [(700, 8, 2), (5003, 16, 4), (20011, 24, 8), (20011, 64, 2), (60011, 64, 2)])
 def test_learned_correction_item_sizes(n, grid, group):
     from barneshut.gb300 import learned, native, workloads
 
@@ -100,3 +100,82 @@ def test_learned_correction_item_sizes(n, grid, group):
         corr.append(acc[1] - acc[0])
     assert np.abs(corr[0]).max() > 0
     assert rel_rms(corr[0], corr[1]) < 1e-4
+
+
+# FP64 sums of at most 1e5 terms: 1e-16 a rounding, far below 1e-12.  Tiles of 4 to 64 targets, one
+# chunk and many, a target count over the scratch, softened and not.
+@pytest.mark.parametrize("n,nt,eps", [(1, 1, 0.1), (5, 5, 0.0), (1000, 3, 1e-4), (1000, 1000, 0.0), (4099, 65, 1e-2),
+                                      (100003, 1, 1e-4), (30011, 700, 0.0)])
+def test_direct_sample_tiles_and_chunks(n, nt, eps):
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(n + nt)
+    x, y, vx, vy = rng.random((4, n))
+    m = 1.0 + rng.random(n)
+    plan = native.Plan([n], [4], native.make_params(0.7, 1e-5, eps, 0.0, 0.5))
+    plan.load(x, y, m, vx, vy)
+    plan.step(1)
+    state = {k: v.cpu().numpy() for k, v in plan.store().items()}
+    x, y = state["x"], state["y"]
+    t = rng.choice(n, nt, replace=False)
+    ax, ay = plan.direct_sample(t)
+    rx, ry = np.empty(nt), np.empty(nt)
+    for k, i in enumerate(t):
+        dx, dy = np.delete(x, i) - x[i], np.delete(y, i) - y[i]
+        w = np.delete(m, i) / (dx * dx + dy * dy + eps * eps)
+        rx[k], ry[k] = 0.7 * np.sum(w * dx), 0.7 * np.sum(w * dy)
+    got, ref = np.concatenate([ax.cpu().numpy(), ay.cpu().numpy()]), np.concatenate([rx, ry])
+    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
+    after = plan.store()  # the sampler leaves the state alone
+    assert all(np.array_equal(after[k].cpu().numpy(), state[k]) for k in state)
+
+
+def test_direct_sample_of_a_system_in_a_batch():
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(5)
+    n = [300, 2000]
+    x, y, v = rng.random((3, 2300))
+    m = 1.0 + rng.random(2300)
+    plan = native.Plan(n, [2, 4], native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5))
+    plan.load(x, y, m, v, v)
+    alone = native.Plan([2000], [4], native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5))
+    alone.load(x[300:], y[300:], m[300:], v[300:], v[300:])
+    t = np.array([300, 1234, 2299, 299, 0])
+    ax, _ = plan.direct_sample(t, sys=1)
+    bx, _ = alone.direct_sample(t[:3] - 300)
+    assert torch.allclose(ax[:3], bx, rtol=1e-12, atol=0)
+    assert torch.isnan(ax[3:]).all()  # not particles of the system
+
+
+# The walking force kernel with one CTA per item (a batch whose items fill the chip) and with two (a
+# system alone): the same sums.  Leaf sums differ by their chunk offsets (1e-7 of a box edge), so
+# accelerations agree within 1e-5 relative RMS, the oracle tests' own bound.
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("cutoff,eps", [(0.0, 0.0), (1e-5, 0.0), (1e-5, 1e-3), (0.0, 1e-3)])
+def test_walk_items_one_or_two_ctas(prec, cutoff, eps):
+    from barneshut.gb300 import native, workloads
+
+    sizes, grids = [1, 3, 700, 2049, 5000, 9000, 1500, 4000, 6001], [1, 2, 2, 3, 4, 8, 16, 16, 12]
+    systems = [workloads.uniform(n, seed=n) for n in sizes]
+    prm = native.make_params(1.0, 1e-5, eps, cutoff, 0.0, 1, prec)
+
+    def accel(n, g, cols):
+        plan = native.Plan(n, g, prm)
+        plan.load(*cols)
+        plan.create_tree()
+        plan.summarize()
+        plan.evaluate()
+        out = plan.store()
+        assert plan.error_flags() == 0
+        return torch.stack([out["ax"], out["ay"]]).cpu().numpy(), plan.pair_counts()
+
+    big, pairs = accel(sizes, grids, [np.concatenate([s[k] for s in systems]) for k in range(5)])
+    o, near, far = 0, 0, 0
+    for s, n, g in zip(systems, sizes, grids):
+        one, (a, b) = accel([n], [g], s)
+        near, far = near + a, far + b
+        if n > 1:
+            assert rel_rms(big[:, o:o + n], one) < 1e-5
+        o += n
+    assert pairs == (near, far)
