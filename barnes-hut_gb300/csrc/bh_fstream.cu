@@ -29,6 +29,8 @@
 #include "bh_pairs.cuh"
 #include "bh_tc.cuh"
 
+#include <type_traits>
+
 namespace bh {
 
 constexpr int NR = FORCE_R;
@@ -65,8 +67,44 @@ struct FsLayout {
     static_assert(WFAR % 32 == 0, "far staging passes are whole lane rounds");
 };
 static_assert(32 * NR >= STREAM_CHUNK, "a warp must cover every target of a work item");
+static_assert(ITEM_BUCKETS == 32, "a lane per cost bucket");
+constexpr float SPLIT4 = 512.f, SPLIT2 = 1024.f;  // an item of more than 1 / SPLIT of the whole cost is split
+constexpr int SPLIT4_BUCKET = 18;  // in four only from 2,048 sources of a full item on
 
-template <bool KAHAN, int MINB>
+// One pair: (ax, ay) += m (x - xt, y - yt) / (r^2 + eps2), in the rounding steps of the packed sweeps.
+__device__ __forceinline__ void pair1(float x, float y, float m, float ntx, float nty, float eps2, float &ax, float &ay) {
+    const float dx = __fadd_rn(x, ntx), dy = __fadd_rn(y, nty);
+    const float w = __fmul_rn(m, rcp_approx(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, eps2))));
+    ax = __fmaf_rn(w, dx, ax);
+    ay = __fmaf_rn(w, dy, ay);
+}
+
+// (float)k for |k| < 2^22 by an exact addition: the conversion instruction runs on the reciprocals'
+// pipe, which bounds the sweeps.
+__device__ __forceinline__ float small_int_f(int k) { return __fsub_rn(__int_as_float(0x4B400000 + k), 12582912.f); }
+
+// How many of the heaviest items run as four warps' work (.x) and how many of the next as two (.y),
+// from the cost histogram (bucket b: costs in [2^b, 2^(b+1))).  A warp alone takes about 70 cycles
+// per source of a full item where a busy scheduler takes 40, so an item of more than 1/1,000 of the
+// whole cost outlasts everything else on 608 schedulers; a part of it holds half or a quarter of the
+// targets of every quad, with the same slices and order of sources (the same bits), and sweeps with
+// that much less work and more sources in flight.  The parts repeat the item's staging, so items
+// below the line stay whole.
+__device__ __forceinline__ int2 stream_split(const int *hist) {
+    const int lane = threadIdx.x & 31;
+    const int h = hist[lane];  // ITEM_BUCKETS == 32
+    float w = h > 0 ? (float)h * ldexpf(1.5f, lane) : 0.f;
+    const float c = ldexpf(1.5f, lane);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    const bool four = c * SPLIT4 > w && lane >= SPLIT4_BUCKET;
+    int n4 = four ? h : 0, n2 = !four && c * SPLIT2 > w ? h : 0;
+    n4 = __reduce_add_sync(0xffffffffu, n4);
+    n2 = __reduce_add_sync(0xffffffffu, n2);
+    return make_int2(n4, n2);
+}
+
+template <bool KAHAN, int MINB, bool SPLIT>
 __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, int accumulate) {
     extern __shared__ __align__(128) unsigned char smem[];
     using Ly = FsLayout<MINB>;
@@ -98,19 +136,39 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
     }
     __syncwarp();
 
+    // The queue: items in cost order, heaviest first; the first n4 of them are four entries each,
+    // the next n2 two (stream_split), each entry a part of the item's targets.
+    const int2 split = SPLIT ? stream_split(d.item_bucket) : make_int2(0, 0);
+    const long long nentry = nitems + 3LL * split.x + split.y;
     // lane 0 takes the queue slot of its next item one item ahead (the atomic's latency hides
     // behind the current item)
     int qnext = 0;
     if (lane == 0) qnext = (int)atomicAdd(&d.glob->item_next, 1u);
     for (;;) {
-        int item = 0;
+        int item = -1, part = 0;  // part: 4 np + the part's first target within a quad
         if (lane == 0) {
-            const int q = qnext;
-            item = q < nitems ? d.item_order[q] : q;  // heaviest items first
-            if (q < nitems) qnext = (int)atomicAdd(&d.glob->item_next, 1u);
+            int q = qnext;
+            if (q < nentry) {
+                qnext = (int)atomicAdd(&d.glob->item_next, 1u);
+                if (!SPLIT) {
+                } else if (q < 4 * split.x) {
+                    part = 4 + (q & 3);
+                    q >>= 2;
+                } else if (q < 4 * split.x + 2 * split.y) {
+                    q -= 4 * split.x;
+                    part = 8 + 2 * (q & 1);
+                    q = split.x + (q >> 1);
+                } else {
+                    part = 16;
+                    q -= 3 * split.x + split.y;
+                }
+                item = d.item_order[q];  // heaviest items first
+            }
         }
         item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= nitems) break;
+        if (SPLIT) part = __shfl_sync(0xffffffffu, part, 0);
+        if (item < 0) break;
+        const int np = SPLIT ? part >> 2 : NR, r0 = SPLIT ? part & 3 : 0;  // targets per lane: r0 .. r0 + np - 1 of its quad
         const long long g = d.sitem_group[item];
         const int sub = d.sitem_sub[item];  // box within the group, or -1: the sparse boxes
         const int2 ck = d.sitem_chunk[item];
@@ -188,15 +246,17 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
         const float step_f = __double2float_rn(dy.step);
         const float eps2 = d.eps2_f;
 
-        // ---- lane -> (slice, NR targets)
+        // ---- lane -> (slice, quad of targets); the lane sums the slice for np targets of the quad
         const int nthr = (T + NR - 1) / NR;
         const int nslice = 32 / nthr;
         const bool active = lane < nslice * nthr;
         const int slice = active ? lane / nthr : 0, tl = active ? lane % nthr : 0;
+        auto run = [&](auto npc) {
+        constexpr int NP = decltype(npc)::value, NQ = NP > 1 ? NP / 2 : 1;  // targets, packed pairs
         // sorted index of the lane's target r (recomputed in the epilogue rather than kept live)
         // (the run is the target's box within the group, column-major)
         auto target_index = [&](int r, int &run) {
-            const int v = tl * NR + r;
+            const int v = tl * NR + r0 + r;
             const int u = c0 + (v < T ? v : 0);
             int lo = 0, hi = nrun;  // the run r with rpre[r] <= u < rpre[r + 1]
             while (hi - lo > 1) {
@@ -206,9 +266,9 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
             run = lo;
             return rstart[lo] + (u - rpre[lo]);
         };
-        float tx[NR], ty[NR];
+        float tx[NP], ty[NP];
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
+        for (int r = 0; r < NP; r++) {
             int run;
             const int ti = target_index(r, run);
             const float4 p = d.PD[2 * (long long)ti];  // (x, x, y, y) box-relative
@@ -216,18 +276,19 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
             ty[r] = __fadd_rn(__fmul_rn((float)(run & (TG - 1)), step_f), p.z);
         }
         // negated target coordinates, near accumulators, far sums and compensations, in pairs
-        f2_t ntx2[NR / 2], nty2[NR / 2], nax2[NR / 2], nay2[NR / 2];
-        f2_t fsx2[NR / 2], fsy2[NR / 2], fcx2[NR / 2], fcy2[NR / 2];
+        f2_t ntx2[NQ], nty2[NQ], nax2[NQ], nay2[NQ];
+        f2_t fsx2[NQ], fsy2[NQ], fcx2[NQ], fcy2[NQ];
         const f2_t eps2x2 = f2_pack(eps2, eps2);
         const f2_t m1x2 = f2_pack(-1.f, -1.f);
 #pragma unroll
-        for (int k = 0; k < NR / 2; k++) {
-            ntx2[k] = f2_pack(-tx[2 * k], -tx[2 * k + 1]);
-            nty2[k] = f2_pack(-ty[2 * k], -ty[2 * k + 1]);
+        for (int k = 0; k < NQ; k++) {
+            ntx2[k] = f2_pack(-tx[2 * k], -tx[NP > 1 ? 2 * k + 1 : 0]);
+            nty2[k] = f2_pack(-ty[2 * k], -ty[NP > 1 ? 2 * k + 1 : 0]);
             nax2[k] = nay2[k] = f2_pack(0.f, 0.f);
             fsx2[k] = fsy2[k] = fcx2[k] = fcy2[k] = f2_pack(0.f, 0.f);
         }
         const int4 *ln = d.lnear + sd.lnoff + lg * 2 * (sd.lncap + 1);
+        int nfs = 0, nns = 0;  // far entries and near sources swept
 
         // sweep nf staged far entries; the pass's plain FP32 sum enters the far total through a
         // Kahan-compensated addition (compensate: the group's far list), or the near accumulators
@@ -236,23 +297,35 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
             if (active) {
                 const ulonglong2 *fp = reinterpret_cast<const ulonglong2 *>(farxy);
                 const f2_t *fm = reinterpret_cast<const f2_t *>(farm);
-                f2_t px2[NR / 2], py2[NR / 2];
+                f2_t px2[NQ], py2[NQ];
 #pragma unroll
-                for (int kk = 0; kk < NR / 2; kk++) px2[kk] = py2[kk] = f2_pack(0.f, 0.f);
-#pragma unroll 4
-                for (int k = slice; k < nf; k += nslice) {
-                    const ulonglong2 rxy = fp[k];  // (rx, rx), (ry, ry)
-                    const f2_t mm = fm[k];         // (M, M)
+                for (int kk = 0; kk < NQ; kk++) px2[kk] = py2[kk] = f2_pack(0.f, 0.f);
+                if constexpr (NP > 1) {
+#pragma unroll 16 / NP
+                    for (int k = slice; k < nf; k += nslice) {
+                        const ulonglong2 rxy = fp[k];  // (rx, rx), (ry, ry)
+                        const f2_t mm = fm[k];         // (M, M)
 #pragma unroll
-                    for (int kk = 0; kk < NR / 2; kk++) {
-                        const f2_t dx = f2_add(rxy.x, ntx2[kk]), dyy = f2_add(rxy.y, nty2[kk]);
-                        const f2_t w = f2_mul(mm, f2_rcp(f2_fma(dx, dx, f2_fma(dyy, dyy, eps2x2))));
-                        px2[kk] = f2_fma(w, dx, px2[kk]);
-                        py2[kk] = f2_fma(w, dyy, py2[kk]);
+                        for (int kk = 0; kk < NQ; kk++) {
+                            const f2_t dx = f2_add(rxy.x, ntx2[kk]), dyy = f2_add(rxy.y, nty2[kk]);
+                            const f2_t w = f2_mul(mm, f2_rcp(f2_fma(dx, dx, f2_fma(dyy, dyy, eps2x2))));
+                            px2[kk] = f2_fma(w, dx, px2[kk]);
+                            py2[kk] = f2_fma(w, dyy, py2[kk]);
+                        }
                     }
+                } else {
+                    float px = 0.f, py = 0.f;
+                    const float ntx = -tx[0], nty = -ty[0];
+#pragma unroll 8
+                    for (int k = slice; k < nf; k += nslice) {
+                        const float4 e = farxy[k];
+                        pair1(e.x, e.z, farm[k].x, ntx, nty, eps2, px, py);
+                    }
+                    px2[0] = f2_pack(px, px);
+                    py2[0] = f2_pack(py, py);
                 }
 #pragma unroll
-                for (int kk = 0; kk < NR / 2; kk++) {
+                for (int kk = 0; kk < NQ; kk++) {
                     if (KAHAN && compensate) {  // y = f - c; t = s + y; c = (t - s) - y; s = t
                         const f2_t yx = f2_fma(fcx2[kk], m1x2, px2[kk]), t1 = f2_add(fsx2[kk], yx);
                         fcx2[kk] = f2_fma(yx, m1x2, f2_fma(fsx2[kk], m1x2, t1));
@@ -269,7 +342,7 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
                     }
                 }
             }
-            if (lane == 0) wcnt[1] += (unsigned long long)T * nf;
+            nfs += nf;
             __syncwarp();  // the staging is rewritten next
         };
 
@@ -306,7 +379,7 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
         // the compensated far sums s - c start the near accumulators; the far sums and their
         // compensations are dead from here on
 #pragma unroll
-        for (int kk = 0; kk < NR / 2; kk++) {
+        for (int kk = 0; kk < NQ; kk++) {
             nax2[kk] = f2_fma(fcx2[kk], m1x2, fsx2[kk]);
             nay2[kk] = f2_fma(fcy2[kk], m1x2, fsy2[kk]);
         }
@@ -474,8 +547,8 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
                 for (int j = lane; j < ns; j += 32) {
                     float4 v = s4[2 * j];
                     const int code = __float_as_int(s4[2 * j + 1].w);
-                    const float shx = __fmul_rn((float)((code >> 16) - gx0), step_f);
-                    const float shy = __fmul_rn((float)((code & 0xffff) - gy0), step_f);
+                    const float shx = __fmul_rn(small_int_f((code >> 16) - gx0), step_f);
+                    const float shy = __fmul_rn(small_int_f((code & 0xffff) - gy0), step_f);
                     v.x = __fadd_rn(shx, v.x);
                     v.y = v.x;
                     v.z = __fadd_rn(shy, v.z);
@@ -484,21 +557,35 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
                 }
                 __syncwarp();
                 if (active) {
-#pragma unroll 4
-                    for (int j = slice; j < ns; j += nslice) {
-                        const ulonglong2 sxy = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j);
-                        const f2_t mm = *reinterpret_cast<const f2_t *>(s4 + 2 * j + 1);
+                    if constexpr (NP > 1) {
+#pragma unroll 16 / NP
+                        for (int j = slice; j < ns; j += nslice) {
+                            const ulonglong2 sxy = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j);
+                            const f2_t mm = *reinterpret_cast<const f2_t *>(s4 + 2 * j + 1);
 #pragma unroll
-                        for (int kk = 0; kk < NR / 2; kk++) {
-                            const f2_t dx = f2_add(sxy.x, ntx2[kk]), dyy = f2_add(sxy.y, nty2[kk]);
-                            const f2_t r2 = f2_fma(dx, dx, f2_fma(dyy, dyy, eps2x2));
-                            const f2_t w = f2_mul(mm, f2_rcp(r2));
-                            nax2[kk] = f2_fma(w, dx, nax2[kk]);
-                            nay2[kk] = f2_fma(w, dyy, nay2[kk]);
+                            for (int kk = 0; kk < NQ; kk++) {
+                                const f2_t dx = f2_add(sxy.x, ntx2[kk]), dyy = f2_add(sxy.y, nty2[kk]);
+                                const f2_t r2 = f2_fma(dx, dx, f2_fma(dyy, dyy, eps2x2));
+                                const f2_t w = f2_mul(mm, f2_rcp(r2));
+                                nax2[kk] = f2_fma(w, dx, nax2[kk]);
+                                nay2[kk] = f2_fma(w, dyy, nay2[kk]);
+                            }
                         }
+                    } else {
+                        float ax, ay, u;
+                        f2_unpack(nax2[0], ax, u);
+                        f2_unpack(nay2[0], ay, u);
+                        const float ntx = -tx[0], nty = -ty[0];
+#pragma unroll 8
+                        for (int j = slice; j < ns; j += nslice) {
+                            const float4 e = s4[2 * j];
+                            pair1(e.x, e.z, s4[2 * j + 1].x, ntx, nty, eps2, ax, ay);
+                        }
+                        nax2[0] = f2_pack(ax, ax);
+                        nay2[0] = f2_pack(ay, ay);
                     }
                 }
-                if (lane == 0) wcnt[0] += (unsigned long long)T * ns;
+                nns += ns;
                 __syncwarp();  // every lane is done with this buffer
                 if (p + 2 < npass) issue(p + 2);
             }
@@ -506,28 +593,34 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
         }
 
 
+        if (lane == 0 && r0 == 0) {
+            wcnt[0] += (unsigned long long)T * nns;
+            wcnt[1] += (unsigned long long)T * nfs;
+        }
         // ---- reduce slice partials (through the source buffers) and write
         if (active) {
 #pragma unroll
-            for (int k = 0; k < NR / 2; k++) {
+            for (int k = 0; k < NQ; k++) {
                 float a0, a1, b0, b1;
                 f2_unpack(nax2[k], a0, a1);
                 f2_unpack(nay2[k], b0, b1);
-                float *o = red + 2 * ((slice * nthr + tl) * NR + 2 * k);
+                float *o = red + 2 * ((slice * nthr + tl) * NP + 2 * k);
                 o[0] = a0;
                 o[1] = b0;
-                o[2] = a1;
-                o[3] = b1;
+                if (NP > 1) {
+                    o[2] = a1;
+                    o[3] = b1;
+                }
             }
         }
         __syncwarp();
-        // every lane takes targets v = lane, lane + 32, ... (not only the first slice's lanes)
-        for (int v = lane; v < T; v += 32) {
-            {
-                const int vt = v / NR, r = v - vt * NR;  // the lane and register that held it
+        // every lane takes targets k = lane, lane + 32, ... of the part (not only the first slice's lanes)
+        for (int k = lane; k < nthr * NP; k += 32) {
+            const int vt = k / NP, r = k - vt * NP, v = vt * NR + r0 + r;  // the lane and register that held it
+            if (v < T) {
                 float sx = 0.f, sy = 0.f;
-                for (int k = 0; k < nslice; k++) {
-                    const float *o = red + 2 * ((k * nthr + vt) * NR + r);
+                for (int q = 0; q < nslice; q++) {
+                    const float *o = red + 2 * ((q * nthr + vt) * NP + r);
                     sx += o[0];
                     sy += o[1];
                 }
@@ -555,6 +648,10 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
             }
         }
         __syncwarp();  // the staging and the column table are reused by the next item
+        };
+        if (!SPLIT || np == NR) run(std::integral_constant<int, NR>());
+        else if (np == 2) run(std::integral_constant<int, 2>());
+        else run(std::integral_constant<int, 1>());
     }
     if (lane == 0) {
         atomicAdd(&d.glob->near_pairs, wcnt[0]);
@@ -562,26 +659,45 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
     }
 }
 
-template <bool KAHAN, int MINB>
-static cudaError_t launch_fstream_t(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
-                                    const cudaEvent_t *ev) {
-    long long items_max = d.NG_total + d.n_total / d.dense_min +
-                          (d.quad_min > 0 ? 4 * (d.n_total / d.quad_min) : 0) + d.n_total / STREAM_ITEM_DIV + 1;
-    long long grid = (long long)d.nsm * MINB;
-    if (grid * FW > items_max) grid = (items_max + FW - 1) / FW;
+template <bool KAHAN, int MINB, bool SPLIT>
+static cudaError_t launch_fstream_s(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
+                                    const cudaEvent_t *ev, long long entries_max, int ctas) {
+    long long grid = (long long)d.nsm * ctas;
+    if (grid * FW > entries_max) grid = (entries_max + FW - 1) / FW;
     if (grid < 1) grid = 1;
     cudaError_t e = cudaMemsetAsync(&d.glob->item_next, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
-    k_fstream<KAHAN, MINB><<<(unsigned)grid, FW * 32, FsLayout<MINB>::SMEM, st>>>(d, tick ? 1 : 0, accumulate ? 1 : 0);
+    k_fstream<KAHAN, MINB, SPLIT>
+        <<<(unsigned)grid, FW * 32, FsLayout<MINB>::SMEM, st>>>(d, tick ? 1 : 0, accumulate ? 1 : 0);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return ev ? cudaEventRecord(ev[1], st) : cudaSuccess;
 }
 
+// Plans of few items (by their bound, about four times the count) take the build that can split
+// items, with fewer CTAs per SM: all items resident at once leave an SM's share of the cost to
+// chance (131,071 particles of one Gaussian: the busiest SM had twice the mean), two rounds or more
+// even it out.  131,071 particles, the step: 950 us with whole items on 24 warps per SM, 700 split,
+// 528 split on 8 warps (12 warps 557, 4 warps 603).  250,000 of one Gaussian: 1,941 us -> 1,273 with three CTAs (two 1,232, four 1,374); 400,000 clustered 689 -> 608 with four;
+// 1,048,576 clustered 981 with six whole, 983 with five, 1,098 with three.
+template <bool KAHAN, int MINB>
+static cudaError_t launch_fstream_t(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
+                                    const cudaEvent_t *ev) {
+    const long long items_max = d.NG_total + d.n_total / d.dense_min +
+                                (d.quad_min > 0 ? 4 * (d.n_total / d.quad_min) : 0) + d.n_total / STREAM_ITEM_DIV + 1;
+    const long long step = 16LL * d.nsm * MINB;
+    if (items_max <= 4 * step)
+        return launch_fstream_s<KAHAN, MINB, true>(d, tick, accumulate, st, ev, 4 * items_max,
+                                                   2 + (int)((items_max - 1) / step));
+    return launch_fstream_s<KAHAN, MINB, false>(d, tick, accumulate, st, ev, items_max, MINB);
+}
+
 template <bool KAHAN, int MINB>
 static cudaError_t init_fstream_t() {
-    return cudaFuncSetAttribute(k_fstream<KAHAN, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)FsLayout<MINB>::SMEM);
+    const int sm = (int)FsLayout<MINB>::SMEM;
+    cudaError_t e = cudaFuncSetAttribute(k_fstream<KAHAN, MINB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_fstream<KAHAN, MINB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
 cudaError_t fstream_init() {

@@ -179,3 +179,30 @@ def test_walk_items_one_or_two_ctas(prec, cutoff, eps):
             assert rel_rms(big[:, o:o + n], one) < 1e-5
         o += n
     assert pairs == (near, far)
+
+
+# A small plan splits its heaviest work items over several warps: half or a quarter of each quad of
+# targets with the same slices and the same order of sources.  The same system in a batch whose other
+# systems raise the item bound past the rule runs whole items; without boxes that straddle leaf chunks
+# (every system's particle count a multiple of 32) its leaf sums are the same, and so is every bit.
+@pytest.mark.parametrize("n,grid,group,dense,quad,layout", [(32, 1, 1, 16, -1, "uniform"), (4096, 8, 1, 16, 128, "cluster"),
+                                                            (20000, 16, 2, 0, 0, "cluster"), (65536, 8, 4, 16, -1, "uniform")])
+@pytest.mark.parametrize("prec,tune", [(0, 0), (1, 0), (1, 1)])
+def test_split_items_are_the_same_bits(n, grid, group, dense, quad, layout, prec, tune):
+    from barneshut.gb300 import native, workloads
+
+    s = (workloads.uniform if layout == "uniform" else workloads.cluster_mixture)(n, seed=n)
+    rest = workloads.uniform(1 << 21, seed=7)
+    prm = native.make_params(1.0, 1e-5, 1e-4, 0.0, 0.5, group, prec, 0, tune, dense_min=dense, quad_min=quad)
+
+    def accel(sizes, grids, cols):
+        plan = native.Plan(sizes, grids, prm)
+        plan.load(*cols)
+        plan.step(1)
+        out = plan.store()
+        assert plan.error_flags() == 0
+        return [out[k][:n].cpu().numpy() for k in ("ax", "ay", "x", "y", "vx", "vy")]
+
+    alone = accel([n], [grid], s)
+    both = accel([n, 1 << 21], [grid, 181], [np.concatenate([s[k], rest[k]]) for k in range(5)])
+    assert all(np.array_equal(a, b) for a, b in zip(alone, both))
