@@ -50,6 +50,8 @@ constexpr int SITEM_TILE = 8;     // target groups per tile of the streaming wor
 constexpr int SUM_TILE = 16;      // leaf boxes per side of a summarize tile (pyramid levels 0..4)
 constexpr int STREAM_CHUNK = 128;  // targets per work item of the list-streaming force kernel
 constexpr int LIST_MAX_G = 16384;  // largest G of the list-streaming path (32-bit group indices)
+constexpr long long STORE_GATHER_MIN = 262144;  // k_store: from here on a disordered state is gathered
+constexpr int STORE_NEAR = 64;
 constexpr int ITEM_BUCKETS = 32;   // log2 cost buckets of the heaviest-first item order
 
 struct SysDesc {
@@ -92,6 +94,7 @@ struct Globals {
     unsigned int bbox_done;         // bounding-box blocks finished (the last one finalises)
     unsigned int nbig;              // entries of the long-quadrant list (k_segsort)
     unsigned int nhuge;             // entries of the very-long-quadrant list, from its far end
+    unsigned int far_pids;          // box-sorted neighbours whose pids lie more than STORE_NEAR apart
 };
 
 struct DevPlan {

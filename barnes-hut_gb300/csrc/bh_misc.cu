@@ -33,16 +33,35 @@ __global__ void k_load(DevPlan d, const double *x, const double *y, const double
     }
 }
 
+// A state whose box order is far from its pid order (more than a quarter of the neighbours, counted
+// by k_gather) is downloaded by gathering: random reads of whole sectors, coalesced writes.  The
+// scatter writes each 8-byte value to a sector of its own, which only pays where neighbours share
+// sectors.  27.3M particles of 512 systems in file order: 4,078 us -> 1,363 us with the inverse; 1,048,576: 66 -> 44 us; 4,194,304 in
+// box order stay with the scatter (59 us, the memory's rate).
+__device__ __forceinline__ bool store_gathers(const DevPlan &d) {
+    return 4ull * d.glob->far_pids > (unsigned long long)d.n_total;
+}
+
+// inverse permutation of the current state into the key array, where k_store will gather
+__global__ void k_store_inverse(DevPlan d) {
+    if (!store_gathers(d)) return;
+    const int b = (d.glob->epoch + 1) & 1;
+    long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride)
+        d.key[d.PID[b][i]] = (int)i;
+}
+
 // Download in pid order.  rec: N x 10 records (px, py, mass, vx, vy, ax, ay,
 // gx, gy, pid) or NULL; SoA outputs may be NULL.  gx/gy come from the box
 // keys of the last create_tree (skey), 0 before the first one; ax/ay are 0
-// when no evaluation followed the last load (has_acc = 0).
+// when no evaluation followed the last load (has_acc = 0).  gather: k_store_inverse ran before.
 __global__ void k_store(DevPlan d, double *rec, double *x, double *y, double *vx, double *vy,
-                        double *ax, double *ay, int has_tree, int has_acc) {
+                        double *ax, double *ay, int has_tree, int has_acc, int gather) {
     const int b = (d.glob->epoch + 1) & 1;
     long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride) {
-        long long p = d.PID[b][i];
+    const bool inv = gather && store_gathers(d);
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < d.n_total; k += stride) {
+        const long long i = inv ? d.key[k] : k, p = inv ? k : d.PID[b][k];
         double px = d.X[b][i], py = d.Y[b][i], pvx = d.VX[b][i], pvy = d.VY[b][i];
         const double pax = has_acc ? d.AX[i] : 0.0, pay = has_acc ? d.AY[i] : 0.0;
         if (rec) {
@@ -264,7 +283,11 @@ cudaError_t launch_load(const DevPlan &d, const double *x, const double *y, cons
 cudaError_t launch_store(const DevPlan &d, int has_tree, bool has_acc, double *rec, double *x, double *y,
                          double *vx, double *vy, double *ax, double *ay, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    k_store<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d, rec, x, y, vx, vy, ax, ay, has_tree, has_acc ? 1 : 0);
+    // (before the first create_tree the state is in pid order)
+    const bool gather = has_tree && d.n_total >= STORE_GATHER_MIN;
+    if (gather) k_store_inverse<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d);
+    k_store<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d, rec, x, y, vx, vy, ax, ay, has_tree, has_acc ? 1 : 0,
+                                                           gather ? 1 : 0);
     return cudaGetLastError();
 }
 

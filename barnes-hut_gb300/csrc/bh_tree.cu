@@ -31,6 +31,7 @@ __global__ void k_prologue(DevPlan d) {
         d.glob->near_pairs = 0;
         d.glob->far_pairs = 0;
         d.glob->corr_pairs = 0;
+        d.glob->far_pids = 0;
     }
     if (tid < d.nsys) {
         d.dyn[tid].bbmin[0] = d.dyn[tid].bbmin[1] = ~0ull;
@@ -157,7 +158,22 @@ __global__ void __launch_bounds__(TPB) k_bbox(DevPlan d) {
         bool one_sys = d.poff_tab[s_first + 1] >= t1;
         unsigned long long mn0 = ~0ull, mn1 = ~0ull, mx0 = 0, mx1 = 0;
         int cs = s_first;
-        for (long long i = t0 + threadIdx.x; i < t1; i += TPB) {
+        if (one_sys && t1 - t0 == tile) {  // a whole tile of one system: 16-byte pairs, all in flight
+            const double2 *X2 = reinterpret_cast<const double2 *>(X + t0), *Y2 = reinterpret_cast<const double2 *>(Y + t0);
+            double2 a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                a[u] = X2[threadIdx.x + u * TPB];
+                b[u] = Y2[threadIdx.x + u * TPB];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                minmax_ord(ord_bits(a[u].x), mn0, mx0);
+                minmax_ord(ord_bits(a[u].y), mn0, mx0);
+                minmax_ord(ord_bits(b[u].x), mn1, mx1);
+                minmax_ord(ord_bits(b[u].y), mn1, mx1);
+            }
+        } else for (long long i = t0 + threadIdx.x; i < t1; i += TPB) {
             if (!one_sys) {
                 int s = find_seg(d.poff_tab, d.nsys, i);
                 if (s != cs) {
@@ -182,7 +198,8 @@ __global__ void __launch_bounds__(TPB) k_bbox(DevPlan d) {
         }
         __syncthreads();
     }
-    // the last block to finish squares every system's box and tabulates the box origins
+    // the last block to finish squares every system's box, a thread per system (512 systems one after
+    // another took 1.4 ms)
     __shared__ unsigned ticket;
     __threadfence();
     __syncthreads();
@@ -190,18 +207,21 @@ __global__ void __launch_bounds__(TPB) k_bbox(DevPlan d) {
     __syncthreads();
     if (ticket != gridDim.x - 1) return;
     __threadfence();
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < d.nsys; s++)
-            if (d.sys[s].n > 0) bbox_finalize_sys(d, s);
-        d.glob->bbox_done = 0u;
-    }
-    __syncthreads();
-    for (int s = 0; s < d.nsys; s++) {
+    for (int s = threadIdx.x; s < d.nsys; s += TPB)
+        if (d.sys[s].n > 0) bbox_finalize_sys(d, s);
+    if (threadIdx.x == 0) d.glob->bbox_done = 0u;
+}
+
+// The box-origin tables of the systems (read by k_gather): the blocks share a single system's table,
+// or take whole systems.
+__device__ __forceinline__ void fill_origins(const DevPlan &d) {
+    for (int s = d.nsys == 1 ? 0 : blockIdx.x; s < d.nsys; s += d.nsys == 1 ? 1 : gridDim.x) {
         if (d.sys[s].n == 0) continue;
         const SysDyn &dy = d.dyn[s];
         const int G = d.sys[s].G;
         double *org = d.org + d.sys[s].ooff;
-        for (int k = threadIdx.x; k < G; k += blockDim.x) {
+        const int k0 = d.nsys == 1 ? blockIdx.x * TPB : 0, dk = d.nsys == 1 ? gridDim.x * TPB : TPB;
+        for (int k = k0 + threadIdx.x; k < G; k += dk) {
             org[k] = box_origin(dy.minx, k, dy.step);
             org[G + k] = box_origin(dy.miny, k, dy.step);
         }
@@ -223,6 +243,7 @@ __global__ void __launch_bounds__(TPB, 4) k_place(DevPlan d) {
     const double *X = d.X[cur], *Y = d.Y[cur];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e0 = (int)threadIdx.x * PLACE_PP;  // the thread's first particle in the round
+    fill_origins(d);
     for (long long base = (long long)blockIdx.x * PT; base < d.n_total; base += (long long)gridDim.x * PT) {
         const long long i0 = base + e0;
         double x[PLACE_PP], y[PLACE_PP];
@@ -649,7 +670,7 @@ __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
 //   k_perm     perm[box_start + earlier quadrants + slot] = input index (slots: k_place);
 //   k_segsort  each quadrant's stretch of perm sorted ascending -- up to SEG_REG entries in a
 //              thread's registers, longer ones listed for k_segsort_big (up to SEG_WARP entries
-//              a warp each, a bitonic network in its slice of shared memory; longer ones a CTA
+//              a warp each, a bitonic network in its registers or shared memory; longer ones a CTA
 //              each, four stable 8-bit radix passes through the dead slot array);
 //   k_gather   output particle t takes input perm[t]: the FP64 state of the next buffer, the
 //              32-byte packed record (offsets from the box origin computed in FP64, rounded
@@ -723,18 +744,82 @@ __global__ void __launch_bounds__(TPB) k_segsort(DevPlan d) {
     }
 }
 
+// Ascending sort of the warp's 32 R values (element 32 r + lane in v[r]): a bitonic network, strides
+// below 32 by shuffles, the others between a lane's registers.
+template <int R>
+__device__ __forceinline__ void warp_bitonic(int v[R]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * R; size <<= 1)
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const bool up = ((32 * r + lane) & size) == 0;
+                if (stride >= 32) {
+                    const int q = r ^ (stride >> 5);
+                    if (q > r) {
+                        const int lo = min(v[r], v[q]), hi = max(v[r], v[q]);
+                        v[r] = up ? lo : hi;
+                        v[q] = up ? hi : lo;
+                    }
+                } else {
+                    const int o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+                    v[r] = up == ((lane & stride) == 0) ? min(v[r], o) : max(v[r], o);
+                }
+            }
+}
+
+// a stretch of n <= 32 R entries in registers; left alone when its slots were handed out in order
+template <int R>
+__device__ __forceinline__ void seg_regs(int *p, int n) {
+    const int lane = threadIdx.x & 31;
+    int v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = 32 * r + lane < n ? p[32 * r + lane] : 0x7FFFFFFF;
+    bool sorted = true;  // (padding sorts after every index)
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        int nx = __shfl_down_sync(0xffffffffu, v[r], 1);
+        if (r + 1 < R) {
+            const int first = __shfl_sync(0xffffffffu, v[r + 1], 0);
+            if (lane == 31) nx = first;
+        } else if (lane == 31) {
+            nx = 0x7FFFFFFF;
+        }
+        sorted &= v[r] <= nx;
+    }
+    if (__all_sync(0xffffffffu, sorted)) return;
+    warp_bitonic<R>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (32 * r + lane < n) p[32 * r + lane] = v[r];
+}
+
+// Long stretches.  Up to SEG_LANES entries a warp sorts in its registers (batches of small boxes in
+// file order have most of theirs here: 27.3M particles 670 -> 344 us, against the shared-memory
+// network), up to SEG_WARP in its slice of shared memory, longer ones a CTA.
+constexpr int SEG_LANES = 256;
+
 __global__ void __launch_bounds__(TPB) k_segsort_big(DevPlan d) {
     __shared__ int sv[TPB / 32][SEG_WARP];
     __shared__ int hist[256], base[256], run[256], wcnt[TPB / 32][256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // stretches of SEG_REG + 1 .. SEG_WARP entries: a warp each, a bitonic network over the next
-    // power of two (padded with INT_MAX) in the warp's slice of shared memory
+    // stretches of SEG_REG + 1 .. SEG_WARP entries: a warp each; beyond SEG_LANES a bitonic network
+    // over the next power of two (padded with INT_MAX) in the warp's slice of shared memory
     const unsigned nbig = d.glob->nbig;
     int *w = sv[warp];
     for (unsigned e = (unsigned)(blockIdx.x * (TPB / 32) + warp); e < nbig; e += gridDim.x * (TPB / 32)) {
         const int2 sg = d.bigseg[e];
         const int s0 = sg.x, n = sg.y;
-        int m = 32;
+        if (n <= SEG_LANES) {
+            if (n <= 32) seg_regs<1>(d.perm + s0, n);
+            else if (n <= 64) seg_regs<2>(d.perm + s0, n);
+            else if (n <= 128) seg_regs<4>(d.perm + s0, n);
+            else seg_regs<8>(d.perm + s0, n);
+            continue;
+        }
+        int m = 2 * SEG_LANES;
         while (m < n) m <<= 1;
         // a stretch whose slots the atomics happened to hand out in input order is done already
         // (the common case when the input is the previous step's order)
@@ -895,6 +980,8 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
     const bool one = d.nsys == 1;
     const int G0 = d.sys[0].G;
     const long long boff0 = d.sys[0].boff, ooff0 = d.sys[0].ooff;
+    const bool count_far = n >= STORE_GATHER_MIN;  // for k_store
+    unsigned far_pids = 0;  // neighbours whose pids lie far apart (the lane's count)
     for (long long w0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); w0 < n; w0 += SU * stride) {
         const long long t0 = w0 + lane;
         int src[SU], key4[SU];
@@ -913,6 +1000,7 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
 #pragma unroll
         for (int u = 0; u < SU; u++) {
             const long long t = t0 + u * stride;
+            pid[u] = 0;
             if (t < n) {
                 const int i = src[u];
                 x[u] = d.X[cur][i];
@@ -928,7 +1016,9 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
         for (int u = 0; u < SU; u++) {
             const long long t = t0 + u * stride;
             lx[u] = ly[u] = lm[u] = 0.f;
+            const int pn = count_far ? __shfl_down_sync(0xffffffffu, pid[u], 1) : pid[u];
             if (t >= n) continue;
+            if (lane < 31 && t + 1 < n && (unsigned)(pn - pid[u] + STORE_NEAR) > 2u * STORE_NEAR) far_pids++;
             const int key = key4[u] >> 2;
             const int s = one ? 0 : find_seg(d.boff_tab, d.nsys, key);
             const int G = one ? G0 : d.sys[s].G;
@@ -941,7 +1031,7 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
             d.VY[nxt][t] = vy[u];
             d.M[nxt][t] = m[u];
             d.PID[nxt][t] = pid[u];
-            const double *org = d.org + ooff;  // box origins (tabulated by k_bbox's last block)
+            const double *org = d.org + ooff;  // box origins (tabulated by k_place)
             const float ox = f64_to_f32_rn(__dsub_rn(x[u], org[kx]));
             const float oy = f64_to_f32_rn(__dsub_rn(y[u], org[G + ky]));
             const float mf = f64_to_f32_rn(m[u]);
@@ -961,6 +1051,10 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
             if (t < n) leaf_terms<SECOND>(lx[u], ly[u], lm[u], v);
             leaf_chunk<SECOND>(d, wu >> 5, t < n ? key4[u] >> 2 : -1, v);
         }
+    }
+    if (count_far) {
+        far_pids = __reduce_add_sync(0xffffffffu, far_pids);
+        if (lane == 0 && far_pids) atomicAdd(&d.glob->far_pids, far_pids);
     }
 }
 
@@ -1212,7 +1306,8 @@ cudaError_t launch_prologue(const DevPlan &d, cudaStream_t st) {
 }
 cudaError_t launch_bbox(const DevPlan &d, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    k_bbox<<<d.nsys == 1 ? (unsigned)(d.nsm * 4) : grid_for(d.n_total, TPB * 16, d.nsm * 8LL), TPB, 0, st>>>(d);
+    // (a block per 2,048 particles at least: its five atomics meet every other block's)
+    k_bbox<<<grid_for(d.n_total, TPB * (d.nsys == 1 ? 8 : 16), d.nsm * (d.nsys == 1 ? 4LL : 8LL)), TPB, 0, st>>>(d);
     return cudaGetLastError();
 }
 cudaError_t launch_place(const DevPlan &d, cudaStream_t st) {

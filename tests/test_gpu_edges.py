@@ -206,3 +206,79 @@ def test_split_items_are_the_same_bits(n, grid, group, dense, quad, layout, prec
     alone = accel([n], [grid], s)
     both = accel([n, 1 << 21], [grid, 181], [np.concatenate([s[k], rest[k]]) for k in range(5)])
     assert all(np.array_equal(a, b) for a, b in zip(alone, both))
+
+
+# Download of a state whose box order is far from the pid order (gathered from 262,144 particles on) or
+# close to it (scattered): create_tree reorders the state and changes nothing else.
+@pytest.mark.parametrize("n", [1, 262143, 262144, 300007])
+@pytest.mark.parametrize("order", ["file", "box"])
+def test_store_returns_the_state(n, order):
+    from barneshut.gb300 import native, workloads
+
+    s = workloads.cluster_mixture(n, seed=3)
+    if order == "box":
+        o = workloads.box_order(s[0], s[1], 64)
+        s = tuple(a[o] for a in s)
+    plan = native.Plan([n], [64], native.make_params(1.0, 1e-5, 1e-4, 0.0, 0.5))
+    vx, vy = np.random.default_rng(n).random((2, n))
+    plan.load(s[0], s[1], s[2], vx, vy)
+    for _ in range(2):
+        out = plan.store()
+        rec = plan.store_records().cpu().numpy()
+        for k, a in (("x", s[0]), ("y", s[1]), ("vx", vx), ("vy", vy)):
+            assert np.array_equal(out[k].cpu().numpy(), a)
+        assert np.array_equal(rec[:, :5], np.stack([s[0], s[1], s[2], vx, vy], axis=1))
+        assert np.array_equal(rec[:, 9], np.arange(n)) and not rec[:, 5:7].any()
+        plan.create_tree()
+    assert plan.error_flags() == 0
+
+
+# The order within a quadrant is the input order whatever slots the placement handed out: quadrants at
+# the edges of the sorting forms (registers of a thread, of a warp, shared memory, a CTA), in random
+# input order against the same particles loaded in box order.
+@pytest.mark.parametrize("count", [2, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 1024, 1025, 3000])
+def test_quadrant_sort_sizes(count):
+    from barneshut.gb300 import native, workloads
+
+    rng = np.random.default_rng(count)
+    counts = np.array([count, count, max(1, count - 1), 3])
+    q = np.repeat(np.arange(4), counts)
+    n = len(q) + 2
+    x = np.concatenate([[0.0, 1.0], 0.25 * (q >> 1) + 0.01 + 0.22 * rng.random(len(q))])
+    y = np.concatenate([[0.0, 1.0], 0.25 * (q & 1) + 0.01 + 0.22 * rng.random(len(q))])
+    o = rng.permutation(n)
+    x, y = x[o], y[o]
+    m = 1.0 + rng.random(n)
+    z = np.zeros(n)
+    prm = native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5, 1, quad_min=128)
+
+    def accel(cols):
+        plan = native.Plan([n], [2], prm)
+        plan.load(*cols, z, z)
+        plan.step(1)
+        out = plan.store()
+        assert plan.error_flags() == 0
+        return torch.stack([out["ax"], out["ay"]]).cpu().numpy()
+
+    b = workloads.box_order(x, y, 2)
+    assert np.array_equal(accel((x, y, m))[:, b], accel((x[b], y[b], m[b])))
+
+
+# A batch of more systems than a block has threads, empty ones among them: each with its own box.
+def test_bounding_boxes_of_many_systems():
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(9)
+    sizes = [int(v) for v in rng.integers(0, 40, 300)] + [5000, 0, 8192, 1]
+    shift = rng.uniform(-5, 5, (len(sizes), 2))
+    pts = [shift[k] + rng.random((v, 2)) for k, v in enumerate(sizes)]
+    x, y = np.concatenate(pts).T.copy()
+    n = len(x)
+    plan = native.Plan(sizes, [3] * len(sizes), native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5))
+    plan.load(x, y, np.ones(n), np.zeros(n), np.zeros(n))
+    plan.create_tree()
+    for k, p in enumerate(pts):
+        if len(p):
+            g = plan.grid_info(k)
+            assert (g["min_x"], g["min_y"]) == (p[:, 0].min(), p[:, 1].min())
+    assert plan.error_flags() == 0
