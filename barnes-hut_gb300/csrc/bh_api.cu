@@ -41,6 +41,7 @@ struct bh_plan {
     void *ws = nullptr;
     int device = -1;
     int nsm = 1;  // streaming multiprocessors of `device`
+    int cl_ctas = 8;  // CTAs of a small system's tree kernel
     DevPlan dev;
     bool has_tree = false;
     bool acc_stale = true;  // next bh_evaluate overwrites instead of accumulating
@@ -397,6 +398,7 @@ static void fill_dev(bh_plan *p) {
     d.item_bucket = (int *)(w + p->o_ibkt);
     d.item_cost = (unsigned char *)(w + p->o_icost);
     d.nsm = p->nsm;
+    d.cl_ctas = p->cl_ctas;
     d.stream = p->stream ? 1 : 0;
     d.chunk = p->chunk;
     const bh_params &pr = p->params;
@@ -425,6 +427,7 @@ extern "C" int bh_bind(bh_plan *p, void *workspace, size_t bytes, void *stream) 
     if (p->nsm < 1) p->nsm = 1;
     CK(p, force_init(), "force kernel attributes");
     CK(p, learned_init(), "learned kernel attributes");
+    CK(p, tree_init(&p->cl_ctas), "tree kernel attributes");
     if (!p->side) CK(p, cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking), "side stream");
     if (!p->fork_ev) CK(p, cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming), "fork event");
     if (!p->join_ev) CK(p, cudaEventCreateWithFlags(&p->join_ev, cudaEventDisableTiming), "join event");
@@ -506,7 +509,19 @@ extern "C" int bh_store(bh_plan *p, double *x, double *y, double *vx, double *vy
     return BH_OK;
 }
 
-static int enqueue_tree(bh_plan *p, cudaStream_t st) {
+// One small system without the learned correction: its tree is one kernel's work.
+static bool cluster_tree(const bh_plan *p) {
+    return p->nsys == 1 && !(p->params.flags & BH_FLAG_LEARNED) && p->n_total > 0 && p->n_total <= CL_MAX_N &&
+           p->B_total <= CL_MAX_BOXES;
+}
+
+// summary: the summarize phase too (launched by the caller where the tree is not one kernel's work)
+static int enqueue_tree(bh_plan *p, bool summary, cudaStream_t st) {
+    if (cluster_tree(p)) {
+        CK(p, launch_tree_cluster(p->dev, summary, st), "tree");
+        p->leaves_stale = false;
+        return BH_OK;
+    }
     CK(p, launch_prologue(p->dev, st), "prologue");
     CK(p, launch_bbox(p->dev, st), "bbox");
     CK(p, launch_place(p->dev, st), "place");
@@ -519,13 +534,14 @@ static int enqueue_tree(bh_plan *p, cudaStream_t st) {
     CK(p, launch_scatter(p->dev, st), "scatter");  // (and the leaf sums)
     p->leaves_stale = false;
     CK(p, cudaStreamWaitEvent(st, p->join_ev, 0), "join wait");
+    if (summary) CK(p, launch_summarize(p->dev, false, st), "summarize");
     return BH_OK;
 }
 
 extern "C" int bh_create_tree(bh_plan *p, void *stream) {
     int r = need_bound(p);
     if (r) return r;
-    r = enqueue_tree(p, (cudaStream_t)stream);
+    r = enqueue_tree(p, false, (cudaStream_t)stream);
     if (r) return r;
     p->has_tree = true;
     p->acc_stale = true;
@@ -573,9 +589,8 @@ extern "C" int bh_timestep(bh_plan *p, void *stream) {
 
 static int enqueue_steps(bh_plan *p, int nsteps, cudaStream_t st) {
     for (int k = 0; k < nsteps; k++) {
-        int r = enqueue_tree(p, st);
+        int r = enqueue_tree(p, true, st);
         if (r) return r;
-        CK(p, launch_summarize(p->dev, false, st), "summarize");
         if (p->dev.learned) {
             if (!p->mlp_img) return fail(p, BH_ERR_INVALID, "BH_FLAG_LEARNED without bh_set_correction");
             CK(p, launch_force(p->dev, false, false, st), "force");
@@ -676,8 +691,11 @@ extern "C" int bh_kernels_per_step(const bh_plan *p, int *count) {
     // correction, one kernel for list streaming
     const bool walk_items = !p->stream || (p->params.flags & BH_FLAG_LEARNED);
     // (a walking plan's tick is a kernel of its own: the walk reads the state the tick writes)
-    *count = 1 + 1 + (walk_items ? 3 : 0) + 1 + (p->n_total > 0 ? 7 : 0) + (p->stream ? 1 : 0) +
-             (p->stream && p->n_total > 0 ? 3 : 0) + (!p->stream && p->n_total > 0 ? 1 : 0);
+    // A small system's tree, work items and summarize are one kernel (cluster_tree).
+    const int tree = cluster_tree(p) ? 1 : 1 + 1 + (walk_items ? 3 : 0) + 1 + (p->n_total > 0 ? 6 : 0) + (p->stream ? 1 : 0);
+    const long long items_max = p->NG_total + p->n_total / p->dense_min +
+                                (p->quad_min > 0 ? 4 * (p->n_total / p->quad_min) : 0) + p->n_total / STREAM_ITEM_DIV + 1;
+    *count = tree + (p->n_total > 0 ? 1 : 0) + (p->stream && p->n_total > 0 ? list_kernels(items_max) : 0) + (!p->stream && p->n_total > 0 ? 1 : 0);
     return BH_OK;
 }
 

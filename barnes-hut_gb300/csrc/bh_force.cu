@@ -630,6 +630,11 @@ k_force(DevPlan d, int tick, int accumulate) {
     if (tid == 0) {
         atomicAdd(&d.glob->near_pairs, npairs);
         atomicAdd(&d.glob->far_pairs, fpairs);
+        // the last CTA leaves the queue as the next launch wants it (no other CTA takes from it now)
+        if (atomicAdd(&d.glob->force_done, 1u) == gridDim.x - 1) {
+            d.glob->item_next = 0u;
+            d.glob->force_done = 0u;
+        }
     }
 }
 
@@ -658,8 +663,6 @@ static cudaError_t launch_force_nr(const DevPlan &d, bool accumulate, cudaStream
 template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 6 : 8)>
 static cudaError_t launch_force_t(const DevPlan &d, bool accumulate, cudaStream_t st) {
     const long long items_max = d.NG_total + d.n_total / d.chunk + 1;
-    cudaError_t e = cudaMemsetAsync(&d.glob->item_next, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
     if constexpr (sizeof(R) == 4)
         if (2 * items_max <= (long long)d.nsm * MINB)
             return launch_force_nr<R, 2, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);

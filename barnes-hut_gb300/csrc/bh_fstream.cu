@@ -656,6 +656,11 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
     if (lane == 0) {
         atomicAdd(&d.glob->near_pairs, wcnt[0]);
         atomicAdd(&d.glob->far_pairs, wcnt[1]);
+        // the last warp leaves the queue as the next launch wants it (no other warp takes from it now)
+        if (atomicAdd(&d.glob->force_done, 1u) == gridDim.x * FW - 1) {
+            d.glob->item_next = 0u;
+            d.glob->force_done = 0u;
+        }
     }
 }
 
@@ -665,8 +670,7 @@ static cudaError_t launch_fstream_s(const DevPlan &d, bool tick, bool accumulate
     long long grid = (long long)d.nsm * ctas;
     if (grid * FW > entries_max) grid = (entries_max + FW - 1) / FW;
     if (grid < 1) grid = 1;
-    cudaError_t e = cudaMemsetAsync(&d.glob->item_next, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
     k_fstream<KAHAN, MINB, SPLIT>
         <<<(unsigned)grid, FW * 32, FsLayout<MINB>::SMEM, st>>>(d, tick ? 1 : 0, accumulate ? 1 : 0);

@@ -50,6 +50,7 @@ constexpr int SITEM_TILE = 8;     // target groups per tile of the streaming wor
 constexpr int SUM_TILE = 16;      // leaf boxes per side of a summarize tile (pyramid levels 0..4)
 constexpr int STREAM_CHUNK = 128;  // targets per work item of the list-streaming force kernel
 constexpr int LIST_MAX_G = 16384;  // largest G of the list-streaming path (32-bit group indices)
+constexpr int CL_MAX_N = 32768, CL_MAX_SIDE = 64, CL_MAX_BOXES = 4096;  // systems whose tree one cluster builds (k_tree_cluster)
 constexpr long long STORE_GATHER_MIN = 262144;  // k_store: from here on a disordered state is gathered
 constexpr int STORE_NEAR = 64;
 constexpr int ITEM_BUCKETS = 32;   // log2 cost buckets of the heaviest-first item order
@@ -86,12 +87,14 @@ struct Globals {
     unsigned int epoch;
     unsigned int err;
     unsigned long long near_pairs, far_pairs;
-    unsigned int item_next;   // force work queue head (zeroed before each force launch)
+    unsigned int item_next;   // force work queue head (reset by each force launch's last warp or CTA)
     unsigned int item_next2;  // learned-correction work queue head
     unsigned long long corr_pairs;  // (target, cell) pairs the learned correction evaluated
     unsigned int scan_ticket[3];    // next tile of each single-pass scan (its last tile resets it)
     unsigned int scan_gen[3];       // generation of each scan's tile states (its last tile bumps it)
     unsigned int bbox_done;         // bounding-box blocks finished (the last one finalises)
+    unsigned int force_done;        // warps (list streaming) or CTAs (walk) of the force launch that left
+                                    // the queue (the last one resets its head)
     unsigned int nbig;              // entries of the long-quadrant list (k_segsort)
     unsigned int nhuge;             // entries of the very-long-quadrant list, from its far end
     unsigned int far_pids;          // box-sorted neighbours whose pids lie more than STORE_NEAR apart
@@ -158,6 +161,7 @@ struct DevPlan {
     unsigned char *item_cost;  // per list-streaming work item, its cost bucket (k_item_hist)
     int nsm;     // streaming multiprocessors of the plan's device (queried at bh_bind): sizes the
                  // persistent and grid-stride launches
+    int cl_ctas;  // CTAs of a small system's tree kernel (tree_init)
     int stream;  // 1: lists are built by k_lists and streamed by k_fstream
     int chunk;   // targets per work item (TARGET_CHUNK, TARGET_CHUNK64, or STREAM_CHUNK when stream)
     // parameters
@@ -289,6 +293,12 @@ __device__ __forceinline__ int half_key1_f32(double p, double mn, double step, d
     const float k = floorf(q);
     const float fr = q - k;
     const float tol2 = 2.f * tol;
+    if (tol2 < 0.25f) {
+        // in the first or the last half box whatever the quotient's floor is (the particles that
+        // define the bounding box lie on its edges)
+        if (q < 1.f - tol2) return 0;
+        if (q > (float)(2 * G - 1) + tol2) return 2 * G - 1;
+    }
     if (!(tol2 < 0.25f) || fr < tol2 || fr > 1.f - tol2) return half_key1_fast(p, mn, step, inv, G);
     return min(max((int)k, 0), 2 * G - 1);
 }
@@ -365,6 +375,9 @@ __device__ __forceinline__ void raise_err(Globals *g, unsigned f) {
 
 // kernel launch wrappers (bh_tree.cu, bh_force.cu, bh_misc.cu)
 namespace bh {
+cudaError_t tree_init(int *ctas);  // *ctas: the cluster's size on this device
+// create_tree of a small system (and its summarize) as one kernel
+cudaError_t launch_tree_cluster(const DevPlan &d, bool summary, cudaStream_t st);
 cudaError_t launch_prologue(const DevPlan &d, cudaStream_t st);
 cudaError_t launch_bbox(const DevPlan &d, cudaStream_t st);
 cudaError_t launch_place(const DevPlan &d, cudaStream_t st);
@@ -381,6 +394,7 @@ cudaError_t launch_pyramid(const DevPlan &d, cudaStream_t st, bool second = fals
 cudaError_t launch_force(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
                          const cudaEvent_t *ev = nullptr);
 cudaError_t launch_lists(const DevPlan &d, cudaStream_t st);
+int list_kernels(long long items_max);  // kernels launch_lists launches for a plan of at most so many items
 cudaError_t launch_fstream(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
                            const cudaEvent_t *ev = nullptr);
 cudaError_t fstream_init();

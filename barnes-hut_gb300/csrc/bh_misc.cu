@@ -317,9 +317,9 @@ cudaError_t launch_direct(const DevPlan &d, int sys, long long poff, long long n
     }
     for (long long t0 = 0; t0 < nt; t0 += (1LL << 28)) {
         const long long c = nt - t0 < (1LL << 28) ? nt - t0 : (1LL << 28), tiles = (c + T - 1) / T;
-        // chunks: four CTAs per SM, each with some work for every slice, within the scratch
+        // chunks: four CTAs per SM, at least two sources for every slice, within the scratch
         long long nchunk = (fill + tiles - 1) / tiles;
-        const long long most = n / (16LL * (DT * DR / T)), room = d.n_total / c;
+        const long long most = n / (2LL * (DT * DR / T)), room = d.n_total / c;
         nchunk = nchunk < most ? nchunk : most;
         nchunk = nchunk < room ? nchunk : room;
         if (nchunk < 1) nchunk = 1;

@@ -7,6 +7,8 @@
 //   (python-bh/barneshut/kernels/grid_decomposition/gpu/grid.py:15-76).
 // summarize = one kernel over tiles of leaf boxes: leaf moments, pyramid, records.
 //   Replaces g_summarize (gpu/grid.py:78-114) and calc_COM (internals/cloud.py:9-17).
+#include <cstring>
+
 #include "bh_internal.cuh"
 
 namespace bh {
@@ -32,6 +34,8 @@ __global__ void k_prologue(DevPlan d) {
         d.glob->far_pairs = 0;
         d.glob->corr_pairs = 0;
         d.glob->far_pids = 0;
+        d.glob->nbig = 0;
+        d.glob->nhuge = 0;
     }
     if (tid < d.nsys) {
         d.dyn[tid].bbmin[0] = d.dyn[tid].bbmin[1] = ~0ull;
@@ -44,8 +48,7 @@ __global__ void k_prologue(DevPlan d) {
 
 // One thread per system: the square bounding box (helpers/grid.py:10-26), its
 // box edge step = edge / G (base.py:233) and 1 / step, once per step.
-__device__ void bbox_finalize_sys(const DevPlan &d, int s) {
-    SysDyn &dy = d.dyn[s];
+__device__ void bbox_finalize_sys(const DevPlan &d, int s, SysDyn &dy) {
     double mnx = unord_bits(dy.bbmin[0]), mny = unord_bits(dy.bbmin[1]);
     double mxx = unord_bits(dy.bbmax[0]), mxy = unord_bits(dy.bbmax[1]);
     if (d.sys[s].fixed_grid) {  // part of a larger system: the whole system's extents
@@ -69,7 +72,7 @@ __device__ void bbox_finalize_sys(const DevPlan &d, int s) {
     dy.inv_step_f = __double2float_rn(dy.inv_step);
     if (step > 0.0 && isfinite(step)) {
         const double am = fmax(fabs(mnx), fabs(mny)), G = (double)d.sys[s].G;
-        const double tol = 4.0 * ((2.0 * am + G * step) / step + 2.0 * G) * 5.9604644775390625e-8;
+        const double tol = 4.0 * ((2.0 * am + G * step) * dy.inv_step + 2.0 * G) * 5.9604644775390625e-8;
         dy.key_tol = tol < 0.25 ? (float)tol : 1.f;
     } else {
         dy.key_tol = 1.f;  // the FP64 key for every particle
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(TPB) k_bbox(DevPlan d) {
     if (ticket != gridDim.x - 1) return;
     __threadfence();
     for (int s = threadIdx.x; s < d.nsys; s += TPB)
-        if (d.sys[s].n > 0) bbox_finalize_sys(d, s);
+        if (d.sys[s].n > 0) bbox_finalize_sys(d, s, d.dyn[s]);
     if (threadIdx.x == 0) d.glob->bbox_done = 0u;
 }
 
@@ -550,6 +553,100 @@ __global__ void __launch_bounds__(TPB) k_fill_items(DevPlan d) {
 constexpr int SITEM_WARPS = SITEM_TILE;  // one group per warp
 static_assert(MAX_TG * MAX_TG <= 64, "a lane holds at most two boxes of a group");
 
+// The items of one group, by a warp: the lane's boxes bi = lane, lane + 32 (bi = cx * TG + cy).
+struct GroupItems {
+    int kind[2], cnt[2], inc[2];  // the boxes' kinds, item counts and their inclusive prefixes in bi order
+    int4 qc[2];
+    int ns, nbox, tot0, total;    // sparse items, boxes, items of the first 32 boxes, all items
+};
+
+__device__ __forceinline__ void group_items(const DevPlan &d, long long g, GroupItems &r) {
+    const int lane = threadIdx.x & 31;
+    int nb[2] = {0, 0};
+    r.kind[0] = r.kind[1] = r.cnt[0] = r.cnt[1] = 0;
+    r.qc[0] = r.qc[1] = make_int4(0, 0, 0, 0);
+    r.nbox = 0;
+    int sparse = 0;
+    if (g < d.NG_total) {
+        const int s = find_seg(d.goff_tab, d.nsys, g);
+        const SysDesc &sd = d.sys[s];
+        const long long lg = g - sd.goff;
+        const int gi = (int)(lg / sd.NGs), gj = (int)(lg - (long long)gi * sd.NGs);
+        const int TG = sd.TG, tgs = __ffs(TG) - 1;
+        r.nbox = TG * TG;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int bi = lane + 32 * u;
+            const int cx = bi >> tgs, cy = bi & (TG - 1);
+            if (bi < r.nbox && gi * TG + cx < sd.G && gj * TG + cy < sd.G) {
+                const long long b = sd.boff + (long long)(gi * TG + cx) * sd.G + gj * TG + cy;
+                nb[u] = d.box_start[b + 1] - d.box_start[b];
+                r.kind[u] = box_item_kind(nb[u], d.dense_min, d.quad_min);
+                if (r.kind[u] == 2) {
+                    const int4 q = reinterpret_cast<const int4 *>(d.qcounts)[b];
+                    r.qc[u] = q;
+                    r.cnt[u] = sitem_count(q.x) + sitem_count(q.y) + sitem_count(q.z) + sitem_count(q.w);
+                } else if (r.kind[u] == 1) {
+                    r.cnt[u] = sitem_count(nb[u]);
+                } else {
+                    sparse += nb[u];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sparse += __shfl_xor_sync(0xffffffffu, sparse, o);
+    r.ns = sitem_count(sparse);
+    // prefixes of the boxes' item counts in bi order (lane's first box, then second)
+    r.inc[0] = r.cnt[0];
+    r.inc[1] = r.cnt[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y0 = __shfl_up_sync(0xffffffffu, r.inc[0], o), y1 = __shfl_up_sync(0xffffffffu, r.inc[1], o);
+        if (lane >= o) {
+            r.inc[0] += y0;
+            r.inc[1] += y1;
+        }
+    }
+    r.tot0 = __shfl_sync(0xffffffffu, r.inc[0], 31);
+    const int tot1 = __shfl_sync(0xffffffffu, r.inc[1], 31);
+    r.total = g < d.NG_total ? r.ns + r.tot0 + tot1 : 0;
+}
+
+// ... written from item `off` on
+__device__ __forceinline__ void group_items_write(const DevPlan &d, long long g, const GroupItems &r, int off) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) d.sitem_off[g] = off;
+    for (int k = lane; k < r.ns; k += 32) {  // the sparse boxes' items
+        d.sitem_group[off + k] = (int)g;
+        d.sitem_sub[off + k] = -1;
+        d.sitem_chunk[off + k] = make_int2(k, r.ns);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int bi = lane + 32 * u;
+        int o = off + r.ns + (u ? r.tot0 : 0) + r.inc[u] - r.cnt[u];
+        if (r.kind[u] == 1) {
+            const int nk = r.cnt[u];
+            for (int k = 0; k < nk; k++, o++) {
+                d.sitem_group[o] = (int)g;
+                d.sitem_sub[o] = bi;
+                d.sitem_chunk[o] = make_int2(k, nk);
+            }
+        } else if (r.kind[u] == 2) {
+            const int qv[4] = {r.qc[u].x, r.qc[u].y, r.qc[u].z, r.qc[u].w};
+            for (int q = 0; q < 4; q++) {
+                const int nk = sitem_count(qv[q]);
+                for (int k = 0; k < nk; k++, o++) {
+                    d.sitem_group[o] = (int)g;
+                    d.sitem_sub[o] = r.nbox + 4 * bi + q;
+                    d.sitem_chunk[o] = make_int2(k, nk);
+                }
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
     __shared__ int wtot[SITEM_WARPS], wpre[SITEM_WARPS];
     __shared__ int s_tile, s_excl;
@@ -563,52 +660,9 @@ __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
     __syncthreads();
     const int tile = s_tile;
     const long long g = (long long)tile * SITEM_TILE + warp;
-    // the lane's boxes bi = lane, lane + 32 of the group (bi = cx * TG + cy)
-    int nb[2] = {0, 0}, kind[2] = {0, 0}, cnt[2] = {0, 0};
-    int4 qc[2] = {make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0)};
-    int sparse = 0, nbox = 0;
-    if (g < d.NG_total) {
-        const int s = find_seg(d.goff_tab, d.nsys, g);
-        const SysDesc &sd = d.sys[s];
-        const long long lg = g - sd.goff;
-        const int gi = (int)(lg / sd.NGs), gj = (int)(lg - (long long)gi * sd.NGs);
-        const int TG = sd.TG, tgs = __ffs(TG) - 1;
-        nbox = TG * TG;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int bi = lane + 32 * u;
-            const int cx = bi >> tgs, cy = bi & (TG - 1);
-            if (bi < nbox && gi * TG + cx < sd.G && gj * TG + cy < sd.G) {
-                const long long b = sd.boff + (long long)(gi * TG + cx) * sd.G + gj * TG + cy;
-                nb[u] = d.box_start[b + 1] - d.box_start[b];
-                kind[u] = box_item_kind(nb[u], d.dense_min, d.quad_min);
-                if (kind[u] == 2) {
-                    qc[u] = reinterpret_cast<const int4 *>(d.qcounts)[b];
-                    cnt[u] = sitem_count(qc[u].x) + sitem_count(qc[u].y) + sitem_count(qc[u].z) + sitem_count(qc[u].w);
-                } else if (kind[u] == 1) {
-                    cnt[u] = sitem_count(nb[u]);
-                } else {
-                    sparse += nb[u];
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) sparse += __shfl_xor_sync(0xffffffffu, sparse, o);
-    const int ns = sitem_count(sparse);
-    // exclusive prefix of the boxes' item counts in bi order (lane's first box, then second)
-    int inc0 = cnt[0], inc1 = cnt[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y0 = __shfl_up_sync(0xffffffffu, inc0, o), y1 = __shfl_up_sync(0xffffffffu, inc1, o);
-        if (lane >= o) {
-            inc0 += y0;
-            inc1 += y1;
-        }
-    }
-    const int tot0 = __shfl_sync(0xffffffffu, inc0, 31), tot1 = __shfl_sync(0xffffffffu, inc1, 31);
-    const int gtot = g < d.NG_total ? ns + tot0 + tot1 : 0;
-    if (lane == 0) wtot[warp] = gtot;
+    GroupItems gi;
+    group_items(d, g, gi);
+    if (lane == 0) wtot[warp] = gi.total;
     __syncthreads();
     if (threadIdx.x < 32) {
         int v = lane < SITEM_WARPS ? wtot[lane] : 0, x = v;
@@ -630,37 +684,7 @@ __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
         }
     }
     __syncthreads();
-    if (g >= d.NG_total) return;
-    const int off = s_excl + wpre[warp];
-    if (lane == 0) d.sitem_off[g] = off;
-    for (int k = lane; k < ns; k += 32) {  // the sparse boxes' items
-        d.sitem_group[off + k] = (int)g;
-        d.sitem_sub[off + k] = -1;
-        d.sitem_chunk[off + k] = make_int2(k, ns);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const int bi = lane + 32 * u;
-        int o = off + ns + (u ? tot0 : 0) + (u ? inc1 : inc0) - cnt[u];
-        if (kind[u] == 1) {
-            const int nk = cnt[u];
-            for (int k = 0; k < nk; k++, o++) {
-                d.sitem_group[o] = (int)g;
-                d.sitem_sub[o] = bi;
-                d.sitem_chunk[o] = make_int2(k, nk);
-            }
-        } else if (kind[u] == 2) {
-            const int qv[4] = {qc[u].x, qc[u].y, qc[u].z, qc[u].w};
-            for (int q = 0; q < 4; q++) {
-                const int nk = sitem_count(qv[q]);
-                for (int k = 0; k < nk; k++, o++) {
-                    d.sitem_group[o] = (int)g;
-                    d.sitem_sub[o] = nbox + 4 * bi + q;
-                    d.sitem_chunk[o] = make_int2(k, nk);
-                }
-            }
-        }
-    }
+    if (g < d.NG_total) group_items_write(d, g, gi, s_excl + wpre[warp]);
 }
 
 // ------------------------------------------------------------------ scatter
@@ -689,6 +713,29 @@ __global__ void __launch_bounds__(TPB) k_perm(DevPlan d) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride)
         d.perm[quad_first(d, d.key[i]) + d.slot[i]] = (int)i;
+}
+
+// a stretch of n <= SEG_REG entries in a thread's registers
+__device__ __forceinline__ void seg_thread(int *p, int n) {
+    int v[SEG_REG];
+#pragma unroll
+    for (int k = 0; k < SEG_REG; k++) v[k] = k < n ? p[k] : 0x7FFFFFFF;
+    bool sorted = true;  // (padding sorts after every index)
+#pragma unroll
+    for (int k = 0; k + 1 < SEG_REG; k++) sorted &= v[k] <= v[k + 1];
+    if (sorted) return;
+    // odd-even transposition network: SEG_REG rounds sort SEG_REG entries
+#pragma unroll
+    for (int r = 0; r < SEG_REG; r++)
+#pragma unroll
+        for (int k = r & 1; k + 1 < SEG_REG; k += 2) {
+            const int lo = min(v[k], v[k + 1]), hi = max(v[k], v[k + 1]);
+            v[k] = lo;
+            v[k + 1] = hi;
+        }
+#pragma unroll
+    for (int k = 0; k < SEG_REG; k++)
+        if (k < n) p[k] = v[k];
 }
 
 __global__ void __launch_bounds__(TPB) k_segsort(DevPlan d) {
@@ -722,25 +769,7 @@ __global__ void __launch_bounds__(TPB) k_segsort(DevPlan d) {
             d.bigseg[k] = make_int2(s0, n);
             continue;
         }
-        int v[SEG_REG];
-#pragma unroll
-        for (int k = 0; k < SEG_REG; k++) v[k] = k < n ? d.perm[s0 + k] : 0x7FFFFFFF;
-        bool sorted = true;  // (padding sorts after every index)
-#pragma unroll
-        for (int k = 0; k + 1 < SEG_REG; k++) sorted &= v[k] <= v[k + 1];
-        if (sorted) continue;
-        // odd-even transposition network: SEG_REG rounds sort SEG_REG entries
-#pragma unroll
-        for (int r = 0; r < SEG_REG; r++)
-#pragma unroll
-            for (int k = r & 1; k + 1 < SEG_REG; k += 2) {
-                const int lo = min(v[k], v[k + 1]), hi = max(v[k], v[k + 1]);
-                v[k] = lo;
-                v[k + 1] = hi;
-            }
-#pragma unroll
-        for (int k = 0; k < SEG_REG; k++)
-            if (k < n) d.perm[s0 + k] = v[k];
+        seg_thread(d.perm + s0, n);
     }
 }
 
@@ -796,6 +825,65 @@ __device__ __forceinline__ void seg_regs(int *p, int n) {
         if (32 * r + lane < n) p[32 * r + lane] = v[r];
 }
 
+// Ascending sort of src[0 .. n) by a CTA of NT threads: four stable 8-bit radix passes src -> dst ->
+// src -> dst -> src.
+template <int NT>
+struct RadixScratch {
+    int hist[256], base[256], run[256], wcnt[NT / 32][256];
+};
+
+template <int NT>
+__device__ void cta_radix_sort(int *src, int *dst, int n, RadixScratch<NT> &rs) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int pass = 0; pass < 4; pass++) {
+        const int sh = 8 * pass;
+        for (int k = tid; k < 256; k += NT) {
+            rs.hist[k] = 0;
+            rs.run[k] = 0;
+        }
+        __syncthreads();
+        for (int k = tid; k < n; k += NT) atomicAdd(&rs.hist[(src[k] >> sh) & 255], 1);
+        __syncthreads();
+        if (tid == 0) {
+            int acc = 0;
+            for (int k = 0; k < 256; k++) {
+                rs.base[k] = acc;
+                acc += rs.hist[k];
+            }
+        }
+        __syncthreads();
+        for (int c0 = 0; c0 < n; c0 += NT) {
+            const int k = c0 + tid;
+            const bool ok = k < n;
+            const int v = ok ? src[k] : 0;
+            const int dg = ok ? (v >> sh) & 255 : 256 + lane;  // invalid lanes match nobody
+            for (int q = tid; q < (NT / 32) * 256; q += NT) (&rs.wcnt[0][0])[q] = 0;
+            __syncthreads();
+            const unsigned peers = __match_any_sync(0xffffffffu, dg);
+            const int rank = __popc(peers & ((1u << lane) - 1u));
+            if (ok && rank == 0) rs.wcnt[warp][dg] = __popc(peers);
+            __syncthreads();
+            if (ok) {
+                int pos = rs.base[dg] + rs.run[dg] + rank;
+                for (int q = 0; q < warp; q++) pos += rs.wcnt[q][dg];
+                dst[pos] = v;
+            }
+            __syncthreads();
+            for (int q = tid; q < 256; q += NT) {
+                int t = 0;
+                for (int ww = 0; ww < NT / 32; ww++) t += rs.wcnt[ww][q];
+                rs.run[q] += t;
+            }
+            __syncthreads();
+        }
+        int *t = src;
+        src = dst;
+        dst = t;
+        __threadfence_block();
+        __syncthreads();
+    }
+}
+
 // Long stretches.  Up to SEG_LANES entries a warp sorts in its registers (batches of small boxes in
 // file order have most of theirs here: 27.3M particles 670 -> 344 us, against the shared-memory
 // network), up to SEG_WARP in its slice of shared memory, longer ones a CTA.
@@ -803,7 +891,7 @@ constexpr int SEG_LANES = 256;
 
 __global__ void __launch_bounds__(TPB) k_segsort_big(DevPlan d) {
     __shared__ int sv[TPB / 32][SEG_WARP];
-    __shared__ int hist[256], base[256], run[256], wcnt[TPB / 32][256];
+    __shared__ RadixScratch<TPB> rs;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // stretches of SEG_REG + 1 .. SEG_WARP entries: a warp each; beyond SEG_LANES a bitonic network
     // over the next power of two (padded with INT_MAX) in the warp's slice of shared memory
@@ -852,60 +940,11 @@ __global__ void __launch_bounds__(TPB) k_segsort_big(DevPlan d) {
         for (int k = lane; k < n; k += 32) d.perm[s0 + k] = w[k];
         __syncwarp();
     }
-    // longer stretches: a CTA each, four stable 8-bit radix passes perm -> slot -> perm -> slot
-    // -> perm (the slot array is dead once k_perm has run)
+    // longer stretches: a CTA each
     const unsigned nhuge = d.glob->nhuge;
     for (unsigned b = blockIdx.x; b < nhuge; b += gridDim.x) {
         const int2 sg = d.bigseg[d.bigseg_cap - 1 - b];
-        const int s0 = sg.x, n = sg.y;
-        int *src = d.perm + s0, *dst = d.slot + s0;
-        for (int pass = 0; pass < 4; pass++) {
-            const int sh = 8 * pass;
-            for (int k = tid; k < 256; k += TPB) {
-                hist[k] = 0;
-                run[k] = 0;
-            }
-            __syncthreads();
-            for (int k = tid; k < n; k += TPB) atomicAdd(&hist[(src[k] >> sh) & 255], 1);
-            __syncthreads();
-            if (tid == 0) {
-                int acc = 0;
-                for (int k = 0; k < 256; k++) {
-                    base[k] = acc;
-                    acc += hist[k];
-                }
-            }
-            __syncthreads();
-            for (int c0 = 0; c0 < n; c0 += TPB) {
-                const int k = c0 + tid;
-                const bool ok = k < n;
-                const int v = ok ? src[k] : 0;
-                const int dg = ok ? (v >> sh) & 255 : 256 + lane;  // invalid lanes match nobody
-                for (int q = tid; q < (TPB / 32) * 256; q += TPB) (&wcnt[0][0])[q] = 0;
-                __syncthreads();
-                const unsigned peers = __match_any_sync(0xffffffffu, dg);
-                const int rank = __popc(peers & ((1u << lane) - 1u));
-                if (ok && rank == 0) wcnt[warp][dg] = __popc(peers);
-                __syncthreads();
-                if (ok) {
-                    int pos = base[dg] + run[dg] + rank;
-                    for (int q = 0; q < warp; q++) pos += wcnt[q][dg];
-                    dst[pos] = v;
-                }
-                __syncthreads();
-                for (int q = tid; q < 256; q += TPB) {
-                    int t = 0;
-                    for (int ww = 0; ww < TPB / 32; ww++) t += wcnt[ww][q];
-                    run[q] += t;
-                }
-                __syncthreads();
-            }
-            int *t = src;
-            src = dst;
-            dst = t;
-            __threadfence_block();
-            __syncthreads();
-        }
+        cta_radix_sort<TPB>(d.perm + sg.x, d.slot + sg.x, sg.y, rs);
     }
 }
 
@@ -1153,15 +1192,51 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float x) {
     s = t;
 }
 
-// leaves_given: the leaf moments are already in d.mom (bh_set_leaf_moments); build the rest.
+// The moments of box lb of a system into m (6 values) and mom: a box inside one chunk has them from
+// the chunk's sums; a box over several chunks adds its partials in chunk order.
 template <bool SECOND>
-__global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int leaves_given) {
+__device__ __forceinline__ void leaf_sum(const DevPlan &d, const SysDesc &sd, long long lb, double *m) {
+    constexpr int NM = SECOND ? 6 : 3;
+    const int i0 = d.box_start[sd.boff + lb], i1 = d.box_start[sd.boff + lb + 1];
+    double *mb = d.mom + 6 * (sd.coff + lb);
+    if (i1 == i0) {  // empty: zeros
+#pragma unroll
+        for (int q = 0; q < 6; q++) m[q] = mb[q] = 0.0;
+        return;
+    }
+    const long long c0 = i0 >> 5, c1 = (long long)(i1 - 1) >> 5;
+    if (c0 == c1) {
+#pragma unroll
+        for (int q = 0; q < 6; q++) m[q] = mb[q];
+        return;
+    }
+    float sm_[6], cc_[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        sm_[q] = q < NM ? d.leafpart[12 * c0 + 6 + q] : 0.f;
+        cc_[q] = 0.f;
+    }
+    for (long long c = c0 + 1; c <= c1; c++)
+#pragma unroll
+        for (int q = 0; q < NM; q++) kahan_add(sm_[q], cc_[q], d.leafpart[12 * c + q]);
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        const double v = f32_to_f64(__fsub_rn(sm_[q], cc_[q]));
+        m[q] = v;
+        mb[q] = v;
+    }
+}
+
+// One tile by a CTA of NT threads.  leaf_records: also the records of the boxes.  leaves_given: the leaf moments are already in d.mom
+// (bh_set_leaf_moments); build the rest.  cm: the tile's cells, level by level (SUM_CELLS x 6); chm:
+// shifted child moments, 64 cells x 4 children (x 6).
+template <bool SECOND, int NT>
+__device__ __forceinline__ void summarize_tile(const DevPlan &d, long long t, int leaves_given, bool leaf_records, double *cm,
+                                               double *chm) {
     constexpr int NM = SECOND ? 6 : 3;  // moments a pyramid cell carries
-    __shared__ double cm[SUM_CELLS * 6];  // the tile's cells, level by level
-    __shared__ double chm[4 * 64 * 6];    // shifted child moments: 64 cells x 4 children
     const int tid = threadIdx.x;
     const int loff[5] = {0, 256, 320, 336, 340};
-    for (long long t = blockIdx.x; t < d.T_total; t += gridDim.x) {
+    {
         const int s = find_seg(d.toff_tab, d.nsys, t);
         const SysDesc &sd = d.sys[s];
         const double step = d.dyn[s].step;
@@ -1170,7 +1245,7 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
         const int nbx = min(SUM_TILE, G - bx0), nby = min(SUM_TILE, G - by0);
         const int lmax = min(SUM_UP - 1, sd.L - 1);  // the tile's top level
         // ---- level 0: the tile's boxes (zeros outside the grid)
-        for (int k = tid; k < 6 * SUM_TILE * SUM_TILE; k += SUM_THREADS) {
+        for (int k = tid; k < 6 * SUM_TILE * SUM_TILE; k += NT) {
             const int box = k / 6, cx = box / SUM_TILE, cy = box - cx * SUM_TILE;
             double v = 0.0;
             if (leaves_given && cx < nbx && cy < nby)
@@ -1182,38 +1257,10 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
             // a box inside one chunk has its moments from the chunk's sums; a box over several
             // chunks adds its partials in chunk order (the first chunk's tail, whole middle
             // chunks, the last chunk's head) and writes the sum to mom, as an empty box its zeros
-            for (int k = tid; k < SUM_TILE * SUM_TILE; k += SUM_THREADS) {
+            for (int k = tid; k < SUM_TILE * SUM_TILE; k += NT) {
                 const int cx = k / SUM_TILE, cy = k - cx * SUM_TILE;
                 if (cx >= nbx || cy >= nby) continue;
-                const long long lb = (long long)(bx0 + cx) * G + (by0 + cy);
-                const int i0 = d.box_start[sd.boff + lb], i1 = d.box_start[sd.boff + lb + 1];
-                double *mb = d.mom + 6 * (sd.coff + lb);
-                if (i1 == i0) {  // empty: zeros
-#pragma unroll
-                    for (int q = 0; q < 6; q++) mb[q] = 0.0;
-                    continue;
-                }
-                const long long c0 = i0 >> 5, c1 = (long long)(i1 - 1) >> 5;
-                if (c0 == c1) {
-#pragma unroll
-                    for (int q = 0; q < 6; q++) cm[6 * k + q] = mb[q];
-                    continue;
-                }
-                float sm_[6], cc_[6];
-#pragma unroll
-                for (int q = 0; q < 6; q++) {
-                    sm_[q] = q < NM ? d.leafpart[12 * c0 + 6 + q] : 0.f;
-                    cc_[q] = 0.f;
-                }
-                for (long long c = c0 + 1; c <= c1; c++)
-#pragma unroll
-                    for (int q = 0; q < NM; q++) kahan_add(sm_[q], cc_[q], d.leafpart[12 * c + q]);
-#pragma unroll
-                for (int q = 0; q < 6; q++) {
-                    const double v = f32_to_f64(__fsub_rn(sm_[q], cc_[q]));
-                    cm[6 * k + q] = v;
-                    mb[q] = v;
-                }
+                leaf_sum<SECOND>(d, sd, (long long)(bx0 + cx) * G + (by0 + cy), cm + 6 * k);
             }
             __syncthreads();
         }
@@ -1223,7 +1270,7 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
             const int nl = SUM_TILE >> l, nc = nl << 1;  // cells per side at l and l - 1
             const int gl = sd.lvg[l], gc = sd.lvg[l - 1];
             const int I0 = bx0 >> l, J0 = by0 >> l;
-            for (int t = tid; t < 4 * nl * nl; t += SUM_THREADS) {
+            for (int t = tid; t < 4 * nl * nl; t += NT) {
                 const int cell = t >> 2, a = (t >> 1) & 1, b = t & 1;
                 const int ci = cell / nl, cj = cell - ci * nl;
                 const bool has = 2 * (I0 + ci) + a < gc && 2 * (J0 + cj) + b < gc;
@@ -1231,7 +1278,7 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
                                     l, step, chm + 6 * t);
             }
             __syncthreads();
-            for (int c = tid; c < nl * nl; c += SUM_THREADS) {
+            for (int c = tid; c < nl * nl; c += NT) {
                 const int ci = c / nl, cj = c - ci * nl;
                 const bool inside = I0 + ci < gl && J0 + cj < gl;
                 double p[6];
@@ -1242,16 +1289,18 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
                     const long long cc = sd.coff + sd.lvoff[l] + (long long)(I0 + ci) * gl + (J0 + cj);
 #pragma unroll
                     for (int k = 0; k < NM; k++) d.mom[6 * cc + k] = p[k];
-                    cell_record<SECOND>(d, cc, l, step, p);
                 }
             }
             __syncthreads();
         }
-        // ---- records of the tile's boxes
-        for (int k = tid; k < SUM_TILE * SUM_TILE; k += SUM_THREADS) {
-            const int cx = k / SUM_TILE, cy = k - cx * SUM_TILE;
-            if (cx >= nbx || cy >= nby) continue;
-            cell_record<SECOND>(d, sd.coff + (long long)(bx0 + cx) * G + (by0 + cy), 0, step, cm + 6 * k);
+        // ---- records of the tile's cells, all levels at once (a record is a chain of FP64 operations)
+        for (int k = leaf_records ? tid : 256 + tid; k < SUM_CELLS; k += NT) {
+            const int l = k < 256 ? 0 : k < 320 ? 1 : k < 336 ? 2 : k < 340 ? 3 : 4;
+            if (l > lmax) continue;
+            const int nl = SUM_TILE >> l, c = k - loff[l], ci = c / nl, cj = c - ci * nl;
+            const int gl = sd.lvg[l], I = (bx0 >> l) + ci, J = (by0 >> l) + cj;
+            if (I < gl && J < gl)
+                cell_record<SECOND>(d, sd.coff + sd.lvoff[l] + (long long)I * gl + J, l, step, cm + 6 * k);
         }
         // ---- above the tiles: the tile's top cell arrives at its parent; the CTA whose child
         // arrives last builds the parent (children in (0, 0), (0, 1), (1, 0), (1, 1) order, the
@@ -1298,7 +1347,366 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
     }
 }
 
+template <bool SECOND>
+__global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int leaves_given) {
+    __shared__ double cm[SUM_CELLS * 6];
+    __shared__ double chm[4 * 64 * 6];
+    for (long long t = blockIdx.x; t < d.T_total; t += gridDim.x)
+        summarize_tile<SECOND, SUM_THREADS>(d, t, leaves_given, true, cm, chm);
+}
+
+// ------------------------------------------------------------------ small systems
+// create_tree (and, fused into a step, summarize) of one small system as one kernel: a cluster of
+// 16 CTAs runs the phases of k_prologue, k_bbox, k_place, the box scan, k_perm, k_segsort and
+// k_gather one after another with a cluster barrier between them, and makes the work items.  Bound: latency -- a phase is one or two dependent loads for every thread, and a
+// kernel of its own costs three to five microseconds, its launch and its ramp, where a barrier costs
+// half of one.  Every result is the same bits: the phases are the same arithmetic over the same chunks,
+// and what depends on atomics (slots) is put in input order as in k_segsort.  10,000 particles on
+// 16 x 16 boxes, a step: @CL10A@ -> @CL10B@ us; beyond CL_MAX_N particles 16 SMs' share of the
+// memory system costs more than the launches (@CLMAX@).
+constexpr int CL_THREADS = 1024;
+struct ClusterSmem {
+    int start[CL_MAX_BOXES + 1];  // box_start
+    SysDyn dyn;
+    double org[2][CL_MAX_SIDE];  // box origins
+    unsigned long long red[4][CL_THREADS / 32], ext[4];
+    unsigned long long items;  // work items of the CTA's groups
+    int scan[32], wtot[32], base;
+    int nbig;
+    union {
+        struct {
+            int2 big[2048];  // the CTA's long quadrants
+            RadixScratch<CL_THREADS> rs;
+        } sort;
+        struct {
+            double cm[SUM_CELLS * 6], chm[4 * 64 * 6];
+        } sum;
+    } u;
+};
+static_assert(4 * CL_MAX_BOXES <= 2048 * 8 && CL_MAX_SIDE * CL_MAX_SIDE == CL_MAX_BOXES, "eight CTAs or more: 2,048 quadrants each at most");
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    cluster_arrive();
+    cluster_wait();
+}
+// a 64-bit value in another CTA's shared memory
+__device__ __forceinline__ unsigned long long ld_cluster(const unsigned long long *p, unsigned rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    unsigned long long v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(r) : "memory");
+    return v;
+}
+
+// Work items of the groups [g0, g1) by one CTA, from item `base` on; returns their number.  WRITE:
+// write them (the number alone needs no base).
+// Walking plan: k_group_items, its scan and k_fill_items.
+template <bool WRITE>
+__device__ int cluster_walk_items(const DevPlan &d, ClusterSmem &sm, int g0, int g1, int base) {
+    const SysDesc &sd = d.sys[0];
+    int sum = 0;
+    for (int k0 = g0; k0 < g1; k0 += CL_THREADS) {
+        const int g = k0 + threadIdx.x;
+        int cnt = 0;
+        if (g < g1) {
+            const int gi = g / sd.NGs, gj = g - gi * sd.NGs;
+            const int gx0 = gi * sd.TG, gy0 = gj * sd.TG, gx1 = min(sd.G, gx0 + sd.TG), gy1 = min(sd.G, gy0 + sd.TG);
+            int nt = 0;
+            for (int c = gx0; c < gx1; c++) nt += sm.start[c * sd.G + gy1] - sm.start[c * sd.G + gy0];
+            cnt = (nt + d.chunk - 1) / d.chunk;
+        }
+        int tot;
+        const int off = base + sum + block_excl_scan(cnt, sm.scan, &tot);
+        if (WRITE && g < g1) {
+            d.item_cnt[g] = cnt;
+            d.item_off[g] = off;
+            for (int k = 0; k < cnt; k++) d.item_group[off + k] = g;
+        }
+        sum += tot;
+    }
+    return sum;
+}
+
+// List streaming: k_sitems, a warp per group, a round per 32 groups.
+template <bool WRITE>
+__device__ int cluster_stream_items(const DevPlan &d, ClusterSmem &sm, int g0, int g1, int base) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int sum = 0;
+    for (int k0 = g0; k0 < g1; k0 += CL_THREADS / 32) {
+        const int g = k0 + warp;
+        GroupItems gi;
+        group_items(d, g < g1 ? g : d.NG_total, gi);
+        if (lane == 0) sm.wtot[warp] = gi.total;
+        __syncthreads();
+        if (warp == 0) {
+            const int v = sm.wtot[lane];
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            sm.wtot[lane] = x - v;
+            if (lane == 31) sm.base = x;
+        }
+        __syncthreads();
+        if (WRITE && g < g1) group_items_write(d, g, gi, base + sum + sm.wtot[warp]);
+        sum += sm.base;
+        __syncthreads();
+    }
+    return sum;
+}
+
+__global__ void __launch_bounds__(CL_THREADS, 1) k_tree_cluster(DevPlan d, int summary) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ClusterSmem &sm = *reinterpret_cast<ClusterSmem *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = blockIdx.x, nct = gridDim.x;  // (the grid is one cluster)
+    const int gt = rank * CL_THREADS + tid, GT = nct * CL_THREADS;
+    const SysDesc &sd = d.sys[0];
+    const int n = (int)d.n_total, G = sd.G, B = G * G;
+    const unsigned epoch = d.glob->epoch + 1;  // (advanced below, once every CTA has read it)
+    const int cur = epoch & 1, nxt = cur ^ 1;
+    const double *X = d.X[cur], *Y = d.Y[cur];
+    // ---- empty histograms; extents of the CTA's particles
+    for (int b = gt; b < B; b += GT) reinterpret_cast<int4 *>(d.qcounts)[b] = make_int4(0, 0, 0, 0);
+    unsigned long long e[4] = {~0ull, ~0ull, 0ull, 0ull};
+    for (int i = gt; i < n; i += GT) {
+        minmax_ord(ord_bits(X[i]), e[0], e[2]);
+        minmax_ord(ord_bits(Y[i]), e[1], e[3]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, e[q], o);
+            e[q] = q < 2 ? (v < e[q] ? v : e[q]) : (v > e[q] ? v : e[q]);
+        }
+        if (lane == 0) sm.red[q][warp] = e[q];
+    }
+    __syncthreads();
+    if (warp < 4) {
+        unsigned long long v = sm.red[warp][lane];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = warp < 2 ? (w < v ? w : v) : (w > v ? w : v);
+        }
+        if (lane == 0) sm.ext[warp] = v;
+    }
+    if (tid == 0) sm.nbig = 0;
+    cluster_sync();
+    // ---- the square box, by every CTA for itself; CTA 0 publishes it
+    if (warp == 0) {
+        unsigned long long v = ld_cluster(&sm.ext[lane >> 3], lane & 7);
+        if (nct > 8) {  // 8 or 16 CTAs
+            const unsigned long long w = ld_cluster(&sm.ext[lane >> 3], 8 + (lane & 7));
+            v = lane < 16 ? (w < v ? w : v) : (w > v ? w : v);
+        }
+#pragma unroll
+        for (int o = 4; o; o >>= 1) {
+            const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = lane < 16 ? (w < v ? w : v) : (w > v ? w : v);
+        }
+        if ((lane & 7) == 0) (lane < 16 ? sm.dyn.bbmin : sm.dyn.bbmax)[(lane >> 3) & 1] = v;
+        __syncwarp();
+        if (lane == 0) {
+            bbox_finalize_sys(d, 0, sm.dyn);
+            if (rank == 0) {
+                d.dyn[0] = sm.dyn;
+                d.glob->epoch = epoch;
+                d.glob->near_pairs = 0;
+                d.glob->far_pairs = 0;
+                d.glob->corr_pairs = 0;
+                d.glob->far_pids = 0;
+            }
+        }
+    }
+    __syncthreads();
+    const SysDyn &dy = sm.dyn;
+    if (tid < 2 * G) sm.org[tid >= G][tid >= G ? tid - G : tid] = box_origin(tid >= G ? dy.miny : dy.minx, tid >= G ? tid - G : tid, dy.step);
+    // ---- keys and slots (a run of equal keys in a warp shares an addition)
+    for (int i0 = gt - lane; i0 < n; i0 += GT) {
+        const int i = i0 + lane;
+        int key = -1;
+        if (i < n) {
+            const double x = X[i], y = Y[i];
+            const unsigned hx = (unsigned)(__double_as_longlong(x) >> 52) & 0x7FFu;
+            const unsigned hy = (unsigned)(__double_as_longlong(y) >> 52) & 0x7FFu;
+            if (hx == 0x7FFu || hy == 0x7FFu) raise_err(d.glob, 1u /*BH_DEV_NAN_POSITION*/);
+            const int k2x = half_key1_f32(x, dy.minx, dy.step, dy.inv_step, dy.minx_f, dy.inv_step_f, dy.key_tol, G);
+            const int k2y = half_key1_f32(y, dy.miny, dy.step, dy.inv_step, dy.miny_f, dy.inv_step_f, dy.key_tol, G);
+            key = 4 * ((k2x >> 1) * G + (k2y >> 1)) + (k2x & 1) * 2 + (k2y & 1);
+        }
+        const int kp = __shfl_up_sync(0xffffffffu, key, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != kp);
+        const int h = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));            // the run's first lane
+        const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+        const int len = later ? __ffs(later) : 32 - lane;                          // (at its first lane)
+        int s0 = 0;
+        if (lane == h && key >= 0) s0 = atomicAdd(&d.qcounts[key], len);
+        s0 = __shfl_sync(0xffffffffu, s0, h);
+        if (i < n) {
+            d.key[i] = key;
+            d.slot[i] = s0 + lane - h;
+        }
+    }
+    cluster_sync();
+    // ---- box scan, by every CTA for itself; CTA 0 publishes it
+    {
+        constexpr int PER = (CL_MAX_BOXES + CL_THREADS - 1) / CL_THREADS;
+        int v[PER], sum = 0;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int b = tid * PER + q;
+            int4 c = make_int4(0, 0, 0, 0);
+            if (b < B) c = reinterpret_cast<const int4 *>(d.qcounts)[b];
+            v[q] = c.x + c.y + c.z + c.w;
+            sum += v[q];
+        }
+        int pre = block_excl_scan(sum, sm.scan, nullptr);
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int b = tid * PER + q;
+            if (b <= B) {  // (past the last box: the total)
+                sm.start[b] = pre;
+                if (rank == 0) d.box_start[b] = pre;
+            }
+            pre += v[q];
+        }
+        if (tid == CL_THREADS - 1 && PER * CL_THREADS == B) {
+            sm.start[B] = pre;
+            if (rank == 0) d.box_start[B] = pre;
+        }
+    }
+    __syncthreads();
+    // ---- permutation
+    auto first = [&](int key4) {
+        const int4 qc = reinterpret_cast<const int4 *>(d.qcounts)[key4 >> 2];
+        const int quad = key4 & 3;
+        return sm.start[key4 >> 2] + (quad > 0 ? qc.x : 0) + (quad > 1 ? qc.y : 0) + (quad > 2 ? qc.z : 0);
+    };
+    for (int i = gt; i < n; i += GT) d.perm[first(d.key[i]) + d.slot[i]] = i;
+    cluster_sync();
+    // ---- the CTA's groups (CTA 0, which has a pyramid to build, takes none) and their work items
+    const int ng = (int)d.NG_total, per = (ng + nct - 2) / (nct - 1);
+    const int ig0 = min(ng, max(0, rank - 1) * per), ig1 = rank == 0 ? ig0 : min(ng, rank * per);
+    {
+        const int c = d.stream ? cluster_stream_items<false>(d, sm, ig0, ig1, 0) : cluster_walk_items<false>(d, sm, ig0, ig1, 0);
+        if (tid == 0) sm.items = (unsigned long long)c;
+    }
+    // ---- each quadrant's stretch in input order
+    for (int q = tid * nct + rank; q < 4 * B; q += GT) {  // (every CTA takes its share of a few)
+        const int cnt = d.qcounts[q];
+        if (cnt < 2) continue;
+        const int s0 = first(q);
+        if (cnt > SEG_REG) {
+            sm.u.sort.big[atomicAdd(&sm.nbig, 1)] = make_int2(s0, cnt);
+            continue;
+        }
+        seg_thread(d.perm + s0, cnt);
+    }
+    __syncthreads();
+    {
+        const int nbig = sm.nbig;
+        for (int k = warp; k < nbig; k += CL_THREADS / 32) {
+            const int2 sg = sm.u.sort.big[k];
+            if (sg.y > SEG_LANES) continue;
+            if (sg.y <= 32) seg_regs<1>(d.perm + sg.x, sg.y);
+            else if (sg.y <= 64) seg_regs<2>(d.perm + sg.x, sg.y);
+            else if (sg.y <= 128) seg_regs<4>(d.perm + sg.x, sg.y);
+            else seg_regs<8>(d.perm + sg.x, sg.y);
+        }
+        for (int k = 0; k < nbig; k++) {
+            const int2 sg = sm.u.sort.big[k];
+            if (sg.y > SEG_LANES) cta_radix_sort<CL_THREADS>(d.perm + sg.x, d.slot + sg.x, sg.y, sm.u.sort.rs);
+        }
+    }
+    cluster_sync();
+    int item_base = 0;  // (every thread)
+    for (int r = 0; r < rank; r++) item_base += (int)ld_cluster(&sm.items, r);
+    // ---- gather the state, sum the leaves
+    {
+        for (int w0 = gt - lane; w0 < n; w0 += GT) {
+            const int t = w0 + lane;
+            int key = -1;
+            float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (t < n) {
+                const int i = d.perm[t];
+                key = d.key[i] >> 2;
+                const double x = X[i], y = Y[i], m = d.M[cur][i];
+                const int kx = key / G, ky = key - kx * G;
+                d.X[nxt][t] = x;
+                d.Y[nxt][t] = y;
+                d.VX[nxt][t] = d.VX[cur][i];
+                d.VY[nxt][t] = d.VY[cur][i];
+                d.M[nxt][t] = m;
+                d.PID[nxt][t] = d.PID[cur][i];
+                const float ox = f64_to_f32_rn(__dsub_rn(x, sm.org[0][kx]));
+                const float oy = f64_to_f32_rn(__dsub_rn(y, sm.org[1][ky]));
+                const float mf = f64_to_f32_rn(m);
+                d.PD[2 * t] = make_float4(ox, ox, oy, oy);
+                d.PD[2 * t + 1] = make_float4(mf, mf, __int_as_float(t), __int_as_float((kx << 16) | ky));
+                d.skey[t] = key;
+                leaf_terms<false>(ox, oy, mf, v);
+            }
+            leaf_chunk<false>(d, w0 >> 5, key, v);
+        }
+    }
+    cluster_sync();
+    if (summary) {
+        // ---- summarize: the boxes' moments and records over all CTAs, then the tiles' pyramids
+        for (int b = tid * nct + rank; b < B; b += GT) {
+            double m[6];
+            leaf_sum<false>(d, sd, b, m);
+            cell_record<false>(d, sd.coff + b, 0, dy.step, m);
+        }
+        cluster_sync();
+        for (int t = rank; t < (int)d.T_total; t += nct)
+            summarize_tile<false, CL_THREADS>(d, t, 1, false, sm.u.sum.cm, sm.u.sum.chm);
+    }
+    // ---- the work items, which nothing here waits for
+    if (d.stream) cluster_stream_items<true>(d, sm, ig0, ig1, item_base);
+    else cluster_walk_items<true>(d, sm, ig0, ig1, item_base);
+    if (rank == nct - 1 && tid == 0) (d.stream ? d.sitem_off : d.item_off)[ng] = item_base + (int)sm.items;
+}
+
 // ------------------------------------------------------------------ launches
+// Launch of k_tree_cluster: 16 CTAs where the device keeps a cluster that large, else 8.
+static cudaError_t cluster_config(cudaLaunchConfig_t &c, cudaLaunchAttribute &a, int ctas, cudaStream_t st) {
+    memset(&c, 0, sizeof(c));
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = ctas;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    c.gridDim = dim3(ctas);
+    c.blockDim = dim3(CL_THREADS);
+    c.dynamicSmemBytes = sizeof(ClusterSmem);
+    c.stream = st;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaSuccess;
+}
+cudaError_t tree_init(int *ctas) {
+    cudaError_t e = cudaFuncSetAttribute(k_tree_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem));
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_tree_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t c;
+    cudaLaunchAttribute a;
+    cluster_config(c, a, 16, nullptr);
+    int fit = 0;
+    *ctas = cudaOccupancyMaxActiveClusters(&fit, k_tree_cluster, &c) == cudaSuccess && fit > 0 ? 16 : 8;
+    cudaGetLastError();
+    return cudaSuccess;
+}
+cudaError_t launch_tree_cluster(const DevPlan &d, bool summary, cudaStream_t st) {
+    cudaLaunchConfig_t c;
+    cudaLaunchAttribute a;
+    cluster_config(c, a, d.cl_ctas, st);
+    return cudaLaunchKernelEx(&c, k_tree_cluster, d, summary ? 1 : 0);
+}
 cudaError_t launch_prologue(const DevPlan &d, cudaStream_t st) {
     long long n = d.B_total > d.nsys ? d.B_total : d.nsys;
     k_prologue<<<grid_for(n, TPB, d.nsm * 16LL), TPB, 0, st>>>(d);
@@ -1343,8 +1751,6 @@ cudaError_t launch_items(const DevPlan &d, cudaStream_t st) {
 }
 cudaError_t launch_scatter(const DevPlan &d, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(&d.glob->nbig, 0, 2 * sizeof(unsigned), st);  // nbig, nhuge
-    if (e != cudaSuccess) return e;
     k_perm<<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
     k_segsort<<<grid_for(4 * d.B_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
     k_segsort_big<<<(unsigned)(d.nsm * 4), TPB, 0, st>>>(d);
