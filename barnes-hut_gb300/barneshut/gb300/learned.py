@@ -37,6 +37,8 @@ def _lib():
         L.bh_mlp_train_batch.restype = i
         L.bh_mlp_adam.argtypes = [vp, vp, vp, vp, i, f, vp]
         L.bh_mlp_adam.restype = i
+        L.bh_mlp_adam_pack.argtypes = [vp, vp, vp, vp, i, f, vp, vp]
+        L.bh_mlp_adam_pack.restype = i
         L._mlp_typed = True
     return L
 
@@ -84,18 +86,18 @@ class LearnedCorrection:
         self.pack()
 
     def _st(self):
-        return ctypes.c_void_p(self.torch.cuda.current_stream(self.device).cuda_stream)
+        return native.current_stream_ptr(self.device)
 
     def _img(self):
-        off = (-self.image.data_ptr()) % 256
-        return ctypes.c_void_p(self.image.data_ptr() + off)
+        p = self.image.data_ptr()
+        return p + (-p) % 256
 
     def _check(self, rc, what):
         if rc != 0:
             raise native.BHError(rc, what)
 
     def pack(self):
-        self._check(self.L.bh_mlp_pack(ctypes.c_void_p(self.params.data_ptr()), self._img(),
+        self._check(self.L.bh_mlp_pack(self.params.data_ptr(), self._img(),
                                        self._st()), "bh_mlp_pack")
 
     def check_errors(self):
@@ -109,10 +111,10 @@ class LearnedCorrection:
         torch = self.torch
         f = feats.to(self.device, torch.float32).contiguous()
         out = torch.empty((f.shape[0], 2), dtype=torch.float32, device=self.device)
-        self._check(self.L.bh_mlp_forward(ctypes.c_void_p(f.data_ptr()), f.shape[1], f.shape[0],
-                                          self._img(), ctypes.c_void_p(self.params.data_ptr()),
-                                          ctypes.c_void_p(out.data_ptr()),
-                                          ctypes.c_void_p(self.err.data_ptr()), self._st()),
+        self._check(self.L.bh_mlp_forward(f.data_ptr(), f.shape[1], f.shape[0],
+                                          self._img(), self.params.data_ptr(),
+                                          out.data_ptr(),
+                                          self.err.data_ptr(), self._st()),
                     "bh_mlp_forward")
         return out
 
@@ -123,20 +125,17 @@ class LearnedCorrection:
         t = targets.to(self.device, torch.float32).contiguous()
         self.loss.zero_()
         self._check(self.L.bh_mlp_train_batch(
-            ctypes.c_void_p(f.data_ptr()), f.shape[1], ctypes.c_void_p(t.data_ptr()), f.shape[0],
-            self._img(), ctypes.c_void_p(self.params.data_ptr()),
-            ctypes.c_void_p(self.grad.data_ptr()), ctypes.c_void_p(self.loss.data_ptr()),
-            ctypes.c_void_p(self.err.data_ptr()), self._st()), "bh_mlp_train_batch")
+            f.data_ptr(), f.shape[1], t.data_ptr(), f.shape[0],
+            self._img(), self.params.data_ptr(),
+            self.grad.data_ptr(), self.loss.data_ptr(),
+            self.err.data_ptr(), self._st()), "bh_mlp_train_batch")
         return self.loss
 
     def adam_step(self, lr):
         self.step_count += 1
-        self._check(self.L.bh_mlp_adam(ctypes.c_void_p(self.params.data_ptr()),
-                                       ctypes.c_void_p(self.m.data_ptr()),
-                                       ctypes.c_void_p(self.v.data_ptr()),
-                                       ctypes.c_void_p(self.grad.data_ptr()), self.step_count,
-                                       float(lr), self._st()), "bh_mlp_adam")
-        self.pack()
+        self._check(self.L.bh_mlp_adam_pack(self.params.data_ptr(), self.m.data_ptr(), self.v.data_ptr(),
+                                            self.grad.data_ptr(), self.step_count, float(lr), self._img(),
+                                            self._st()), "bh_mlp_adam_pack")
 
     def train(self, feats, targets, epochs=4, batch=65536, lr=2e-3, seed=0, log=None):
         """Mini-batch Adam on device tensors; returns the per-epoch mean loss."""

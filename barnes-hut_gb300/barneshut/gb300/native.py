@@ -40,7 +40,7 @@ EXPORTS = (
     "bh_summarize", "bh_evaluate", "bh_timestep", "bh_step", "bh_step_graph", "bh_error_flags",
     "bh_pair_counts", "bh_box_moments", "bh_grid_info", "bh_direct_sample", "bh_diagnostics",
     "bh_kernels_per_step", "bh_mlp_param_count", "bh_mlp_image_bytes", "bh_mlp_pack",
-    "bh_mlp_forward", "bh_mlp_train_batch", "bh_mlp_adam", "bh_set_correction", "bh_learned_pairs",
+    "bh_mlp_forward", "bh_mlp_train_batch", "bh_mlp_adam", "bh_mlp_adam_pack", "bh_set_correction", "bh_learned_pairs",
     "bh_direct_sum_noalloc", "bh_generate", "bh_graph_kernel_nodes", "bh_set_kernel_timing",
     "bh_force_kernel_ms", "bh_corrected_pairs", "bh_set_grid", "bh_leaf_moments", "bh_set_leaf_moments",
 )
@@ -164,7 +164,16 @@ def make_params(grav_constant=1.0, tick_seconds=0.005, softening=0.0, cutoff_r2=
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
+
+
+def current_stream_ptr(device):
+    """The cudaStream_t (an int) of torch's current stream on a device: without the stream object,
+    whose construction costs more host time than a launch."""
+    import torch
+
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 class Plan:
@@ -211,9 +220,7 @@ class Plan:
 
     # ------------------------------------------------------------ plumbing
     def _st(self):
-        torch = self._torch
-        s = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
-        return ctypes.c_void_p(s.cuda_stream)
+        return self.stream.cuda_stream if self.stream is not None else current_stream_ptr(self.device)
 
     def _check(self, rc):
         if rc != BH_OK:

@@ -874,8 +874,15 @@ extern "C" int bh_mlp_train_batch(const float *feats, int fs, const float *targe
 extern "C" int bh_mlp_adam(float *params, float *m, float *v, float *grad, int step, float lr,
                            void *stream) {
     if (!params || !m || !v || !grad || step < 1) return BH_ERR_INVALID;
-    return mlp_adam(params, m, v, grad, step, lr, (cudaStream_t)stream) == cudaSuccess ? BH_OK
-                                                                                     : BH_ERR_CUDA;
+    return mlp_adam(params, m, v, grad, step, lr, nullptr, (cudaStream_t)stream) == cudaSuccess ? BH_OK
+                                                                                              : BH_ERR_CUDA;
+}
+
+extern "C" int bh_mlp_adam_pack(float *params, float *m, float *v, float *grad, int step, float lr,
+                                void *image, void *stream) {
+    if (!params || !m || !v || !grad || step < 1 || !image || (((uintptr_t)image) & 15)) return BH_ERR_INVALID;
+    return mlp_adam(params, m, v, grad, step, lr, (uint8_t *)image, (cudaStream_t)stream) == cudaSuccess ? BH_OK
+                                                                                                       : BH_ERR_CUDA;
 }
 
 extern "C" int bh_set_correction(bh_plan *p, const void *image, const float *params) {

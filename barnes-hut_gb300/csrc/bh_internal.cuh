@@ -421,7 +421,8 @@ cudaError_t mlp_infer(const float *feats, int fs, long long P, const uint8_t *im
 cudaError_t mlp_train(const float *feats, int fs, const float *targets, long long P,
                       const uint8_t *img, const float *params, float *grad, float *loss,
                       unsigned *err, cudaStream_t st);
-cudaError_t mlp_adam(float *p, float *m, float *v, float *g, int step, float lr, cudaStream_t st);
+// img (or NULL): the packed images follow the parameters
+cudaError_t mlp_adam(float *p, float *m, float *v, float *g, int step, float lr, uint8_t *img, cudaStream_t st);
 cudaError_t learned_init();
 cudaError_t launch_learned_correct(const DevPlan &d, double theta_lo, const uint8_t *img,
                                    const float *params, bool tick, cudaStream_t st);

@@ -444,9 +444,31 @@ __global__ void __launch_bounds__(TT, 1) k_mlp_train(const float *feats, int fs,
     if (tid < 32) tc::tmem_dealloc(tm, 512);
 }
 
-// Adam (Kingma & Ba) on the master parameters; zeroes the gradient.
+// the operand images' copies of parameter i (k_mlp_pack's layout)
+__device__ __forceinline__ void pack_param(uint8_t *img, int i, float v) {
+    auto put = [&](int off) { *reinterpret_cast<uint16_t *>(img + off) = bf16_bits(v); };
+    if (i < P_B1) {  // W1[k][n]
+        const int k = (i - P_W1) / 64, n = (i - P_W1) % 64;
+        put(I_B1 + tc::kmajor_off(n, k, 2));
+    } else if (i >= P_W2 && i < P_B2) {
+        const int k = (i - P_W2) / 64, n = (i - P_W2) % 64;
+        put(I_B2 + tc::kmajor_off(n, k, 8));
+        put(I_B2T + tc::kmajor_off(k, n, 8));
+    } else if (i >= P_W3 && i < P_B3) {
+        const int k = (i - P_W3) / 64, n = (i - P_W3) % 64;
+        put(I_B3 + tc::kmajor_off(n, k, 8));
+        put(I_B3T + tc::kmajor_off(k, n, 8));
+    } else if (i >= P_W4 && i < P_B4) {  // W4[k][n]
+        const int k = (i - P_W4) / 16, n = (i - P_W4) % 16;
+        put(I_B4 + tc::kmajor_off(n, k, 8));
+        put(I_B4T + tc::kmajor_off(k, n, 2));
+    }
+}
+
+// Adam (Kingma & Ba) on the master parameters; zeroes the gradient.  img (or NULL): the operand
+// images follow the parameters (a launch less per training step).
 __global__ void k_mlp_adam(float *p, float *m, float *v, float *g, int step, float lr, float b1,
-                           float b2, float eps) {
+                           float b2, float eps, uint8_t *img) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P_TOTAL) return;
     // structurally zero entries stay zero
@@ -456,6 +478,7 @@ __global__ void k_mlp_adam(float *p, float *m, float *v, float *g, int step, flo
     g[i] = 0.f;
     if (fixed) {
         p[i] = 0.f;
+        if (img) pack_param(img, i, 0.f);
         return;
     }
     float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -464,7 +487,9 @@ __global__ void k_mlp_adam(float *p, float *m, float *v, float *g, int step, flo
     v[i] = vi;
     float mh = mi / (1.f - powf(b1, (float)step));
     float vh = vi / (1.f - powf(b2, (float)step));
-    p[i] -= lr * mh / (sqrtf(vh) + eps);
+    const float pi = p[i] - lr * mh / (sqrtf(vh) + eps);
+    p[i] = pi;
+    if (img) pack_param(img, i, pi);
 }
 
 // -------------------------------------------------------------------- launches
@@ -503,8 +528,8 @@ cudaError_t mlp_train(const float *feats, int fs, const float *targets, long lon
     return cudaGetLastError();
 }
 
-cudaError_t mlp_adam(float *p, float *m, float *v, float *g, int step, float lr, cudaStream_t st) {
-    k_mlp_adam<<<(P_TOTAL + 255) / 256, 256, 0, st>>>(p, m, v, g, step, lr, 0.9f, 0.999f, 1e-8f);
+cudaError_t mlp_adam(float *p, float *m, float *v, float *g, int step, float lr, uint8_t *img, cudaStream_t st) {
+    k_mlp_adam<<<(P_TOTAL + 127) / 128, 128, 0, st>>>(p, m, v, g, step, lr, 0.9f, 0.999f, 1e-8f, img);
     return cudaGetLastError();
 }
 

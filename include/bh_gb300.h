@@ -294,6 +294,10 @@ int bh_mlp_train_batch(const float *feats, int feat_stride, const float *targets
 /* One Adam step (beta 0.9 / 0.999, eps 1e-8) on params with moments m, v;
  * zeroes grad.  step counts from 1. */
 int bh_mlp_adam(float *params, float *m, float *v, float *grad, int step, float lr, void *stream);
+/* The same, and the operand images follow the parameters (bh_mlp_adam, then bh_mlp_pack, as one
+ * launch). */
+int bh_mlp_adam_pack(float *params, float *m, float *v, float *grad, int step, float lr, void *image,
+                     void *stream);
 
 /* Bind the MLP (image from bh_mlp_pack, FP32 parameters; the caller keeps
  * both alive) that bh_evaluate and bh_step apply when params.flags has

@@ -282,3 +282,72 @@ def test_bounding_boxes_of_many_systems():
             g = plan.grid_info(k)
             assert (g["min_x"], g["min_y"]) == (p[:, 0].min(), p[:, 1].min())
     assert plan.error_flags() == 0
+
+
+# One small system's tree, work items and moments by one cluster against the general kernels (the same
+# system first in a batch; its particle count a multiple of 32 keeps the leaf chunks' offsets): the same
+# bits, phase by phase and fused.  Quadrants of 0 to 32,768 particles, one box to 64 x 64.
+@pytest.mark.parametrize("n,grid,layout", [(32, 1, "uniform"), (32, 64, "uniform"), (1056, 3, "cluster"), (8192, 17, "uniform"),
+                                           (16416, 64, "cluster"), (32768, 64, "uniform"), (32768, 5, "cluster"),
+                                           (2048, 16, "coincident"), (32768, 2, "coincident")])
+@pytest.mark.parametrize("mode", ["stream", "walk", "flat", "fp64"])
+def test_cluster_tree_is_the_general_tree(n, grid, layout, mode):
+    from barneshut.gb300 import native, workloads
+
+    if layout == "coincident":  # half of them in one point
+        s = list(workloads.uniform(n, seed=1))
+        s[0][: n // 2], s[1][: n // 2] = 0.37, 0.61
+        o = np.random.default_rng(2).permutation(n)
+        s = tuple(a[o] for a in s)
+    else:
+        s = (workloads.uniform if layout == "uniform" else workloads.cluster_mixture)(n, seed=n + grid)
+    rest = workloads.uniform(64, seed=8)
+    kw = dict(stream=dict(theta=0.5, softening=1e-3, cutoff_r2=0.0), flat=dict(theta=0.0, cutoff_r2=1e-5),
+              walk=dict(theta=0.6, softening=1e-3, cutoff_r2=0.0, flags=native.BH_FLAG_WALK),
+              fp64=dict(theta=0.5, softening=1e-3, cutoff_r2=0.0, precision=native.BH_PREC_FP64))[mode]
+    prm = native.make_params(1.0, 1e-6, group_dim=0 if mode == "flat" else 2, **kw)
+
+    def result(sizes, grids, cols):
+        plan = native.Plan(sizes, grids, prm)
+        out = []
+        for fused in (False, True):
+            plan.load(*cols)
+            if fused:
+                plan.step(2)
+            else:
+                plan.create_tree()
+                plan.summarize()
+                plan.evaluate()
+                out.append(plan.box_moments(0))
+            st = plan.store()
+            out += [st[k][:n] for k in ("x", "y", "vx", "vy", "ax", "ay")]
+            out.append(plan.store_records()[:n])
+        assert plan.error_flags() == 0
+        return [a.cpu().numpy() for a in out]
+
+    alone = result([n], [grid], s)
+    batch = result([n, 64], [grid, 2], [np.concatenate([s[k], rest[k]]) for k in range(5)])
+    for a, b in zip(alone, batch):
+        assert np.array_equal(a, b)
+
+
+def test_adam_with_images_is_adam_then_pack():
+    from barneshut.gb300.learned import LearnedCorrection
+
+    rng = np.random.default_rng(31)
+    f, t = network_rows(500, 31)
+    F, T = torch.from_numpy(f).cuda(), torch.from_numpy(t).cuda()
+    a = LearnedCorrection(seed=31)
+    a.grad_batch(F, T)
+    b = LearnedCorrection(seed=31)
+    b.grad.copy_(a.grad)
+    a.adam_step(1e-3)
+    b.step_count += 1
+    assert b.L.bh_mlp_adam(b.params.data_ptr(), b.m.data_ptr(), b.v.data_ptr(), b.grad.data_ptr(), 1, 1e-3, b._st()) == 0
+    b.pack()
+    assert torch.equal(a.params, b.params) and torch.equal(a.m, b.m) and torch.equal(a.v, b.v)
+    x = torch.from_numpy(rng.standard_normal((300, 6)).astype(np.float32)).cuda()
+    assert torch.equal(a.forward(x), b.forward(x))
+    a.grad_batch(F, T)
+    b.grad_batch(F, T)
+    assert torch.allclose(a.grad, b.grad, rtol=1e-4, atol=1e-6)  # (FP32 additions in another order)
