@@ -50,7 +50,7 @@ constexpr int SITEM_TILE = 8;     // target groups per tile of the streaming wor
 constexpr int SUM_TILE = 16;      // leaf boxes per side of a summarize tile (pyramid levels 0..4)
 constexpr int STREAM_CHUNK = 128;  // targets per work item of the list-streaming force kernel
 constexpr int LIST_MAX_G = 16384;  // largest G of the list-streaming path (32-bit group indices)
-constexpr int CL_MAX_N = 32768, CL_MAX_SIDE = 64, CL_MAX_BOXES = 4096;  // systems whose tree one cluster builds (k_tree_cluster)
+constexpr int CL_MAX_N = 16384, CL_MAX_SIDE = 64, CL_MAX_BOXES = 4096;  // systems whose tree one cluster builds (k_tree_cluster)
 constexpr long long STORE_GATHER_MIN = 262144;  // k_store: from here on a disordered state is gathered
 constexpr int STORE_NEAR = 64;
 constexpr int ITEM_BUCKETS = 32;   // log2 cost buckets of the heaviest-first item order

@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(256) k_item_order(DevPlan d) {
     }
 }
 
-// Both of the above for a few items, by one CTA (a launch less; 10,000 particles: @IO@ us against the
-// pair's @IO2@).
+// Both of the above for a few items, by one CTA (a launch less; 10,000 particles: 6.1 us against the
+// pair's 5.6 and 4.3).
 constexpr int ORDER_THREADS = 1024, ORDER_MAX = 8192;
 
 __global__ void __launch_bounds__(ORDER_THREADS) k_item_order_few(DevPlan d) {
