@@ -350,3 +350,37 @@ def test_adam_with_images_is_adam_then_pack():
     a.grad_batch(F, T)
     b.grad_batch(F, T)
     assert torch.allclose(a.grad, b.grad, rtol=1e-4, atol=1e-6)  # (FP32 additions in another order)
+
+
+# Long direct sums in split floats, with what they leave to FP64: coincident and very close pairs, a
+# system whose masses leave the floats' range, one far from the origin; and a target of another system.
+@pytest.mark.parametrize("kind", ["plain", "close", "heavy", "offset"])
+@pytest.mark.parametrize("eps", [0.0, 1e-3])
+def test_direct_sample_long_sums(kind, eps):
+    from barneshut.gb300 import native
+
+    n, nt = 524287 + 1024, 37
+    rng = np.random.default_rng(len(kind))
+    x, y = rng.random((2, n))
+    m = 1.0 + rng.random(n)
+    t = rng.choice(n - 200, nt, replace=False)
+    if kind == "close":
+        x[n - 100:n - 63], y[n - 100:n - 63] = x[t] + 1e-9 * rng.random(nt), y[t] - 1e-12
+        if eps > 0.0:
+            x[n - 50:n - 13], y[n - 50:n - 13] = x[t], y[t]
+    elif kind == "heavy":
+        m[5] = 1e25
+    elif kind == "offset":
+        x, y = x + 12345.0, y - 77.0
+    z = np.zeros(n)
+    plan = native.Plan([100, n], [2, 4], native.make_params(1.0, 1e-5, eps, 0.0, 0.5))
+    pad = rng.random((2, 100))
+    plan.load(np.r_[pad[0], x], np.r_[pad[1], y], np.r_[np.ones(100), m], np.r_[z[:100], z], np.r_[z[:100], z])
+    ax, ay = plan.direct_sample(np.r_[t + 100, 3], sys=1)
+    got = np.stack([ax.cpu().numpy(), ay.cpu().numpy()])
+    assert np.isnan(got[:, nt]).all()
+    for k, i in enumerate(t):
+        dx, dy = np.delete(x, i) - x[i], np.delete(y, i) - y[i]
+        w = np.delete(m, i) / (dx * dx + dy * dy + eps * eps)
+        ref = np.array([np.sum(w * dx), np.sum(w * dy)])
+        assert np.linalg.norm(got[:, k] - ref) <= 1e-12 * np.linalg.norm(ref)
