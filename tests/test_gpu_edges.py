@@ -384,3 +384,48 @@ def test_direct_sample_long_sums(kind, eps):
         w = np.delete(m, i) / (dx * dx + dy * dy + eps * eps)
         ref = np.array([np.sum(w * dx), np.sum(w * dy)])
         assert np.linalg.norm(got[:, k] - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+# FP64 forces whose near pairs run in split floats (from 8,192 particles on), every pair near: close and
+# coincident pairs, pairs at the cutoff, a mass out of the floats' range, a system far off, another in
+# the batch.  FP64 sums of 8,000 terms: 1e-12.
+@pytest.mark.parametrize("kind", ["plain", "close", "cutoff", "heavy", "offset"])
+@pytest.mark.parametrize("theta,eps,cutoff", [(0.0, 0.0, 1e-5), (0.0, 0.0, 0.0), (0.5, 1e-3, 0.0), (0.0, 1e-2, 1e-4)])
+def test_fp64_forces_in_split_floats(kind, theta, eps, cutoff):
+    from barneshut.gb300 import native
+
+    n, extra = 8200, 300
+    rng = np.random.default_rng(len(kind) + 7)
+    x, y = rng.random((2, n))
+    m = 1.0 + rng.random(n)
+    t = rng.choice(n - 200, 40, replace=False)
+    if kind == "close":
+        x[n - 100:n - 60], y[n - 100:n - 60] = x[t] + 1e-7, y[t]
+        x[n - 60:n - 20], y[n - 60:n - 20] = x[t], y[t]
+    elif kind == "cutoff" and cutoff > 0.0:
+        f = np.sqrt(cutoff) * (1.0 + np.array([1e-4, -1e-4, 1e-7, -1e-7] * 10))
+        x[n - 100:n - 60], y[n - 100:n - 60] = x[t] + f * np.cos(t), y[t] + f * np.sin(t)
+    elif kind == "heavy":
+        m[3] = 1e22
+    elif kind == "offset":
+        x, y = x + 4321.0, y - 99.0
+    o = rng.random((2, extra))
+    z = np.zeros(n + extra)
+    prm = native.make_params(1.0, 1e-5, eps, cutoff, theta, 1, native.BH_PREC_FP64)
+    plan = native.Plan([extra, n], [1, 2], prm)
+    plan.load(np.r_[o[0], x], np.r_[o[1], y], np.r_[np.ones(extra), m], z, z)
+    for _ in range(2):  # (the sampler and a second evaluation use the same scratch)
+        plan.create_tree()
+        plan.summarize()
+        plan.evaluate()
+    out = plan.store()
+    assert plan.error_flags() == 0
+    got = np.stack([out["ax"].cpu().numpy(), out["ay"].cpu().numpy()])[:, extra:]
+    for i in t:
+        dx, dy = x - x[i], y - y[i]
+        r2 = dx * dx + dy * dy
+        with np.errstate(divide="ignore", invalid="ignore"):
+            w = np.where(r2 > cutoff, m / (r2 + eps * eps), 0.0)
+        w[i] = 0.0
+        ref = np.array([np.sum(w * dx), np.sum(w * dy)])
+        assert np.linalg.norm(got[:, i] - ref) <= 1e-12 * np.linalg.norm(ref)
