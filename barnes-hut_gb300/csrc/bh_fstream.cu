@@ -79,10 +79,6 @@ __device__ __forceinline__ void pair1(float x, float y, float m, float ntx, floa
     ay = __fmaf_rn(w, dy, ay);
 }
 
-// (float)k for |k| < 2^22 by an exact addition: the conversion instruction runs on the reciprocals'
-// pipe, which bounds the sweeps.
-__device__ __forceinline__ float small_int_f(int k) { return __fsub_rn(__int_as_float(0x4B400000 + k), 12582912.f); }
-
 // How many of the heaviest items run as four warps' work (.x) and how many of the next as two (.y),
 // from the cost histogram (bucket b: costs in [2^b, 2^(b+1))).  A warp alone takes about 70 cycles
 // per source of a full item where a busy scheduler takes 40, so an item of more than 1/1,000 of the

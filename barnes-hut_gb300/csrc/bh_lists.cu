@@ -5,18 +5,18 @@
 // sequential/evaluation.py:73-109); in theta mode this project replaces the flat far field with
 // a walk of the cell pyramid, and this kernel does that walk once per target group instead of
 // once per work item.  One warp per group (grid-stride over groups) walks the pyramid level by
-// level, each lane testing LU frontier cells per round (their records loaded together): a
-// cell whose centre of mass lies at distance d from the group's box rectangle is accepted when
-// s^2 < theta^2 d^2 (s = cell edge) and goes to the far list, a rejected leaf goes to the near
-// list, any other rejected cell opens into its children.  Ballots and a warp scan place the
-// entries in frontier order, so list order is deterministic and matches the walking force
-// kernel's; the test is the same FP32 arithmetic, so both paths accept the same cells.
+// level, each lane testing a frontier cell per round: a cell whose centre of mass lies at distance d
+// from the group's box rectangle is accepted when s^2 < theta^2 d^2 (s = cell edge) and goes to the
+// far list, a rejected leaf goes to the near list, any other rejected cell opens into its children.
+// Ballots (a warp scan where a level's last row or column has fewer children) place the entries in
+// frontier order, so list order is deterministic and matches the walking force kernel's; the test is
+// the same FP32 arithmetic, so both paths accept the same cells.
 //
 // Output per group g of system s: far entries (the accepted cell's centre of mass in the group
-// frame, as the opening test computed it, and its mass) at lfar[s.lfoff + lg * s.lfcap ..]; near descriptors -- (first particle, exclusive prefix of the
-// boxes' particle counts, box-origin shift in the group frame) and (box index, mass, centre of
-// mass in the group frame) -- at lnear[s.lnoff + lg * 2 * (s.lncap + 1) ..] with the total in
-// descriptor [count]; lcnt[g] = (far count, near count).  The slots are
+// frame, as the opening test computed it, and its mass) at lfar[s.lfoff + lg * s.lfcap ..]; near
+// descriptors -- (first particle, exclusive prefix of the boxes' particle counts, box-origin shift in
+// the group frame) and (box index, mass, centre of mass in the group frame) -- at lnear[s.lnoff + lg *
+// 2 * (s.lncap + 1) ..] with the total in descriptor [count]; lcnt[g] = (far count, near count).  The slots are
 // sized on the host so that a level's accepted cells never exceed FRONTIER_CAP; the kernel still
 // checks and raises BH_DEV_LIST_OVERFLOW.
 #include "bh_internal.cuh"
@@ -25,11 +25,12 @@
 namespace bh {
 
 constexpr int LW = 4;  // warps per list-building CTA; one warp walks one group
-constexpr int LU = 1;  // frontier cells per lane per round (a level's frontier averages ~47 cells)
-constexpr int LISTS_MINB = 12;  // CTAs per SM (40 registers): the walk is latency-bound
+// CTAs per SM (64 registers): the walk is bound by its instructions and their latency together.  1,048,576
+// particles, four steps: 3,773 us with twelve (40 registers, which spill), 3,749 with ten, 3,717 with eight
+constexpr int LISTS_MINB = 8;
 
 __global__ void __launch_bounds__(LW * 32, LISTS_MINB) k_lists(DevPlan d) {
-    __shared__ int front[LW][2][FR_CAP];
+    __shared__ __align__(16) int front[LW][2][FR_CAP];  // cells as x << 16 | y; near boxes as indices
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int(*fb)[FR_CAP] = front[warp];
     const float theta2 = d.theta2_f;
@@ -60,39 +61,29 @@ __global__ void __launch_bounds__(LW * 32, LISTS_MINB) k_lists(DevPlan d) {
             const float s2 = __fmul_rn(s_f, s_f);
             const int *fr = fb[cur];
             int *fn = fb[cur ^ 1];  // next frontier; at the leaf level, the near boxes
+            // the cells over the group's rectangle; and whether every cell has its four children
+            const int ox0 = gx0 >> l, ox1 = (gx1 - 1) >> l, oy0 = gy0 >> l, oy1 = (gy1 - 1) >> l;
+            const bool full = gc == 2 * gl;
+            const float4 *rec = d.rec + sd.coff + sd.lvoff[l];
             int nnext = 0;
-            for (int q0 = 0; q0 < nfr; q0 += 32 * LU) {
-                int loc[LU];
-                float4 rr[LU];
-#pragma unroll
-                for (int u = 0; u < LU; u++) {  // issue the round's record loads together
-                    const int q = q0 + u * 32 + lane;
-                    loc[u] = -1;
-                    rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (q < nfr) {
-                        const int c = fr[q];
-                        if ((unsigned)c >= (unsigned)(gl * gl)) {
-                            raise_err(d.glob, 4u /*BH_DEV_BAD_KEY*/);  // never expected: skip it
-                        } else {
-                            loc[u] = c;
-                            rr[u] = d.rec[sd.coff + sd.lvoff[l] + c];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < LU; u++) {  // classify and append in frontier order
-                    int kind = 0, ci = 0, cj = 0;
-                    float rx = 0.f, ry = 0.f;  // centre of mass in the group frame
-                    if (loc[u] >= 0 && rr[u].z > 0.f) {
-                        ci = loc[u] / gl;
-                        cj = loc[u] - ci * gl;
-                        const int lo_x = ci << l, hi_x = (ci + 1) << l;
-                        const int lo_y = cj << l, hi_y = (cj + 1) << l;
-                        const bool overlap = lo_x < gx1 && hi_x > gx0 && lo_y < gy1 && hi_y > gy0;
+            for (int q0 = 0; q0 < nfr; q0 += 32) {
+                const int q = q0 + lane;
+                int ci = 0, cj = 0, kind = 0;
+                float rx = 0.f, ry = 0.f;  // centre of mass in the group frame
+                float4 rr = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (q < nfr) {
+                    const int c = fr[q];
+                    ci = c >> 16;
+                    cj = c & 0xFFFF;
+                    if ((unsigned)ci >= (unsigned)gl || (unsigned)cj >= (unsigned)gl)
+                        raise_err(d.glob, 4u /*BH_DEV_BAD_KEY*/);  // never expected: skip it
+                    else
+                        rr = rec[ci * gl + cj];
+                    if (rr.z > 0.f) {
                         bool accept = false;
-                        if (!overlap) {
-                            rx = __fadd_rn(__fmul_rn((float)(lo_x - gx0), step_f), rr[u].x);
-                            ry = __fadd_rn(__fmul_rn((float)(lo_y - gy0), step_f), rr[u].y);
+                        if (ci < ox0 || ci > ox1 || cj < oy0 || cj > oy1) {
+                            rx = __fadd_rn(__fmul_rn(small_int_f((ci << l) - gx0), step_f), rr.x);
+                            ry = __fadd_rn(__fmul_rn(small_int_f((cj << l) - gy0), step_f), rr.y);
                             const float dxo = fmaxf(0.f, fmaxf(-rx, __fsub_rn(rx, W_f)));
                             const float dyo = fmaxf(0.f, fmaxf(-ry, __fsub_rn(ry, W_f)));
                             const float d2 = __fadd_rn(__fmul_rn(dxo, dxo), __fmul_rn(dyo, dyo));
@@ -100,36 +91,46 @@ __global__ void __launch_bounds__(LW * 32, LISTS_MINB) k_lists(DevPlan d) {
                         }
                         kind = accept ? 1 : (l == 0 ? 2 : 3);
                     }
-                    const unsigned mf = __ballot_sync(0xffffffffu, kind == 1);
-                    const unsigned mn = __ballot_sync(0xffffffffu, kind == 2);
-                    int nch = 0;
-                    if (kind == 3) nch = (2 * ci + 1 < gc ? 2 : 1) * (2 * cj + 1 < gc ? 2 : 1);
+                }
+                // append in frontier order
+                const unsigned mf = __ballot_sync(0xffffffffu, kind == 1);
+                const unsigned mo = __ballot_sync(0xffffffffu, kind >= 2);  // (a level has near boxes or opened cells)
+                if (kind == 1) {
+                    const int pos = nfar + __popc(mf & lt_mask);
+                    if (pos < sd.lfcap) far_out[pos] = make_float4(rx, ry, rr.z, 0.f);
+                }
+                nfar += __popc(mf);
+                if (l == 0) {
+                    if (kind == 2) {
+                        const int pos = nnear + __popc(mo & lt_mask);
+                        if (pos < sd.lncap) fn[pos] = ci * gl + cj;
+                    }
+                    nnear += __popc(mo);
+                } else if (full) {
+                    const int pos = nnext + 4 * __popc(mo & lt_mask), c0 = (ci << 17) | (cj << 1);
+                    if (kind == 3 && pos + 4 <= FR_CAP)
+                        *reinterpret_cast<int4 *>(fn + pos) = make_int4(c0, c0 + 1, c0 + 65536, c0 + 65537);
+                    nnext += 4 * __popc(mo);
+                } else {
+                    const bool bx = 2 * ci + 1 < gc, by = 2 * cj + 1 < gc;  // second children along x, y
+                    const int nch = kind == 3 ? (bx ? 2 : 1) * (by ? 2 : 1) : 0;
                     int inc = nch;  // inclusive warp scan of the children counts
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const int y = __shfl_up_sync(0xffffffffu, inc, o);
                         if (lane >= o) inc += y;
                     }
-                    const int ntot = __shfl_sync(0xffffffffu, inc, 31);
-                    if (kind == 1) {
-                        const int pos = nfar + __popc(mf & lt_mask);
-                        if (pos < sd.lfcap) far_out[pos] = make_float4(rx, ry, rr[u].z, 0.f);
-                    } else if (kind == 2) {
-                        const int pos = nnear + __popc(mn & lt_mask);
-                        if (pos < sd.lncap) fn[pos] = loc[u];
-                    } else if (kind == 3) {
-                        int pos = nnext + inc - nch;
-                        if (pos + nch <= FR_CAP) {
-                            for (int a = 0; a < 2; a++)
-                                for (int b = 0; b < 2; b++)
-                                    if (2 * ci + a < gc && 2 * cj + b < gc) fn[pos++] = (2 * ci + a) * gc + (2 * cj + b);
-                        }
+                    int pos = nnext + inc - nch;
+                    if (nch && pos + nch <= FR_CAP) {
+                        const int c0 = (ci << 17) | (cj << 1);
+                        fn[pos++] = c0;
+                        if (by) fn[pos++] = c0 + 1;
+                        if (bx) fn[pos++] = c0 + 65536;
+                        if (bx && by) fn[pos++] = c0 + 65537;
                     }
-                    nfar += __popc(mf);
-                    nnear += __popc(mn);
-                    if (nnext + ntot > FR_CAP) ovf = true;
-                    nnext += ntot;
+                    nnext += __shfl_sync(0xffffffffu, inc, 31);
                 }
+                if (nnext > FR_CAP) ovf = true;
             }
             __syncwarp();  // the next frontier (or the near list) is complete
             cur ^= 1;
@@ -143,48 +144,33 @@ __global__ void __launch_bounds__(LW * 32, LISTS_MINB) k_lists(DevPlan d) {
         const int nn = min(nnear, sd.lncap);
         const int *nl = fb[cur];
         int base = 0;
-        // LU rounds of 32 boxes at a time: their particle ranges and records are loaded together
-        for (int k0 = 0; k0 <= nn; k0 += 32 * LU) {
-            int loc[LU], st[LU], c[LU];
-            float4 rr[LU];
-#pragma unroll
-            for (int u = 0; u < LU; u++) {
-                const int k = k0 + 32 * u + lane;
-                loc[u] = k < nn ? nl[k] : 0;
+        for (int k0 = 0; k0 <= nn; k0 += 32) {
+            const int k = k0 + lane, loc = k < nn ? nl[k] : 0;
+            int st = 0, c = 0;
+            float4 rr = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < nn) {
+                st = d.box_start[sd.boff + loc];
+                c = d.box_start[sd.boff + loc + 1] - st;
+                rr = d.rec[sd.coff + loc];  // the leaf's record (level 0)
             }
+            int inc = c;
 #pragma unroll
-            for (int u = 0; u < LU; u++) {
-                const int k = k0 + 32 * u + lane;
-                st[u] = c[u] = 0;
-                rr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k < nn) {
-                    st[u] = d.box_start[sd.boff + loc[u]];
-                    c[u] = d.box_start[sd.boff + loc[u] + 1] - st[u];
-                    rr[u] = d.rec[sd.coff + loc[u]];  // the leaf's record (level 0)
-                }
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
             }
-#pragma unroll
-            for (int u = 0; u < LU; u++) {
-                const int k = k0 + 32 * u + lane;
-                int inc = c[u];
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += y;
-                }
-                const int pre = base + inc - c[u];
-                if (k < nn) {
-                    const int kx = loc[u] / sd.G, ky = loc[u] - kx * sd.G;
-                    const float shx = __fmul_rn((float)(kx - gx0), step_f), shy = __fmul_rn((float)(ky - gy0), step_f);
-                    near_out[2 * k] = make_int4(st[u], pre, __float_as_int(shx), __float_as_int(shy));
-                    near_out[2 * k + 1] = make_int4(loc[u], __float_as_int(rr[u].z), __float_as_int(__fadd_rn(shx, rr[u].x)),
-                                                    __float_as_int(__fadd_rn(shy, rr[u].y)));
-                } else if (k == nn) {
-                    near_out[2 * k] = make_int4(0, pre, 0, 0);
-                    near_out[2 * k + 1] = make_int4(0, 0, 0, 0);
-                }
-                base += __shfl_sync(0xffffffffu, inc, 31);
+            const int pre = base + inc - c;
+            if (k < nn) {
+                const int kx = loc / sd.G, ky = loc - kx * sd.G;
+                const float shx = __fmul_rn(small_int_f(kx - gx0), step_f), shy = __fmul_rn(small_int_f(ky - gy0), step_f);
+                near_out[2 * k] = make_int4(st, pre, __float_as_int(shx), __float_as_int(shy));
+                near_out[2 * k + 1] = make_int4(loc, __float_as_int(rr.z), __float_as_int(__fadd_rn(shx, rr.x)),
+                                                __float_as_int(__fadd_rn(shy, rr.y)));
+            } else if (k == nn) {
+                near_out[2 * k] = make_int4(0, pre, 0, 0);
+                near_out[2 * k + 1] = make_int4(0, 0, 0, 0);
             }
+            base += __shfl_sync(0xffffffffu, inc, 31);
         }
         if (lane == 0) {
             if (ovf || nfar > sd.lfcap || nnear > sd.lncap) raise_err(d.glob, 2u /*BH_DEV_LIST_OVERFLOW*/);

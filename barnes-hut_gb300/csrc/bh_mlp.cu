@@ -55,8 +55,8 @@ __global__ void k_mlp_pack(const float *p, uint8_t *img) {
 }
 
 // ---------------------------------------------------------------- inference
-constexpr int INFER_GROUPS = 2;  // 128-row tiles in flight per CTA, one per group of 128 threads
-constexpr int INFER_CTAS = 4;    // CTAs per SM: 64 registers a thread, 54 KB, 128 TMEM columns each
+constexpr int INFER_GROUPS = 8;  // 128-row tiles in flight per CTA, one per group of 128 threads
+constexpr int INFER_CTAS = 1;    // CTAs per SM (64 registers a thread, 151 KB, all of the TMEM columns)
 struct MlpSmemInfer {
     // byte offsets in dynamic shared memory
     static constexpr int W = 0;                              // forward images, I_FWD bytes
@@ -78,8 +78,9 @@ __device__ __forceinline__ void load_bias(float *bias, const float *params) {
 }
 
 // out[r] = MLP(feats[r][0..5]) for r < P; feats row stride fs floats, out row stride 2.
-// 1,000,003 rows, stride 8: 119 us -> 111 us (one 128-thread tile per CTA, scalar epilogue and
-// the whole accumulator row in registers before).
+// 1,000,003 rows, stride 8: 119 us -> 101 us (one 128-thread tile per CTA, scalar epilogue and
+// the whole accumulator row in registers before); 107 us as two CTAs of four groups, 111 as four of
+// two (each stages the weights); 81 us is the MUFU pipe's time for the tanh.
 __global__ void __launch_bounds__(128 * INFER_GROUPS, INFER_CTAS)
 k_mlp_infer(const float *feats, int fs, long long P, const uint8_t *img, const float *params, float *out,
             unsigned *err) {

@@ -65,6 +65,10 @@ __device__ __forceinline__ f2_t f2_rcp(f2_t a) {
     return r;
 }
 
+// (float)k for |k| < 2^22 by an exact addition: the conversion instruction runs on the reciprocals'
+// pipe, which bounds the sweeps.
+__device__ __forceinline__ float small_int_f(int k) { return __fsub_rn(__int_as_float(0x4B400000 + k), 12582912.f); }
+
 // Exclusive block scan of one int per thread; *total = block sum.
 __device__ __forceinline__ int block_scan(int v, int *sh, int *total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
