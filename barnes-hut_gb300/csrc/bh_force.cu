@@ -472,7 +472,7 @@ k_force(DevPlan d, int tick, int accumulate) {
                 __syncthreads();
                 if (active && F32) {
                     const float4 *s4 = reinterpret_cast<const float4 *>(src);
-#pragma unroll 8 / NR
+#pragma unroll 16 / NR
                     for (int j = slice; j < ns; j += nslice) {
                         const ulonglong2 sxy = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j);
                         const ulonglong2 smi = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j + 1);
@@ -790,14 +790,16 @@ static cudaError_t launch_force_nr(const DevPlan &d, bool accumulate, cudaStream
 
 // An item is one CTA's work, or two CTAs' (NR = 2) while the items, doubled, still fit on the chip
 // at once: each CTA then repeats the item's walk and staging, which is what its idle neighbours
-// would have waited for.  100,003 particles on 12 x 12 boxes, flat, FP32: 829 us with one CTA per
-// item and scalar arithmetic, 570 us packed, 408 us with two.
-template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 6 : 8)>
+// would have waited for.  100,003 particles on 12 x 12 boxes, flat, FP32, no cutoff, the round: 958 us with
+// one CTA per item and scalar arithmetic, 699 packed, 502 with two.  With the cutoff test four CTAs per SM
+// (five of the half ones): 200,000 particles on 24 x 24 boxes 917 us, with six, which spill, 1,135.
+template <bool TEST, int MINB> constexpr int HALF_MINB = TEST ? MINB + 1 : MINB;
+template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 4 : 8)>
 static cudaError_t launch_force_t(const DevPlan &d, bool accumulate, cudaStream_t st) {
     const long long items_max = d.NG_total + d.n_total / d.chunk + 1;
     if constexpr (sizeof(R) == 4)
-        if (2 * items_max <= (long long)d.nsm * MINB)
-            return launch_force_nr<R, 2, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);
+        if (2 * items_max <= (long long)d.nsm * HALF_MINB<TEST, MINB>)
+            return launch_force_nr<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>(d, accumulate, st, items_max);
     return launch_force_nr<R, FORCE_R, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);
 }
 
@@ -823,13 +825,13 @@ static cudaError_t launch_force64(const DevPlan &d, bool accumulate, cudaStream_
 
 bool force_splits(long long n_total) { return n_total >= SPLIT_FORCE_MIN; }
 
-template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 6 : 8)>
+template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 4 : 8)>
 static cudaError_t init_force_t() {
     const int sm = (int)force_smem<R>();
     cudaError_t e = cudaFuncSetAttribute(k_force<R, FORCE_R, KAHAN, TEST, EXACT, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess || sizeof(R) == 8) return e;
-    return cudaFuncSetAttribute(k_force<R, 2, KAHAN, TEST, EXACT, MINB>,
+    return cudaFuncSetAttribute(k_force<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
