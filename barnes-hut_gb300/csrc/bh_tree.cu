@@ -693,14 +693,15 @@ __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
 // on the order in which k_place's atomics handed out slots:
 //   k_perm     perm[box_start + earlier quadrants + slot] = input index (slots: k_place);
 //   k_segsort  each quadrant's stretch of perm sorted ascending -- up to SEG_REG entries in a
-//              thread's registers, longer ones listed for k_segsort_big (up to SEG_WARP entries
-//              a warp each, a bitonic network in its registers or shared memory; longer ones a CTA
-//              each, four stable 8-bit radix passes through the dead slot array);
+//              thread's registers, longer ones listed for k_segsort_big (up to SEG_LANES entries
+//              a warp each, a bitonic network in its registers; up to SEG_MERGE a CTA each, such runs
+//              merged in shared memory; longer ones a CTA each, four stable 8-bit radix passes
+//              through the dead slot array);
 //   k_gather   output particle t takes input perm[t]: the FP64 state of the next buffer, the
 //              32-byte packed record (offsets from the box origin computed in FP64, rounded
 //              once to float) and the sorted key; and it sums the leaves (below).
 constexpr int SEG_REG = 16;
-constexpr int SEG_WARP = 1024;
+constexpr int SEG_LANES = 256;  // longest stretch sorted by a warp
 constexpr int SEG_CHECK = 128;  // stretches up to this long are checked for order by their thread
 
 __device__ __forceinline__ int quad_first(const DevPlan &d, int key4) {
@@ -759,7 +760,7 @@ __global__ void __launch_bounds__(TPB) k_segsort(DevPlan d) {
             }
             if (sorted) continue;
         }
-        if (n > SEG_WARP) {  // listed from the far end of the same array
+        if (n > SEG_LANES) {  // listed from the far end of the same array
             const unsigned k = atomicAdd(&d.glob->nhuge, 1u);
             d.bigseg[d.bigseg_cap - 1 - k] = make_int2(s0, n);
             continue;
@@ -844,12 +845,20 @@ __device__ void cta_radix_sort(int *src, int *dst, int n, RadixScratch<NT> &rs) 
         __syncthreads();
         for (int k = tid; k < n; k += NT) atomicAdd(&rs.hist[(src[k] >> sh) & 255], 1);
         __syncthreads();
-        if (tid == 0) {
-            int acc = 0;
-            for (int k = 0; k < 256; k++) {
-                rs.base[k] = acc;
-                acc += rs.hist[k];
+        if (warp == 0) {
+            int own[8], sum = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                own[k] = sum;
+                sum += rs.hist[8 * lane + k];
             }
+            int before = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += u;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) rs.base[8 * lane + k] = before - sum + own[k];
         }
         __syncthreads();
         for (int c0 = 0; c0 < n; c0 += NT) {
@@ -885,66 +894,92 @@ __device__ void cta_radix_sort(int *src, int *dst, int n, RadixScratch<NT> &rs) 
 }
 
 // Long stretches.  Up to SEG_LANES entries a warp sorts in its registers (batches of small boxes in
-// file order have most of theirs here: 27.3M particles 670 -> 344 us, against the shared-memory
-// network), up to SEG_WARP in its slice of shared memory, longer ones a CTA.
-constexpr int SEG_LANES = 256;
+// file order have most of theirs here: 27.3M particles 670 -> 344 us, against a shared-memory
+// network).  Up to SEG_MERGE a CTA sorts runs of SEG_LANES that way and merges them pairwise in shared
+// memory, each entry finding its place in the other run by binary search; longer ones take the radix
+// passes.  (One warp on a shared-memory network took 45 us for a single stretch of 257 to 512
+// entries, the longest chain of the tree build wherever boxes are dense: a whole step of 131,071
+// Gaussian particles on 40 x 40 boxes 648 -> 605 us, of 500,000 on 79 x 79 1,889 -> 1,840.)
+constexpr int SEG_MERGE = 4096;
+
+__device__ __forceinline__ void seg_warp(int *p, int n) {  // n <= SEG_LANES
+    if (n <= 32) seg_regs<1>(p, n);
+    else if (n <= 64) seg_regs<2>(p, n);
+    else if (n <= 128) seg_regs<4>(p, n);
+    else seg_regs<8>(p, n);
+}
+
+template <int NT>
+union LongScratch {
+    RadixScratch<NT> rs;
+    int run[2][SEG_MERGE];
+};
+
+// Ascending sort of the n distinct entries at p by a CTA of NT threads (tmp: n entries of scratch,
+// used beyond SEG_MERGE).
+template <int NT>
+__device__ void cta_sort(int *p, int *tmp, int n, LongScratch<NT> &ls) {
+    if (n > SEG_MERGE) {
+        cta_radix_sort<NT>(p, tmp, n, ls.rs);
+        return;
+    }
+    constexpr int R = SEG_LANES / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int m = SEG_LANES;
+    while (m < n) m <<= 1;
+    int *a = ls.run[0], *b = ls.run[1];
+    // a stretch whose slots the atomics happened to hand out in input order is done already (the
+    // common case when the input is the previous step's order)
+    bool sorted = true;
+    for (int k = tid; k < n; k += NT) {
+        const int v = p[k];
+        sorted &= k == 0 || p[k - 1] < v;
+    }
+    if (__syncthreads_and(sorted)) return;
+    for (int c = warp; c < m / SEG_LANES; c += NT / 32) {
+        int v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int k = SEG_LANES * c + 32 * r + lane;
+            v[r] = k < n ? p[k] : 0x7FFFFFFF;
+        }
+        warp_bitonic<R>(v);
+#pragma unroll
+        for (int r = 0; r < R; r++) a[SEG_LANES * c + 32 * r + lane] = v[r];
+    }
+    __syncthreads();
+    for (int w = SEG_LANES; w < m; w <<= 1) {
+        for (int k = tid; k < m; k += NT) {
+            // the entry's place: its own in its run, plus the entries of the other run before it
+            // (equal ones, all padding, count for the right run only: every place is taken once)
+            const int v = a[k], right = k & w;
+            const int *o = a + ((k & ~(2 * w - 1)) | (right ^ w));
+            int lo = 0;
+            for (int h = w >> 1; h > 0; h >>= 1) lo += (right ? o[lo + h - 1] <= v : o[lo + h - 1] < v) ? h : 0;
+            lo += (right ? o[lo] <= v : o[lo] < v) ? 1 : 0;
+            b[(k & ~(2 * w - 1)) + (k & (w - 1)) + lo] = v;
+        }
+        __syncthreads();
+        int *t = a;
+        a = b;
+        b = t;
+    }
+    for (int k = tid; k < n; k += NT) p[k] = a[k];
+    __syncthreads();  // the runs are the next stretch's
+}
 
 __global__ void __launch_bounds__(TPB) k_segsort_big(DevPlan d) {
-    __shared__ int sv[TPB / 32][SEG_WARP];
-    __shared__ RadixScratch<TPB> rs;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // stretches of SEG_REG + 1 .. SEG_WARP entries: a warp each; beyond SEG_LANES a bitonic network
-    // over the next power of two (padded with INT_MAX) in the warp's slice of shared memory
-    const unsigned nbig = d.glob->nbig;
-    int *w = sv[warp];
-    for (unsigned e = (unsigned)(blockIdx.x * (TPB / 32) + warp); e < nbig; e += gridDim.x * (TPB / 32)) {
-        const int2 sg = d.bigseg[e];
-        const int s0 = sg.x, n = sg.y;
-        if (n <= SEG_LANES) {
-            if (n <= 32) seg_regs<1>(d.perm + s0, n);
-            else if (n <= 64) seg_regs<2>(d.perm + s0, n);
-            else if (n <= 128) seg_regs<4>(d.perm + s0, n);
-            else seg_regs<8>(d.perm + s0, n);
-            continue;
-        }
-        int m = 2 * SEG_LANES;
-        while (m < n) m <<= 1;
-        // a stretch whose slots the atomics happened to hand out in input order is done already
-        // (the common case when the input is the previous step's order)
-        bool sorted = true;
-        for (int k = lane; k < m; k += 32) {
-            const int v = k < n ? d.perm[s0 + k] : 0x7FFFFFFF;
-            w[k] = v;
-        }
-        __syncwarp();
-        for (int k = lane; k + 1 < n; k += 32) sorted &= w[k] < w[k + 1];
-        if (__all_sync(0xffffffffu, sorted)) {
-            __syncwarp();
-            continue;
-        }
-        for (int size = 2; size <= m; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int k = lane; k < m; k += 32) {
-                    const int j = k ^ stride;
-                    if (j > k) {
-                        const bool up = (k & size) == 0;
-                        const int x = w[k], y = w[j];
-                        if ((x > y) == up) {
-                            w[k] = y;
-                            w[j] = x;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        for (int k = lane; k < n; k += 32) d.perm[s0 + k] = w[k];
-        __syncwarp();
-    }
-    // longer stretches: a CTA each
+    __shared__ LongScratch<TPB> ls;
+    const int warp = threadIdx.x >> 5;
     const unsigned nhuge = d.glob->nhuge;
-    for (unsigned b = blockIdx.x; b < nhuge; b += gridDim.x) {
+    for (unsigned b = blockIdx.x; b < nhuge; b += gridDim.x) {  // a CTA each
         const int2 sg = d.bigseg[d.bigseg_cap - 1 - b];
-        cta_radix_sort<TPB>(d.perm + sg.x, d.slot + sg.x, sg.y, rs);
+        cta_sort<TPB>(d.perm + sg.x, d.slot + sg.x, sg.y, ls);
+    }
+    const unsigned nbig = d.glob->nbig;
+    for (unsigned e = (unsigned)(blockIdx.x * (TPB / 32) + warp); e < nbig; e += gridDim.x * (TPB / 32)) {  // a warp each
+        const int2 sg = d.bigseg[e];
+        seg_warp(d.perm + sg.x, sg.y);
     }
 }
 
@@ -1377,7 +1412,7 @@ struct ClusterSmem {
     union {
         struct {
             int2 big[2048];  // the CTA's long quadrants
-            RadixScratch<CL_THREADS> rs;
+            LongScratch<CL_THREADS> ls;
         } sort;
         struct {
             double cm[SUM_CELLS * 6], chm[4 * 64 * 6];
@@ -1615,14 +1650,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_tree_cluster(DevPlan d, int s
         for (int k = warp; k < nbig; k += CL_THREADS / 32) {
             const int2 sg = sm.u.sort.big[k];
             if (sg.y > SEG_LANES) continue;
-            if (sg.y <= 32) seg_regs<1>(d.perm + sg.x, sg.y);
-            else if (sg.y <= 64) seg_regs<2>(d.perm + sg.x, sg.y);
-            else if (sg.y <= 128) seg_regs<4>(d.perm + sg.x, sg.y);
-            else seg_regs<8>(d.perm + sg.x, sg.y);
+            seg_warp(d.perm + sg.x, sg.y);
         }
         for (int k = 0; k < nbig; k++) {
             const int2 sg = sm.u.sort.big[k];
-            if (sg.y > SEG_LANES) cta_radix_sort<CL_THREADS>(d.perm + sg.x, d.slot + sg.x, sg.y, sm.u.sort.rs);
+            if (sg.y > SEG_LANES) cta_sort<CL_THREADS>(d.perm + sg.x, d.slot + sg.x, sg.y, sm.u.sort.ls);
         }
     }
     cluster_sync();

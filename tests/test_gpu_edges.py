@@ -234,10 +234,11 @@ def test_store_returns_the_state(n, order):
 
 
 # The order within a quadrant is the input order whatever slots the placement handed out: quadrants at
-# the edges of the sorting forms (registers of a thread, of a warp, shared memory, a CTA), in random
-# input order against the same particles loaded in box order.
-@pytest.mark.parametrize("count", [2, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 1024, 1025, 3000])
-def test_quadrant_sort_sizes(count):
+# the edges of the sorting forms (registers of a thread, of a warp, merged runs, radix passes), in random
+# input order against the same particles loaded in box order; one system (the small-system kernel) and two.
+@pytest.mark.parametrize("systems", [1, 2])
+@pytest.mark.parametrize("count", [2, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 1024, 1025, 3000, 4096, 4097])
+def test_quadrant_sort_sizes(count, systems):
     from barneshut.gb300 import native, workloads
 
     rng = np.random.default_rng(count)
@@ -253,12 +254,12 @@ def test_quadrant_sort_sizes(count):
     prm = native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5, 1, quad_min=128)
 
     def accel(cols):
-        plan = native.Plan([n], [2], prm)
-        plan.load(*cols, z, z)
+        plan = native.Plan([n] * systems, [2] * systems, prm)
+        plan.load(*(np.tile(c, systems) for c in (*cols, z, z)))
         plan.step(1)
         out = plan.store()
         assert plan.error_flags() == 0
-        return torch.stack([out["ax"], out["ay"]]).cpu().numpy()
+        return torch.stack([out["ax"], out["ay"]]).cpu().numpy().reshape(2, systems, n)[:, -1]
 
     b = workloads.box_order(x, y, 2)
     assert np.array_equal(accel((x, y, m))[:, b], accel((x[b], y[b], m[b])))
