@@ -69,6 +69,7 @@ template <typename R> __device__ __forceinline__ void sum64_flush_r(Sum64 &s, R 
 
 // Frames of the systems' split floats from the extents of the last create_tree, a thread per system.
 __global__ void k_split_frames(DevPlan d) {
+    step_enter();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= d.nsys || d.sys[s].n == 0) return;
     const SysDyn &dy = d.dyn[s];
@@ -79,6 +80,7 @@ __global__ void k_split_frames(DevPlan d) {
 // The box-sorted particles as split floats, into the state buffer that is not current (free between
 // steps).  A particle that has left the extents since, or whose mass does not fit, leaves its system to FP64.
 __global__ void __launch_bounds__(256) k_split_convert(DevPlan d) {
+    step_enter();
     const int b = (d.glob->epoch + 1) & 1;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += (long long)gridDim.x * blockDim.x) {
         Split64 &fr = d.fsplit[find_seg(d.poff_tab, d.nsys, i)];
@@ -114,6 +116,7 @@ template <typename R> __host__ __device__ constexpr int src_bytes() {
 template <typename R, int NR, bool KAHAN, bool TEST, bool EXACT, int MINB, bool SPL = false>
 __global__ void __launch_bounds__(FT, MINB)
 k_force(DevPlan d, int tick, int accumulate) {
+    step_enter();
     using S = typename Src<R>::T;
     constexpr int SCAP = SPL ? SPLIT_CAP : SRC_CAP;  // near sources per pass
     constexpr bool F32 = sizeof(R) == 4;
@@ -784,7 +787,7 @@ static cudaError_t launch_force_nr(const DevPlan &d, bool accumulate, cudaStream
     static_assert(FT * FORCE_R >= TARGET_CHUNK, "a CTA's quads must cover every target of a work item");
     auto k = k_force<R, NR, KAHAN, TEST, EXACT, MINB>;
     const long long slots = (long long)d.nsm * MINB, grid = items_max * (FORCE_R / NR);
-    k<<<(unsigned)(grid < slots ? grid : slots), FT, force_smem<R>(), st>>>(d, 0, accumulate ? 1 : 0);
+    launch_step(k, (unsigned)(grid < slots ? grid : slots), FT, force_smem<R>(), st, d, 0, accumulate ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -812,14 +815,14 @@ static cudaError_t launch_force_t(const DevPlan &d, bool accumulate, cudaStream_
 template <bool TEST>
 static cudaError_t launch_force64(const DevPlan &d, bool accumulate, cudaStream_t st) {
     if (!force_splits(d.n_total)) return launch_force_t<double, false, TEST, false>(d, accumulate, st);
-    k_split_frames<<<(d.nsys + 127) / 128, 128, 0, st>>>(d);
+    launch_step(k_split_frames, (d.nsys + 127) / 128, 128, 0, st, d);
     const long long blocks = (d.n_total + 255) / 256, most = (long long)d.nsm * 16;
-    k_split_convert<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(d);
+    launch_step(k_split_convert, (unsigned)(blocks < most ? blocks : most), 256, 0, st, d);
     static_assert(SPLIT_CAP * sizeof(Src64) <= (size_t)SRC_CAP * src_bytes<double>(), "split sources fit the staging");
     static_assert(SPLIT_CAP * sizeof(int) <= NEAR_CAP * sizeof(float2), "and their indices the shifts' place");
     const long long slots = (long long)d.nsm * 4, items_max = d.NG_total + d.n_total / d.chunk + 1;
-    k_force<double, FORCE_R, false, TEST, false, 4, true>
-        <<<(unsigned)(items_max < slots ? items_max : slots), FT, force_smem<double>(), st>>>(d, 0, accumulate ? 1 : 0);
+    launch_step(k_force<double, FORCE_R, false, TEST, false, 4, true>, (unsigned)(items_max < slots ? items_max : slots), FT,
+                force_smem<double>(), st, d, 0, accumulate ? 1 : 0);
     return cudaGetLastError();
 }
 

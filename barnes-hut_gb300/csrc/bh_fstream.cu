@@ -102,6 +102,7 @@ __device__ __forceinline__ int2 stream_split(const int *hist) {
 
 template <bool KAHAN, int MINB, bool SPLIT>
 __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, int accumulate) {
+    step_enter();
     extern __shared__ __align__(128) unsigned char smem[];
     using Ly = FsLayout<MINB>;
     constexpr int WSRC = Ly::WSRC, WFAR = Ly::WFAR;
@@ -668,9 +669,9 @@ static cudaError_t launch_fstream_s(const DevPlan &d, bool tick, bool accumulate
     if (grid < 1) grid = 1;
     cudaError_t e = cudaSuccess;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
-    k_fstream<KAHAN, MINB, SPLIT>
-        <<<(unsigned)grid, FW * 32, FsLayout<MINB>::SMEM, st>>>(d, tick ? 1 : 0, accumulate ? 1 : 0);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_step(k_fstream<KAHAN, MINB, SPLIT>, (unsigned)grid, FW * 32, FsLayout<MINB>::SMEM, st, d, tick ? 1 : 0,
+                    accumulate ? 1 : 0);
+    if (e != cudaSuccess) return e;
     return ev ? cudaEventRecord(ev[1], st) : cudaSuccess;
 }
 

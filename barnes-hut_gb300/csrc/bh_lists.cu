@@ -30,6 +30,7 @@ constexpr int LW = 4;  // warps per list-building CTA; one warp walks one group
 constexpr int LISTS_MINB = 8;
 
 __global__ void __launch_bounds__(LW * 32, LISTS_MINB) k_lists(DevPlan d) {
+    step_enter();
     __shared__ __align__(16) int front[LW][2][FR_CAP];  // cells as x << 16 | y; near boxes as indices
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int(*fb)[FR_CAP] = front[warp];
@@ -221,6 +222,7 @@ __device__ __forceinline__ int item_cost_bucket(const DevPlan &d, long long item
 }
 
 __global__ void __launch_bounds__(256) k_item_hist(DevPlan d) {
+    step_enter();
     __shared__ int h[ITEM_BUCKETS];
     if (threadIdx.x < ITEM_BUCKETS) h[threadIdx.x] = 0;
     __syncthreads();
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(256) k_item_hist(DevPlan d) {
 }
 
 __global__ void __launch_bounds__(256) k_item_order(DevPlan d) {
+    step_enter();
     __shared__ int off[ITEM_BUCKETS], h[ITEM_BUCKETS], base[ITEM_BUCKETS];
     if (threadIdx.x == 0) {
         int o = 0;
@@ -271,6 +274,7 @@ __global__ void __launch_bounds__(256) k_item_order(DevPlan d) {
 constexpr int ORDER_THREADS = 1024, ORDER_MAX = 8192;
 
 __global__ void __launch_bounds__(ORDER_THREADS) k_item_order_few(DevPlan d) {
+    step_enter();
     __shared__ int h[ITEM_BUCKETS], cur[ITEM_BUCKETS];
     __shared__ unsigned char cost[ORDER_MAX];
     const int tid = threadIdx.x;
@@ -297,17 +301,17 @@ cudaError_t launch_lists(const DevPlan &d, cudaStream_t st) {
     if (d.NG_total == 0) return cudaSuccess;
     long long grid = (long long)d.nsm * LISTS_MINB;
     if (grid * LW > d.NG_total) grid = (d.NG_total + LW - 1) / LW;
-    k_lists<<<(unsigned)grid, LW * 32, 0, st>>>(d);
+    launch_step(k_lists, (unsigned)grid, LW * 32, 0, st, d);
     const long long items_max = d.NG_total + d.n_total / d.dense_min +
                                 (d.quad_min > 0 ? 4 * (d.n_total / d.quad_min) : 0) + d.n_total / STREAM_ITEM_DIV + 1;  // >= items
     if (list_kernels(items_max) == 2) {
-        k_item_order_few<<<1, ORDER_THREADS, 0, st>>>(d);
+        launch_step(k_item_order_few, 1, ORDER_THREADS, 0, st, d);
         return cudaGetLastError();
     }
     long long ig = (items_max + 255) / 256;
     if (ig > (long long)d.nsm * 8) ig = (long long)d.nsm * 8;
-    k_item_hist<<<(unsigned)ig, 256, 0, st>>>(d);
-    k_item_order<<<(unsigned)ig, 256, 0, st>>>(d);
+    launch_step(k_item_hist, (unsigned)ig, 256, 0, st, d);
+    launch_step(k_item_order, (unsigned)ig, 256, 0, st, d);
     return cudaGetLastError();
 }
 

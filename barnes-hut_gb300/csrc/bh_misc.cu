@@ -20,6 +20,7 @@ static inline unsigned grid_of(long long n, int tpb, int nsm) {
 // zero (the host tracks it; k_store then writes zeros).
 __global__ void k_load(DevPlan d, const double *x, const double *y, const double *m,
                        const double *vx, const double *vy, long long rs) {
+    step_enter();
     const int b = (d.glob->epoch + 1) & 1;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride) {
@@ -44,6 +45,7 @@ __device__ __forceinline__ bool store_gathers(const DevPlan &d) {
 
 // inverse permutation of the current state into the key array, where k_store will gather
 __global__ void k_store_inverse(DevPlan d) {
+    step_enter();
     if (!store_gathers(d)) return;
     const int b = (d.glob->epoch + 1) & 1;
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -57,6 +59,7 @@ __global__ void k_store_inverse(DevPlan d) {
 // when no evaluation followed the last load (has_acc = 0).  gather: k_store_inverse ran before.
 __global__ void k_store(DevPlan d, double *rec, double *x, double *y, double *vx, double *vy,
                         double *ax, double *ay, int has_tree, int has_acc, int gather) {
+    step_enter();
     const int b = (d.glob->epoch + 1) & 1;
     long long stride = (long long)gridDim.x * blockDim.x;
     const bool inv = gather && store_gathers(d);
@@ -90,6 +93,7 @@ __global__ void k_store(DevPlan d, double *rec, double *x, double *y, double *vx
 // keep_acc: leave the accelerations in place (the fused step's tick, which keeps the last
 // evaluation's accelerations; the reference's tick, gpu/grid.py:159-174, zeroes them)
 __global__ void k_tick(DevPlan d, int keep_acc) {
+    step_enter();
     const int b = (d.glob->epoch + 1) & 1;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride) {
@@ -465,7 +469,7 @@ cudaError_t launch_box_com(const DevPlan &d, int sys, double *out, cudaStream_t 
 cudaError_t launch_load(const DevPlan &d, const double *x, const double *y, const double *m,
                         const double *vx, const double *vy, long long rs, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    k_load<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d, x, y, m, vx, vy, rs);
+    launch_step(k_load, grid_of(d.n_total, MT, d.nsm), MT, 0, st, d, x, y, m, vx, vy, rs);
     return cudaGetLastError();
 }
 
@@ -474,15 +478,15 @@ cudaError_t launch_store(const DevPlan &d, int has_tree, bool has_acc, double *r
     if (d.n_total == 0) return cudaSuccess;
     // (before the first create_tree the state is in pid order)
     const bool gather = has_tree && d.n_total >= STORE_GATHER_MIN;
-    if (gather) k_store_inverse<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d);
-    k_store<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d, rec, x, y, vx, vy, ax, ay, has_tree, has_acc ? 1 : 0,
-                                                           gather ? 1 : 0);
+    if (gather) launch_step(k_store_inverse, grid_of(d.n_total, MT, d.nsm), MT, 0, st, d);
+    launch_step(k_store, grid_of(d.n_total, MT, d.nsm), MT, 0, st, d, rec, x, y, vx, vy, ax, ay, has_tree, has_acc ? 1 : 0,
+                gather ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_tick(const DevPlan &d, cudaStream_t st, bool keep_acc) {
     if (d.n_total == 0) return cudaSuccess;
-    k_tick<<<grid_of(d.n_total, MT, d.nsm), MT, 0, st>>>(d, keep_acc ? 1 : 0);
+    launch_step(k_tick, grid_of(d.n_total, MT, d.nsm), MT, 0, st, d, keep_acc ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -26,6 +26,7 @@ static inline unsigned grid_for(long long n, int tpb, long long cap) {
 // Zero the box and quadrant histograms, reset the bounding-box accumulators and
 // pair counters, advance the state epoch.
 __global__ void k_prologue(DevPlan d) {
+    step_enter();
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     if (tid == 0) {
@@ -113,6 +114,7 @@ __device__ __forceinline__ void bbox_block_commit(const DevPlan &d, int s, unsig
 }
 
 __global__ void __launch_bounds__(TPB) k_bbox(DevPlan d) {
+    step_enter();
     const int cur = d.glob->epoch & 1;
     const double *X = d.X[cur], *Y = d.Y[cur];
     __shared__ unsigned long long red[4][TPB / 32];
@@ -240,6 +242,7 @@ constexpr int PLACE_PP = 4;  // consecutive particles per thread
 
 // (64 registers: 4 CTAs per SM)
 __global__ void __launch_bounds__(TPB, 4) k_place(DevPlan d) {
+    step_enter();
     constexpr int PT = TPB * PLACE_PP;  // particles per block round
     __shared__ int skeys[PT + 1], runold[PT], wmax[TPB / 32];
     const int cur = d.glob->epoch & 1;
@@ -455,6 +458,7 @@ __device__ int lookback(unsigned long long *state, int tile, unsigned gen, int a
 template <bool QSUM>
 __global__ void __launch_bounds__(TPB) k_scan_lookback(const int *in, long long n, int *out,
                                                       unsigned long long *state, Globals *glob, int k) {
+    step_enter();
     __shared__ int sh[32];
     __shared__ int s_tile, s_excl;
     __shared__ unsigned s_gen;
@@ -505,9 +509,9 @@ static cudaError_t scan_excl(const int *in, int *out, long long n, unsigned long
     long long ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (ntiles < 1) ntiles = 1;
     if (qsum)
-        k_scan_lookback<true><<<(unsigned)ntiles, TPB, 0, st>>>(in, n, out, state, glob, k);
+        launch_step(k_scan_lookback<true>, (unsigned)ntiles, TPB, 0, st, in, n, out, state, glob, k);
     else
-        k_scan_lookback<false><<<(unsigned)ntiles, TPB, 0, st>>>(in, n, out, state, glob, k);
+        launch_step(k_scan_lookback<false>, (unsigned)ntiles, TPB, 0, st, in, n, out, state, glob, k);
     return cudaGetLastError();
 }
 
@@ -515,6 +519,7 @@ static cudaError_t scan_excl(const int *in, int *out, long long n, unsigned long
 // Force work items: a target group with nt targets is split into
 // ceil(nt / TARGET_CHUNK) items so that dense groups spread over many CTAs.
 __global__ void __launch_bounds__(TPB) k_group_items(DevPlan d) {
+    step_enter();
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < d.NG_total; g += stride) {
         int s = find_seg(d.goff_tab, d.nsys, g);
@@ -533,6 +538,7 @@ __global__ void __launch_bounds__(TPB) k_group_items(DevPlan d) {
 }
 
 __global__ void __launch_bounds__(TPB) k_fill_items(DevPlan d) {
+    step_enter();
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < d.NG_total; g += stride) {
         int o = d.item_off[g], c = d.item_cnt[g];
@@ -648,6 +654,7 @@ __device__ __forceinline__ void group_items_write(const DevPlan &d, long long g,
 }
 
 __global__ void __launch_bounds__(SITEM_WARPS * 32) k_sitems(DevPlan d) {
+    step_enter();
     __shared__ int wtot[SITEM_WARPS], wpre[SITEM_WARPS];
     __shared__ int s_tile, s_excl;
     __shared__ unsigned s_gen;
@@ -711,6 +718,7 @@ __device__ __forceinline__ int quad_first(const DevPlan &d, int key4) {
 }
 
 __global__ void __launch_bounds__(TPB) k_perm(DevPlan d) {
+    step_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += stride)
         d.perm[quad_first(d, d.key[i]) + d.slot[i]] = (int)i;
@@ -740,6 +748,7 @@ __device__ __forceinline__ void seg_thread(int *p, int n) {
 }
 
 __global__ void __launch_bounds__(TPB) k_segsort(DevPlan d) {
+    step_enter();
     const long long nq = 4 * d.B_total, stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += stride) {
         const int n = d.qcounts[q];
@@ -969,6 +978,7 @@ __device__ void cta_sort(int *p, int *tmp, int n, LongScratch<NT> &ls) {
 }
 
 __global__ void __launch_bounds__(TPB) k_segsort_big(DevPlan d) {
+    step_enter();
     __shared__ LongScratch<TPB> ls;
     const int warp = threadIdx.x >> 5;
     const unsigned nhuge = d.glob->nhuge;
@@ -1043,6 +1053,7 @@ __device__ __forceinline__ void leaf_chunk(const DevPlan &d, long long c, int ke
 // records when the leaf moments were overwritten since).
 template <bool SECOND>
 __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
+    step_enter();
     const int cur = d.glob->epoch & 1, nxt = cur ^ 1;
     const int lane = threadIdx.x & 31;
     // SU particles per thread per round, each stage's loads issued for all of them before the
@@ -1384,6 +1395,7 @@ __device__ __forceinline__ void summarize_tile(const DevPlan &d, long long t, in
 
 template <bool SECOND>
 __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int leaves_given) {
+    step_enter();
     __shared__ double cm[SUM_CELLS * 6];
     __shared__ double chm[4 * 64 * 6];
     for (long long t = blockIdx.x; t < d.T_total; t += gridDim.x)
@@ -1496,6 +1508,7 @@ __device__ int cluster_stream_items(const DevPlan &d, ClusterSmem &sm, int g0, i
 }
 
 __global__ void __launch_bounds__(CL_THREADS, 1) k_tree_cluster(DevPlan d, int summary) {
+    step_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ClusterSmem &sm = *reinterpret_cast<ClusterSmem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1708,17 +1721,20 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_tree_cluster(DevPlan d, int s
 
 // ------------------------------------------------------------------ launches
 // Launch of k_tree_cluster: 16 CTAs where the device keeps a cluster that large, else 8.
-static cudaError_t cluster_config(cudaLaunchConfig_t &c, cudaLaunchAttribute &a, int ctas, cudaStream_t st) {
+static cudaError_t cluster_config(cudaLaunchConfig_t &c, cudaLaunchAttribute a[2], int ctas, cudaStream_t st) {
     memset(&c, 0, sizeof(c));
-    a.id = cudaLaunchAttributeClusterDimension;
-    a.val.clusterDim.x = ctas;
-    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    memset(a, 0, 2 * sizeof(a[0]));
+    a[0].id = cudaLaunchAttributeClusterDimension;
+    a[0].val.clusterDim.x = ctas;
+    a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+    a[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (launch_step)
+    a[1].val.programmaticStreamSerializationAllowed = 1;
     c.gridDim = dim3(ctas);
     c.blockDim = dim3(CL_THREADS);
     c.dynamicSmemBytes = sizeof(ClusterSmem);
     c.stream = st;
-    c.attrs = &a;
-    c.numAttrs = 1;
+    c.attrs = a;
+    c.numAttrs = 2;
     return cudaSuccess;
 }
 cudaError_t tree_init(int *ctas) {
@@ -1727,7 +1743,7 @@ cudaError_t tree_init(int *ctas) {
     e = cudaFuncSetAttribute(k_tree_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t c;
-    cudaLaunchAttribute a;
+    cudaLaunchAttribute a[2];
     cluster_config(c, a, 16, nullptr);
     int fit = 0;
     *ctas = cudaOccupancyMaxActiveClusters(&fit, k_tree_cluster, &c) == cudaSuccess && fit > 0 ? 16 : 8;
@@ -1736,24 +1752,25 @@ cudaError_t tree_init(int *ctas) {
 }
 cudaError_t launch_tree_cluster(const DevPlan &d, bool summary, cudaStream_t st) {
     cudaLaunchConfig_t c;
-    cudaLaunchAttribute a;
+    cudaLaunchAttribute a[2];
     cluster_config(c, a, d.cl_ctas, st);
     return cudaLaunchKernelEx(&c, k_tree_cluster, d, summary ? 1 : 0);
 }
 cudaError_t launch_prologue(const DevPlan &d, cudaStream_t st) {
     long long n = d.B_total > d.nsys ? d.B_total : d.nsys;
-    k_prologue<<<grid_for(n, TPB, d.nsm * 16LL), TPB, 0, st>>>(d);
+    launch_step(k_prologue, grid_for(n, TPB, d.nsm * 16LL), TPB, 0, st, d);
     return cudaGetLastError();
 }
 cudaError_t launch_bbox(const DevPlan &d, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
     // (a block per 2,048 particles at least: its five atomics meet every other block's)
-    k_bbox<<<grid_for(d.n_total, TPB * (d.nsys == 1 ? 8 : 16), d.nsm * (d.nsys == 1 ? 4LL : 8LL)), TPB, 0, st>>>(d);
+    launch_step(k_bbox, grid_for(d.n_total, TPB * (d.nsys == 1 ? 8 : 16), d.nsm * (d.nsys == 1 ? 4LL : 8LL)), TPB, 0, st,
+                d);
     return cudaGetLastError();
 }
 cudaError_t launch_place(const DevPlan &d, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    k_place<<<grid_for(d.n_total, TPB * PLACE_PP, d.nsm * 8LL), TPB, 0, st>>>(d);
+    launch_step(k_place, grid_for(d.n_total, TPB * PLACE_PP, d.nsm * 8LL), TPB, 0, st, d);
     return cudaGetLastError();
 }
 cudaError_t launch_scan(const DevPlan &d, cudaStream_t st) {
@@ -1765,7 +1782,7 @@ cudaError_t launch_walk_items(const DevPlan &d, cudaStream_t st) {
     k_group_items<<<g, TPB, 0, st>>>(d);
     cudaError_t e = scan_excl(d.item_cnt, d.item_off, d.NG_total, d.sst_witem, d.glob, 1, st);
     if (e != cudaSuccess) return e;
-    k_fill_items<<<g, TPB, 0, st>>>(d);
+    launch_step(k_fill_items, g, TPB, 0, st, d);
     return cudaGetLastError();
 }
 // The step's work items: the walk items where the walk or the learned correction runs, the
@@ -1784,11 +1801,11 @@ cudaError_t launch_items(const DevPlan &d, cudaStream_t st) {
 }
 cudaError_t launch_scatter(const DevPlan &d, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
-    k_perm<<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
-    k_segsort<<<grid_for(4 * d.B_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
-    k_segsort_big<<<(unsigned)(d.nsm * 4), TPB, 0, st>>>(d);
-    if (d.learned) k_gather<true><<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
-    else k_gather<false><<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
+    launch_step(k_perm, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
+    launch_step(k_segsort, grid_for(4 * d.B_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
+    launch_step(k_segsort_big, (unsigned)(d.nsm * 4), TPB, 0, st, d);
+    if (d.learned) launch_step(k_gather<true>, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
+    else launch_step(k_gather<false>, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
     return cudaGetLastError();
 }
 // leaves: the leaf sums of k_gather were overwritten since (bh_set_leaf_moments): redo them

@@ -430,3 +430,52 @@ def test_fp64_forces_in_split_floats(kind, theta, eps, cutoff):
         w[i] = 0.0
         ref = np.array([np.sum(w * dx), np.sum(w * dy)])
         assert np.linalg.norm(got[:, i] - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+# Kernels set up while their predecessor runs still wait for everything before them: tensors written on
+# another stream that the plan's stream was made to wait for (after kernels of its own), and a step captured
+# in a caller's graph, whole call sequence and all, give the results of a plain sequence.
+@pytest.mark.parametrize("n,grid", [(10000, 16), (40000, 32)])
+def test_launches_wait_for_other_streams_and_capture(n, grid):
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(n)
+    prm = native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5, 1)
+    sets = [[torch.from_numpy(rng.random(n)).cuda() for _ in range(3)] for _ in range(2)]
+    z = torch.zeros(n, dtype=torch.float64, device="cuda")
+
+    def run(plan, s):
+        plan.load(*s, z, z)
+        plan.step(2)
+        out = plan.store()
+        return torch.stack([out[k] for k in ("x", "y", "vx", "vy", "ax", "ay")])
+
+    plan = native.Plan([n], [grid], prm)
+    want = [run(plan, s).clone() for s in sets]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    cols = [torch.empty_like(c) for c in sets[0]]
+    big = torch.ones(64 << 20, device="cuda")
+    torch.cuda.synchronize()
+    got = []
+    for k in range(6):
+        with torch.cuda.stream(b):
+            for _ in range(4):
+                big.mul_(1.0)  # keeps the copies below late
+            for c, src in zip(cols, sets[k & 1]):
+                c.copy_(src)
+        with torch.cuda.stream(a):
+            a.wait_stream(b)
+            got.append(run(plan, cols))
+        b.wait_stream(a)
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[k & 1]) for k, g in enumerate(got))
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = run(plan, cols)
+    for k in range(4):
+        for c, src in zip(cols, sets[k & 1]):
+            c.copy_(src)
+        g.replay()
+        assert torch.equal(out, want[k & 1])
+    assert plan.error_flags() == 0
