@@ -253,8 +253,8 @@ struct LSmem {
 // 128, a group of 128 threads per tile.  Bound like the network's forward pass (mlp_group_forward);
 // the pairs are laid out cell by cell, so a warp's lanes read one cell's record at a time and add
 // their outputs to 32 different targets.  262,144 clustered particles, 128 x 128 boxes, theta 0.8
-// corrected below 0.5: 3,895 us -> 1,678 us (before: 8 warps per SM in target-major order, whose
-// shared-memory FP32 atomics met on one target).
+// corrected below 0.5: 3,895 us -> 1,230 us (1,678 with single bf16 conversions; before: 8 warps per
+// SM in target-major order, whose shared-memory FP32 atomics met on one target).
 __global__ void __launch_bounds__(128 * LG, LC_CTAS)
 k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *params, int tick) {
     constexpr int NT = 128 * LG;

@@ -78,9 +78,9 @@ __device__ __forceinline__ void load_bias(float *bias, const float *params) {
 }
 
 // out[r] = MLP(feats[r][0..5]) for r < P; feats row stride fs floats, out row stride 2.
-// 1,000,003 rows, stride 8: 119 us -> 101 us (one 128-thread tile per CTA, scalar epilogue and
-// the whole accumulator row in registers before); 107 us as two CTAs of four groups, 111 as four of
-// two (each stages the weights); 81 us is the MUFU pipe's time for the tanh.
+// 1,000,003 rows, stride 8: 119 us -> 70 us (one 128-thread tile per CTA, scalar epilogue, single
+// conversions and the whole accumulator row in registers before; 101 us with single conversions, when
+// two CTAs of four groups took 107 and four of two 111: each stages the weights).
 __global__ void __launch_bounds__(128 * INFER_GROUPS, INFER_CTAS)
 k_mlp_infer(const float *feats, int fs, long long P, const uint8_t *img, const float *params, float *out,
             unsigned *err) {
@@ -216,8 +216,9 @@ __device__ __forceinline__ void add16(float *grad, const float *g, bool vec) {
 // operands take 143 KB) and the epilogues' FP32 work.  16 warps share a tile, a thread 16 columns
 // of one row, so an epilogue is a sixteenth of the row's work a thread; gelu' is formed with gelu
 // (one tanh) and kept in registers until the way back; the biases' gradients are FP32 column sums
-// by shuffles.  65,536 rows: 3,789 us -> 33 us (before: shared-memory FP32 atomics, 32 lanes to one
-// address, and scattered 2-byte stores of transposed copies of every operand).
+// by shuffles.  65,536 rows, the training step: 3,790 us -> 35 us (39 with single bf16 conversions;
+// before: shared-memory FP32 atomics, 32 lanes to one address, and scattered 2-byte stores of
+// transposed copies of every operand).
 __global__ void __launch_bounds__(TT, 1) k_mlp_train(const float *feats, int fs, const float *targets,
                                                      long long P, const uint8_t *img,
                                                      const float *params, float *grad, float *loss,
@@ -324,9 +325,9 @@ __global__ void __launch_bounds__(TT, 1) k_mlp_train(const float *feats, int fs,
         float yt[2] = {tg[0], tg[1]};
         if (cg == 0) {
             uint4 w;
-            w.x = (uint32_t)bf16_bits(f[0]) | ((uint32_t)bf16_bits(f[1]) << 16);
-            w.y = (uint32_t)bf16_bits(f[2]) | ((uint32_t)bf16_bits(f[3]) << 16);
-            w.z = (uint32_t)bf16_bits(f[4]) | ((uint32_t)bf16_bits(f[5]) << 16);
+            w.x = bf16x2_bits(f[0], f[1]);
+            w.y = bf16x2_bits(f[2], f[3]);
+            w.z = bf16x2_bits(f[4], f[5]);
             w.w = 0u;
             *reinterpret_cast<uint4 *>(sm + L::T03 + tc::kmajor_off(r, 0, KC03)) = w;
             if (t + gridDim.x < ntiles) load(t + gridDim.x);  // in flight while this tile runs
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(TT, 1) k_mlp_train(const float *feats, int fs,
                 gb4[k] += dy[k];
             }
             *reinterpret_cast<uint32_t *>(sm + L::D14 + tc::kmajor_off(r, 64, KC03)) =
-                (uint32_t)bf16_bits(dy[0]) | ((uint32_t)bf16_bits(dy[1]) << 16);
+                bf16x2_bits(dy[0], dy[1]);
         }
         round([&] {  // da3 = dh4 W4^T
             tc::mma(tm + T_DA, tc::kdesc(d14 + 8 * 128, KC03, 0), tc::kdesc(sW + I_B4T, 2, 0), tc::idesc_bf16(128, 64), 0);
