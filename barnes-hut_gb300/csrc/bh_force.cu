@@ -154,8 +154,15 @@ k_force(DevPlan d, int tick, int accumulate) {
         __syncthreads();
     }
 
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(&d.glob->item_next, 1u);
+    // Half items are few: a CTA's first one is its own index, so that they spread over all SMs.  Taken from the
+    // queue, they went to the CTAs that started first: 100,003 particles on 12 x 12 boxes, flat, no cutoff, 576
+    // of them to 115 of 152 SMs, the round 472 us against 385; 131,072 clustered on 16 x 16 boxes, theta 0.5,
+    // 2,900 against 1,949.  Not with EXACT (5,000 on 3 x 3 boxes: 388 us from the queue, 400 so; 60,000 on
+    // 10 x 10: 551 and 561; 100,003: 724 and 672), nor for whole items (130,000 on 24 x 24: 494 and 534).
+    constexpr bool SPREAD = PARTS > 1 && !EXACT;
+    for (bool first = SPREAD;; first = false) {
+        if (tid == 0)
+            s_item = first ? (int)blockIdx.x : (int)((SPREAD ? gridDim.x : 0u) + atomicAdd(&d.glob->item_next, 1u));
         __syncthreads();
         const int item = s_item / PARTS, part = s_item - item * PARTS;
         if (item >= nitems) break;

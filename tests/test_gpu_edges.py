@@ -479,3 +479,29 @@ def test_launches_wait_for_other_streams_and_capture(n, grid):
         g.replay()
         assert torch.equal(out, want[k & 1])
     assert plan.error_flags() == 0
+
+
+# Queues of fewer entries than CTAs or warps, of as many, and of more: every item is taken once (all pairs
+# are near with 2 x 2 boxes) and the accelerations match FP64 sums.  Tolerance: FP32
+# pairs of 3e-7 and FP32 sums of at most n terms (a random walk of 2^-24 steps).
+@pytest.mark.parametrize("n", [1, 5, 129, 1025, 6007])
+@pytest.mark.parametrize("theta", [0.0, 0.5])
+def test_queue_entries_taken_once(n, theta):
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(n)
+    x, y, m = rng.random(n), rng.random(n), rng.uniform(1, 2, n)
+    z = np.zeros(n)
+    plan = native.Plan([n], [2], native.make_params(1.0, 1e-5, 1e-3, 0.0, theta))
+    for _ in range(2):  # the queue starts again for the next launch
+        plan.load(x, y, m, z, z)
+        plan.create_tree()
+        plan.summarize()
+        plan.evaluate()
+        out = plan.store()
+        dx, dy = x[None, :] - x[:, None], y[None, :] - y[:, None]
+        w = m[None, :] / (dx * dx + dy * dy + 1e-6)
+        got = np.stack([out["ax"].cpu().numpy(), out["ay"].cpu().numpy()])
+        ref = np.stack([(w * dx).sum(1), (w * dy).sum(1)])
+        assert np.sqrt(((got - ref) ** 2).sum()) <= 1e-5 * max(np.sqrt((ref ** 2).sum()), 1e-30)
+    assert plan.error_flags() == 0
