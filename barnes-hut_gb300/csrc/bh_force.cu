@@ -155,11 +155,10 @@ k_force(DevPlan d, int tick, int accumulate) {
     }
 
     // Half items are few: a CTA's first one is its own index, so that they spread over all SMs.  Taken from the
-    // queue, they went to the CTAs that started first: 100,003 particles on 12 x 12 boxes, flat, no cutoff, 576
-    // of them to 115 of 152 SMs, the round 472 us against 385; 131,072 clustered on 16 x 16 boxes, theta 0.5,
-    // 2,900 against 1,949.  Not with EXACT (5,000 on 3 x 3 boxes: 388 us from the queue, 400 so; 60,000 on
-    // 10 x 10: 551 and 561; 100,003: 724 and 672), nor for whole items (130,000 on 24 x 24: 494 and 534).
-    constexpr bool SPREAD = PARTS > 1 && !EXACT;
+    // queue, they went to the CTAs that started first: 100,003 particles on 12 x 12 boxes, flat, 576 of them to
+    // 115 of 152 SMs, the round 472 us against 385 without a cutoff, 542 against 460 with one; 131,072 clustered
+    // on 16 x 16 boxes, theta 0.5, 2,900 against 1,949.  Not for whole items (130,000 on 24 x 24: 494 and 534).
+    constexpr bool SPREAD = PARTS > 1;
     for (bool first = SPREAD;; first = false) {
         if (tid == 0)
             s_item = first ? (int)blockIdx.x : (int)((SPREAD ? gridDim.x : 0u) + atomicAdd(&d.glob->item_next, 1u));
@@ -482,8 +481,7 @@ k_force(DevPlan d, int tick, int accumulate) {
                 __syncthreads();
                 if (active && F32) {
                     const float4 *s4 = reinterpret_cast<const float4 *>(src);
-#pragma unroll 16 / NR
-                    for (int j = slice; j < ns; j += nslice) {
+                    auto sweep1 = [&](int j) {
                         const ulonglong2 sxy = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j);
                         const ulonglong2 smi = *reinterpret_cast<const ulonglong2 *>(s4 + 2 * j + 1);
                         const int sidx = (int)(unsigned)smi.y;
@@ -494,6 +492,56 @@ k_force(DevPlan d, int tick, int accumulate) {
                             nax2[kk] = f2_fma(w, dx, nax2[kk]);
                             nay2[kk] = f2_fma(w, dyy, nay2[kk]);
                         }
+                    };
+                    if constexpr (EXACT) {
+                        // U sources at a time with the FP32 predicate alone, one branch for all of them:
+                        // a group with a pair near the cutoff is swept again, source by source.  A branch
+                        // per pair left no two pairs in flight: cutoff 1e-5, flat, 5,000 particles on 3 x 3
+                        // boxes 388 -> 202 us, 100,003 on 12 x 12 724 -> 542, 200,000 on 17 x 17 1,320 ->
+                        // 787.  (U = 4 | 8 with two targets a thread: 229 | 202 and 581 | 543; 2 | 4 with
+                        // four: 788 | 835 at 200,000.)
+                        constexpr int U = NR == 2 ? 8 : 2;
+                        const float cutf = (float)cut, band = cutf * 1e-3f;
+                        int j = slice;
+                        for (; j + (U - 1) * nslice < ns; j += U * nslice) {
+                            f2_t dx[U][NR / 2], dyy[U][NR / 2], w[U][NR / 2];
+                            bool close = false;
+#pragma unroll
+                            for (int u = 0; u < U; u++) {
+                                const float4 *e = s4 + 2 * (j + u * nslice);
+                                const ulonglong2 sxy = *reinterpret_cast<const ulonglong2 *>(e);
+                                const f2_t mm = *reinterpret_cast<const f2_t *>(e + 1);
+#pragma unroll
+                                for (int kk = 0; kk < NR / 2; kk++) {
+                                    dx[u][kk] = f2_add(sxy.x, ntx2[kk]);
+                                    dyy[u][kk] = f2_add(sxy.y, nty2[kk]);
+                                    const f2_t r2 = f2_fma(dx[u][kk], dx[u][kk], f2_mul(dyy[u][kk], dyy[u][kk]));
+                                    float i0, i1, r0, r1;
+                                    f2_unpack(f2_rcp(f2_add(r2, eps2x2)), i0, i1);
+                                    f2_unpack(r2, r0, r1);
+                                    close |= fabsf(r0 - cutf) <= band;
+                                    close |= fabsf(r1 - cutf) <= band;
+                                    w[u][kk] = f2_mul(mm, f2_pack(r0 > cutf ? i0 : 0.f, r1 > cutf ? i1 : 0.f));
+                                }
+                            }
+                            if (close) {
+#pragma unroll 1
+                                for (int u = 0; u < U; u++) sweep1(j + u * nslice);
+                                continue;
+                            }
+#pragma unroll
+                            for (int u = 0; u < U; u++)
+#pragma unroll
+                                for (int kk = 0; kk < NR / 2; kk++) {
+                                    nax2[kk] = f2_fma(w[u][kk], dx[u][kk], nax2[kk]);
+                                    nay2[kk] = f2_fma(w[u][kk], dyy[u][kk], nay2[kk]);
+                                }
+                        }
+#pragma unroll 1
+                        for (; j < ns; j += nslice) sweep1(j);
+                    } else {
+#pragma unroll 16 / NR
+                        for (int j = slice; j < ns; j += nslice) sweep1(j);
                     }
                 } else if (active && SPL) {
                     const int *sidx = reinterpret_cast<const int *>(nshift);

@@ -481,9 +481,9 @@ def test_launches_wait_for_other_streams_and_capture(n, grid):
     assert plan.error_flags() == 0
 
 
-# Queues of fewer entries than CTAs or warps, of as many, and of more: every item is taken once (all pairs
-# are near with 2 x 2 boxes) and the accelerations match FP64 sums.  Tolerance: FP32
-# pairs of 3e-7 and FP32 sums of at most n terms (a random walk of 2^-24 steps).
+# Queues of fewer entries than CTAs or warps, of as many, and of more: every item is taken once and the
+# accelerations match FP64 sums (all pairs are near with 2 x 2 boxes).  Tolerance: FP32 pairs of 3e-7 and FP32
+# sums of at most n terms (a random walk of 2^-24 steps).
 @pytest.mark.parametrize("n", [1, 5, 129, 1025, 6007])
 @pytest.mark.parametrize("theta", [0.0, 0.5])
 def test_queue_entries_taken_once(n, theta):
@@ -504,4 +504,31 @@ def test_queue_entries_taken_once(n, theta):
         got = np.stack([out["ax"].cpu().numpy(), out["ay"].cpu().numpy()])
         ref = np.stack([(w * dx).sum(1), (w * dy).sum(1)])
         assert np.sqrt(((got - ref) ** 2).sum()) <= 1e-5 * max(np.sqrt((ref ** 2).sum()), 1e-30)
+    assert plan.error_flags() == 0
+
+
+# Pairs at the cutoff: a jittered lattice whose neighbours' r^2 straddles it by parts in 1e7, where the FP64
+# positions decide, in half items (few groups) and whole ones (20 x 20 groups), with groups of sources and the
+# remainders of a slice.  A wrong decision changes a force by m / r, a thousand times the tolerance (that of
+# FP32 pairs and sums against FP64 ones).
+@pytest.mark.parametrize("side,grid", [(3, 1), (9, 1), (23, 2), (60, 3), (80, 20), (101, 21)])
+def test_cutoff_decided_in_groups(side, grid):
+    from barneshut.gb300 import native
+    from oracle import oracle
+
+    rng = np.random.default_rng(side)
+    h = np.sqrt(1e-5)
+    i, j = np.meshgrid(np.arange(side), np.arange(side))
+    x = (i.ravel() + rng.uniform(-1, 1, side * side) * 1e-7) * h + 0.25
+    y = (j.ravel() + rng.uniform(-1, 1, side * side) * 1e-7) * h + 0.5
+    m = rng.uniform(1, 2, side * side)
+    z = np.zeros(side * side)
+    plan = native.Plan([side * side], [grid], native.make_params(1.0, 1e-5, 0.0, 1e-5, 0.0))
+    plan.load(x, y, m, z, z)
+    plan.create_tree()
+    plan.summarize()
+    plan.evaluate()
+    out = plan.store()
+    ref = oracle.reference_evaluate(x, y, m, G=grid, gconst=1.0)
+    assert oracle.rel_rms(out["ax"].cpu().numpy(), out["ay"].cpu().numpy(), ref["ax"], ref["ay"]) <= 1e-5
     assert plan.error_flags() == 0
