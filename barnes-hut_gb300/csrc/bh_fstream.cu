@@ -100,6 +100,20 @@ __device__ __forceinline__ int2 stream_split(const int *hist) {
     return make_int2(n4, n2);
 }
 
+// Whether the heaviest item costs more than a warp's share of the whole (the same answer in every warp:
+// the histogram stands until the next step's lists).
+__device__ __forceinline__ bool stream_skewed(const int *hist, unsigned warps) {
+    const int lane = threadIdx.x & 31, h = hist[lane];
+    const float c = h > 0 ? ldexpf(1.5f, lane) : 0.f;
+    float w = (float)h * c, top = c;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        w += __shfl_xor_sync(0xffffffffu, w, o);
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    return top * (float)warps > w;
+}
+
 template <bool KAHAN, int MINB, bool SPLIT>
 __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, int accumulate) {
     step_enter();
@@ -138,17 +152,21 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
     const int2 split = SPLIT ? stream_split(d.item_bucket) : make_int2(0, 0);
     const long long nentry = nitems + 3LL * split.x + split.y;
     // lane 0 takes the queue slot of its next item one item ahead (the atomic's latency hides
-    // behind the current item).  Where items are few, a warp's first one is its place in the grid, so
-    // that the heaviest spread over all SMs instead of four by four over the CTAs that started first
-    // (10,000 particles, ten steps: 641 -> 621 us); long queues lose by it (4,194,304: +0.5 %).
+    // behind the current item).  Where items are few, or the heaviest outlast a warp's share of the
+    // whole, a warp's first one is its place in the grid, so that the heaviest spread over all SMs
+    // instead of four by four over the CTAs that started first (10,000 particles, ten steps: 641 ->
+    // 621 us; 1,048,576 left to collapse, a hundred steps: 5.7 -> 4.8 ms each); even queues lose by it
+    // (4,194,304: +0.5 %).
+    const bool spread = SPLIT || stream_skewed(d.item_bucket, gridDim.x * FW);
+    const unsigned qfirst = spread ? gridDim.x * FW : 0u;
     int qnext = blockIdx.x + warp * gridDim.x;
-    if (!SPLIT && lane == 0) qnext = (int)atomicAdd(&d.glob->item_next, 1u);
+    if (!spread && lane == 0) qnext = (int)atomicAdd(&d.glob->item_next, 1u);
     for (;;) {
         int item = -1, part = 0;  // part: 4 np + the part's first target within a quad
         if (lane == 0) {
             int q = qnext;
             if (q < nentry) {
-                qnext = (int)((SPLIT ? gridDim.x * FW : 0u) + atomicAdd(&d.glob->item_next, 1u));
+                qnext = (int)(qfirst + atomicAdd(&d.glob->item_next, 1u));
                 if (!SPLIT) {
                 } else if (q < 4 * split.x) {
                     part = 4 + (q & 3);
