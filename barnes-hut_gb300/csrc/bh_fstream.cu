@@ -699,8 +699,9 @@ static cudaError_t launch_fstream_s(const DevPlan &d, bool tick, bool accumulate
 // items, with fewer CTAs per SM: all items resident at once leave an SM's share of the cost to
 // chance (131,071 particles of one Gaussian: the busiest SM had twice the mean), two rounds or more
 // even it out.  131,071 particles, the step: 950 us with whole items on 24 warps per SM, 700 split,
-// 528 split on 8 warps (12 warps 557, 4 warps 603).  250,000 of one Gaussian: 1,941 us -> 1,273 with three CTAs (two 1,232, four 1,374); 400,000 clustered 689 -> 608 with four;
-// 1,048,576 clustered 981 with six whole, 983 with five, 1,098 with three.
+// 528 split on 8 warps (12 warps 557, 4 warps 603).  250,000 of one Gaussian: 1,941 us -> 1,273 with
+// three CTAs (two 1,232, four 1,374); 400,000 clustered 689 -> 608 with four; 1,048,576 clustered 981
+// with six whole, 983 with five, 1,098 with three.
 template <bool KAHAN, int MINB>
 static cudaError_t launch_fstream_t(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
                                     const cudaEvent_t *ev) {

@@ -1405,8 +1405,8 @@ __global__ void __launch_bounds__(SUM_THREADS, 7) k_summarize(DevPlan d, int lea
 // ------------------------------------------------------------------ small systems
 // create_tree (and, fused into a step, summarize) of one small system as one kernel: a cluster of
 // 16 CTAs runs the phases of k_prologue, k_bbox, k_place, the box scan, k_perm, k_segsort and
-// k_gather one after another with a cluster barrier between them, and makes the work items.  Bound: latency -- a phase is one or two dependent loads for every thread, and a
-// kernel of its own costs three to five microseconds, its launch and its ramp, where a barrier costs
+// k_gather one after another with a cluster barrier between them, and makes the work items.  Bound:
+// latency -- a phase is one or two dependent loads for every thread, and a kernel of its own costs three to five microseconds, its launch and its ramp, where a barrier costs
 // half of one.  Every result is the same bits: the phases are the same arithmetic over the same chunks,
 // and what depends on atomics (slots) is put in input order as in k_segsort.  10,000 particles on
 // 16 x 16 boxes, load, step and store: 87 us with the general kernels, 77 with this one; 20,000 in box
