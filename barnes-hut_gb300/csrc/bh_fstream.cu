@@ -152,12 +152,13 @@ __global__ void __launch_bounds__(FW * 32, MINB) k_fstream(DevPlan d, int tick, 
     const int2 split = SPLIT ? stream_split(d.item_bucket) : make_int2(0, 0);
     const long long nentry = nitems + 3LL * split.x + split.y;
     // lane 0 takes the queue slot of its next item one item ahead (the atomic's latency hides
-    // behind the current item).  Where items are few, or the heaviest outlast a warp's share of the
-    // whole, a warp's first one is its place in the grid, so that the heaviest spread over all SMs
-    // instead of four by four over the CTAs that started first (10,000 particles, ten steps: 641 ->
-    // 621 us; 1,048,576 left to collapse, a hundred steps: 5.7 -> 4.8 ms each); even queues lose by it
-    // (4,194,304: +0.5 %).
-    const bool spread = SPLIT || stream_skewed(d.item_bucket, gridDim.x * FW);
+    // behind the current item).  Where the heaviest items outlast a warp's share of the whole, a warp's
+    // first one is its place in the grid, so that the heaviest spread over all SMs instead of four by
+    // four over the CTAs that started first (10,000 particles, ten steps: 641 -> 621 us; 1,048,576 left
+    // to collapse, a hundred steps: 5.7 -> 4.8 ms each); other queues lose by it (4,194,304: +0.5 %;
+    // 131,071 of one Gaussian, split: 465 -> 480 us; but 250,000 clustered, split, four steps: 1,382 ->
+    // 1,356).
+    const bool spread = stream_skewed(d.item_bucket, gridDim.x * FW);
     const unsigned qfirst = spread ? gridDim.x * FW : 0u;
     int qnext = blockIdx.x + warp * gridDim.x;
     if (!spread && lane == 0) qnext = (int)atomicAdd(&d.glob->item_next, 1u);
