@@ -30,7 +30,7 @@ struct bh_plan {
     long long org_total = 0;  // entries of the box-origin tables (2 G per system)
     // workspace layout (byte offsets)
     size_t ws_bytes = 0;
-    size_t o_sys, o_dyn, o_glob, o_split, o_fsplit, o_poff, o_boff, o_coff, o_goff, o_toff, o_lvl;
+    size_t o_sys, o_dyn, o_glob, o_split, o_poff, o_boff, o_coff, o_goff, o_toff, o_lvl;
     size_t o_X[2], o_Y[2], o_VX[2], o_VY[2], o_M[2], o_PID[2];
     size_t o_AX, o_AY, o_key, o_slot, o_skey, o_bstart, o_sst, o_leafpart, o_perm, o_bigseg, o_icnt, o_ioff, o_igrp, o_mom, o_rec, o_PD,
         o_rec2, o_org, o_lfar, o_lnear, o_lcnt, o_iord, o_icost, o_ibkt, o_sicnt, o_sioff, o_sigrp, o_sisub, o_sichk, o_qcnt;
@@ -257,7 +257,6 @@ extern "C" int bh_plan_create(bh_plan **out, int nsys, const long long *n, const
     p->o_dyn = take(sizeof(SysDyn) * nsys);
     p->o_glob = take(sizeof(Globals));
     p->o_split = take(sizeof(Split64));
-    p->o_fsplit = take(pr.precision == BH_PREC_FP64 ? sizeof(Split64) * nsys : 0);
     p->o_poff = take(sizeof(long long) * (nsys + 1));
     p->o_boff = take(sizeof(long long) * (nsys + 1));
     p->o_coff = take(sizeof(long long) * (nsys + 1));
@@ -348,7 +347,6 @@ static void fill_dev(bh_plan *p) {
     d.dyn = (SysDyn *)(w + p->o_dyn);
     d.glob = (Globals *)(w + p->o_glob);
     d.split = (Split64 *)(w + p->o_split);
-    d.fsplit = (Split64 *)(w + p->o_fsplit);
     d.poff_tab = (const long long *)(w + p->o_poff);
     d.boff_tab = (const long long *)(w + p->o_boff);
     d.coff_tab = (const long long *)(w + p->o_coff);
@@ -706,8 +704,7 @@ extern "C" int bh_kernels_per_step(const bh_plan *p, int *count) {
     const int tree = cluster_tree(p) ? 1 : 1 + 1 + (walk_items ? 3 : 0) + 1 + (p->n_total > 0 ? 6 : 0) + (p->stream ? 1 : 0);
     const long long items_max = p->NG_total + p->n_total / p->dense_min +
                                 (p->quad_min > 0 ? 4 * (p->n_total / p->quad_min) : 0) + p->n_total / STREAM_ITEM_DIV + 1;
-    *count = tree + (p->n_total > 0 ? 1 : 0) + (p->stream && p->n_total > 0 ? list_kernels(items_max) : 0) + (!p->stream && p->n_total > 0 ? 1 : 0) +
-             (!p->stream && p->params.precision == BH_PREC_FP64 && force_splits(p->n_total) ? 2 : 0);
+    *count = tree + (p->n_total > 0 ? 1 : 0) + (p->stream && p->n_total > 0 ? list_kernels(items_max) : 0) + (!p->stream && p->n_total > 0 ? 1 : 0);
     return BH_OK;
 }
 

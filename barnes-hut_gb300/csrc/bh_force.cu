@@ -22,7 +22,6 @@
 // Positions are box-relative offsets rounded once from FP64, so dx keeps ~1e-7 of a box edge.
 #include "bh_internal.cuh"
 #include "bh_pairs.cuh"
-#include "bh_split64.cuh"
 #include "bh_tc.cuh"
 
 namespace bh {
@@ -37,64 +36,6 @@ __device__ __forceinline__ void src_get(const Src<double>::T &e, double &x, doub
     x = e.x; y = e.y; m = e.m; idx = e.idx;
 }
 
-
-constexpr int SPLIT_CAP = 192;  // near sources per pass in split floats (64 bytes each)
-
-// The split floats of a particle (in the state buffer that is not current, k_split_convert) as a
-// source and, two of them, as targets.
-__device__ __forceinline__ void src64_load(Src64 &e, const DevPlan &d, int old, int i) {
-    const float2 ax = reinterpret_cast<const float2 *>(d.X[old])[i], ay = reinterpret_cast<const float2 *>(d.Y[old])[i];
-    const float2 c = reinterpret_cast<const float2 *>(d.VX[old])[i], m = reinterpret_cast<const float2 *>(d.M[old])[i];
-    src64_make(e, make_float4(ax.x, ax.y, c.x, m.x), make_float4(ay.x, ay.y, c.y, m.y));
-}
-__device__ __forceinline__ void tgt64_load(Tgt64 &t, const DevPlan &d, int old, int i0, int i1) {
-    const float2 x0 = reinterpret_cast<const float2 *>(d.X[old])[i0], x1 = reinterpret_cast<const float2 *>(d.X[old])[i1];
-    const float2 y0 = reinterpret_cast<const float2 *>(d.Y[old])[i0], y1 = reinterpret_cast<const float2 *>(d.Y[old])[i1];
-    const float2 c0 = reinterpret_cast<const float2 *>(d.VX[old])[i0], c1 = reinterpret_cast<const float2 *>(d.VX[old])[i1];
-    t.ax = f2_pack(x0.x, x1.x);
-    t.bx = f2_pack(x0.y, x1.y);
-    t.cx = f2_pack(c0.x, c1.x);
-    t.ay = f2_pack(y0.x, y1.x);
-    t.by = f2_pack(y0.y, y1.y);
-    t.cy = f2_pack(c0.y, c1.y);
-}
-template <typename R> __device__ __forceinline__ void sum64_flush_r(Sum64 &s, R *x, R *y) {
-    double x0 = x[0], x1 = x[1], y0 = y[0], y1 = y[1];
-    sum64_flush(s, x0, x1, y0, y1);
-    x[0] = (R)x0;
-    x[1] = (R)x1;
-    y[0] = (R)y0;
-    y[1] = (R)y1;
-}
-
-// Frames of the systems' split floats from the extents of the last create_tree, a thread per system.
-__global__ void k_split_frames(DevPlan d) {
-    step_enter();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.nsys || d.sys[s].n == 0) return;
-    const SysDyn &dy = d.dyn[s];
-    split_setup(d.fsplit[s], unord_bits(dy.bbmin[0]), unord_bits(dy.bbmax[0]), unord_bits(dy.bbmin[1]),
-                unord_bits(dy.bbmax[1]), d.eps2);
-}
-
-// The box-sorted particles as split floats, into the state buffer that is not current (free between
-// steps).  A particle that has left the extents since, or whose mass does not fit, leaves its system to FP64.
-__global__ void __launch_bounds__(256) k_split_convert(DevPlan d) {
-    step_enter();
-    const int b = (d.glob->epoch + 1) & 1;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.n_total; i += (long long)gridDim.x * blockDim.x) {
-        Split64 &fr = d.fsplit[find_seg(d.poff_tab, d.nsys, i)];
-        const double vx = (d.X[b][i] - fr.cx) * fr.scale, vy = (d.Y[b][i] - fr.cy) * fr.scale;
-        float xa, xb, xc, ya, yb, yc, mh, ml;
-        split3(vx, xa, xb, xc);
-        split3(vy, ya, yb, yc);
-        if (!split_mass(d.M[b][i], mh, ml) || !(fabs(vx) <= 1.0) || !(fabs(vy) <= 1.0)) fr.usable = 0;
-        reinterpret_cast<float2 *>(d.X[b ^ 1])[i] = make_float2(xa, xb);
-        reinterpret_cast<float2 *>(d.Y[b ^ 1])[i] = make_float2(ya, yb);
-        reinterpret_cast<float2 *>(d.VX[b ^ 1])[i] = make_float2(xc, yc);
-        reinterpret_cast<float2 *>(d.M[b ^ 1])[i] = make_float2(mh, ml);
-    }
-}
 
 // bytes per staged far entry: the FP64 record, or (x, x, y, y) + (M, M) in FP32
 template <typename R> __host__ __device__ constexpr int far_bytes() {
@@ -111,14 +52,11 @@ template <typename R> __host__ __device__ constexpr int src_bytes() {
 // each taking half of every quad with the same slices, so every sum runs over the same terms in the
 // same order and the results are the same bits.  A plan whose items do not fill the chip takes
 // NR = 2 (launch_force).
-// SPL (FP64 only): the near pairs on the FP32 pipe in split floats (bh_split64.cuh), close ones in FP64;
-// far cells, some per cent of the pairs and each a larger share of the sum, stay in FP64.
-template <typename R, int NR, bool KAHAN, bool TEST, bool EXACT, int MINB, bool SPL = false>
+template <typename R, int NR, bool KAHAN, bool TEST, bool EXACT, int MINB>
 __global__ void __launch_bounds__(FT, MINB)
 k_force(DevPlan d, int tick, int accumulate) {
     step_enter();
     using S = typename Src<R>::T;
-    constexpr int SCAP = SPL ? SPLIT_CAP : SRC_CAP;  // near sources per pass
     constexpr bool F32 = sizeof(R) == 4;
     constexpr int PARTS = FORCE_R / NR;  // CTAs per item
     static_assert(NR % 2 == 0 && FORCE_R % NR == 0, "targets in packed pairs");
@@ -222,7 +160,7 @@ k_force(DevPlan d, int tick, int accumulate) {
                 int kx = lb / G, ky = lb - kx * G;
                 tx[r] = (R)__fadd_rn(__fmul_rn((float)(kx - gx0), step_f), p.x);
                 ty[r] = (R)__fadd_rn(__fmul_rn((float)(ky - gy0), step_f), p.z);
-            } else if constexpr (!SPL) {
+            } else {
                 tx[r] = (R)(Xs[ti[r]] - gox);
                 ty[r] = (R)(Ys[ti[r]] - goy);
             }
@@ -246,19 +184,6 @@ k_force(DevPlan d, int tick, int accumulate) {
             }
         }
 
-        // split floats: the lane's targets, the runs' sums and their length (anx, any_ hold all
-        // flushed sums, in the frame's units)
-        Tgt64 tg[NR / 2];
-        Sum64 sum[NR / 2];
-        const Split64 *fr = SPL ? d.fsplit + s : nullptr;
-        int run = 0;
-        if constexpr (SPL) {
-#pragma unroll
-            for (int k = 0; k < NR / 2; k++) {
-                tgt64_load(tg[k], d, nxt ^ 1, ti[2 * k], ti[2 * k + 1]);
-                sum64_zero(sum[k]);
-            }
-        }
         // FP64: 1 / (r^2 + eps^2), zero where the cutoff predicate on the unsoftened r^2 fails
         auto pair_inv64 = [&](double dx, double dyy) -> double {
             if (!TEST) return rcp64(dx * dx + (dyy * dyy + (double)eps2));
@@ -328,13 +253,6 @@ k_force(DevPlan d, int tick, int accumulate) {
                     }
                 }
             } else if (active) {
-                if constexpr (SPL) {  // (not kept in registers through the near sweeps)
-#pragma unroll
-                    for (int r = 0; r < NR; r++) {
-                        tx[r] = (R)(Xs[ti[r]] - gox);
-                        ty[r] = (R)(Ys[ti[r]] - goy);
-                    }
-                }
                 for (int k = slice; k < nf; k += nslice) {
                     double sx, sy, sm;
                     int sidx;
@@ -343,13 +261,8 @@ k_force(DevPlan d, int tick, int accumulate) {
                     for (int r = 0; r < NR; r++) {
                         const double dx = sx - (double)tx[r], dyy = sy - (double)ty[r];
                         const double w = sm * pair_inv64(dx, dyy);
-                        if constexpr (SPL) {  // (the mass is staged in the near sums' units)
-                            anx[r] += (R)(w * dx);
-                            any_[r] += (R)(w * dyy);
-                        } else {
-                            afx[r] += (R)(w * dx);
-                            afy[r] += (R)(w * dyy);
-                        }
+                        afx[r] += (R)(w * dx);
+                        afy[r] += (R)(w * dyy);
                     }
                 }
             }
@@ -380,8 +293,8 @@ k_force(DevPlan d, int tick, int accumulate) {
                 if (tid == 0) npre[nn] = total;
             }
             __syncthreads();
-            for (int s0 = 0; s0 < total && tma_ok; s0 += SCAP) {
-                const int ns = min(SCAP, total - s0);
+            for (int s0 = 0; s0 < total && tma_ok; s0 += SRC_CAP) {
+                const int ns = min(SRC_CAP, total - s0);
                 if (F32 && !TEST) {
                     // Bulk copies (TMA) of the 32-byte PD records of every near-box piece
                     // that falls into [s0, s0 + ns), all completing on one mbarrier phase.
@@ -465,9 +378,6 @@ k_force(DevPlan d, int tick, int accumulate) {
                         float4 *s4 = reinterpret_cast<float4 *>(src) + 2 * j;
                         s4[0] = make_float4(x, x, y, y);
                         s4[1] = pm;
-                    } else if constexpr (SPL) {
-                        src64_load(reinterpret_cast<Src64 *>(src)[j], d, nxt ^ 1, idx);
-                        reinterpret_cast<int *>(nshift)[j] = idx;
                     } else {
                         typename Src<double>::T q;
                         q.x = Xs[idx] - gox;
@@ -543,41 +453,6 @@ k_force(DevPlan d, int tick, int accumulate) {
 #pragma unroll 16 / NR
                         for (int j = slice; j < ns; j += nslice) sweep1(j);
                     }
-                } else if (active && SPL) {
-                    const int *sidx = reinterpret_cast<const int *>(nshift);
-                    // one pair in FP64, into the sums' units
-                    auto pair_fp64 = [&](int r, int j) {
-                        const double dx = Xs[j] - Xs[ti[r]], dyy = Ys[j] - Ys[ti[r]];
-                        const double r2 = dx * dx + dyy * dyy;
-                        if (TEST && !(r2 > d.cutoff)) return;
-                        const double w = Ms[j] * rcp64(r2 + d.eps2) * fr->inv_scale;
-                        anx[r] += (R)(w * dx);
-                        any_[r] += (R)(w * dyy);
-                    };
-                    if (fr->usable) {
-                        const f2_t eh = f2_dup(fr->eh), el = f2_dup(fr->el);
-                        // pairs within 2^-18 of the cutoff are decided in FP64, closer ones contribute nothing
-                        const float cs = TEST ? (float)(d.cutoff * fr->scale * fr->scale) : 0.f;
-                        const float lim = TEST ? fmaxf(SPLIT_LIM, cs * 1.000004f) : SPLIT_LIM;
-                        for (int j = slice; j < ns; j += nslice) {
-                            const Src64 e = reinterpret_cast<const Src64 *>(src)[j];
-#pragma unroll
-                            for (int k = 0; k < NR / 2; k++)
-                                pair64<true>(e, tg[k], eh, el, lim, sum[k], [&](int half, float r2) {
-                                    if (TEST && r2 >= SPLIT_LIM && r2 < cs * 0.999996f) return;
-                                    pair_fp64(2 * k + half, sidx[j]);
-                                });
-                            if (++run == SPLIT_RUN) {
-                                run = 0;
-#pragma unroll
-                                for (int k = 0; k < NR / 2; k++)
-                                    sum64_flush_r<R>(sum[k], anx + 2 * k, any_ + 2 * k);
-                            }
-                        }
-                    } else {
-                        for (int j = slice; j < ns; j += nslice)
-                            for (int r = 0; r < NR; r++) pair_fp64(r, sidx[j]);
-                    }
                 } else if (active) {
                     for (int j = slice; j < ns; j += nslice) {
                         double sx, sy, sm;
@@ -619,7 +494,7 @@ k_force(DevPlan d, int tick, int accumulate) {
                     double oy = box_origin(dy.miny, cj << l, dy.step) - goy;
                     e.x = ox + q[1] / q[0];
                     e.y = oy + q[2] / q[0];
-                    e.m = SPL ? q[0] * fr->inv_scale : q[0];
+                    e.m = q[0];
                     e.idx = id;
                     e.pad = 0;
                     reinterpret_cast<typename Src<double>::T *>(far)[pos] = e;
@@ -770,15 +645,6 @@ k_force(DevPlan d, int tick, int accumulate) {
                 acy[2 * k + 1] = (R)b1;
             }
         }
-        if constexpr (SPL) {
-#pragma unroll
-            for (int k = 0; k < NR / 2; k++) sum64_flush_r<R>(sum[k], anx + 2 * k, any_ + 2 * k);
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                anx[r] *= (R)fr->scale;
-                any_[r] *= (R)fr->scale;
-            }
-        }
         if (active) {
 #pragma unroll
             for (int r = 0; r < NR; r++) {
@@ -861,28 +727,6 @@ static cudaError_t launch_force_t(const DevPlan &d, bool accumulate, cudaStream_
     return launch_force_nr<R, FORCE_R, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);
 }
 
-// FP64 pairs: split floats for the near ones from SPLIT_FORCE_MIN particles on.  65,536 clustered
-// particles on 32 x 32 boxes: 6.5 ms -> 1.5 ms a step.  Relative error against quadruple precision where
-// every pair is near (2 x 2 boxes; uniform, clustered and far-off systems, softened and not): 8,192
-// particles 4-6e-16, 20,000: 3-5e-16, 60,000: 2-3e-16.  FP64 pairs of group-relative coordinates, in items
-// of 512 targets, had 2-3e-15 at 5,000, 4-6e-15 at 20,000 and 6-8e-15 at 60,000, and have 2-4e-16 in items
-// of 16 (sixteen times shorter sums).
-template <bool TEST>
-static cudaError_t launch_force64(const DevPlan &d, bool accumulate, cudaStream_t st) {
-    if (!force_splits(d.n_total)) return launch_force_t<double, false, TEST, false>(d, accumulate, st);
-    launch_step(k_split_frames, (d.nsys + 127) / 128, 128, 0, st, d);
-    const long long blocks = (d.n_total + 255) / 256, most = (long long)d.nsm * 16;
-    launch_step(k_split_convert, (unsigned)(blocks < most ? blocks : most), 256, 0, st, d);
-    static_assert(SPLIT_CAP * sizeof(Src64) <= (size_t)SRC_CAP * src_bytes<double>(), "split sources fit the staging");
-    static_assert(SPLIT_CAP * sizeof(int) <= NEAR_CAP * sizeof(float2), "and their indices the shifts' place");
-    const long long slots = (long long)d.nsm * 4, items_max = d.NG_total + d.n_total / d.chunk + 1;
-    launch_step(k_force<double, FORCE_R, false, TEST, false, 4, true>, (unsigned)(items_max < slots ? items_max : slots), FT,
-                force_smem<double>(), st, d, 0, accumulate ? 1 : 0);
-    return cudaGetLastError();
-}
-
-bool force_splits(long long n_total) { return n_total >= SPLIT_FORCE_MIN; }
-
 template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 4 : 8)>
 static cudaError_t init_force_t() {
     const int sm = (int)force_smem<R>();
@@ -898,12 +742,6 @@ static cudaError_t init_force_t() {
 cudaError_t force_init() {
     cudaError_t e;
     if ((e = fstream_init()) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_force<double, FORCE_R, false, true, false, 4, true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem<double>())) != cudaSuccess)
-        return e;
-    if ((e = cudaFuncSetAttribute(k_force<double, FORCE_R, false, false, false, 4, true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem<double>())) != cudaSuccess)
-        return e;
     if ((e = init_force_t<double, false, true, false>()) != cudaSuccess) return e;
     if ((e = init_force_t<double, false, false, false>()) != cudaSuccess) return e;
     if ((e = init_force_t<float, true, true, true>()) != cudaSuccess) return e;
@@ -931,7 +769,8 @@ cudaError_t launch_force(const DevPlan &d, bool tick, bool accumulate, cudaStrea
     const bool test = d.cutoff > 0.0 || d.eps2 == 0.0;
     const bool exact = d.cutoff > 0.0;
     if (d.prec == 2) {
-        e = test ? launch_force64<true>(d, accumulate, st) : launch_force64<false>(d, accumulate, st);
+        e = test ? launch_force_t<double, false, true, false>(d, accumulate, st)
+                 : launch_force_t<double, false, false, false>(d, accumulate, st);
     } else if (d.prec == 1) {
         if (exact) e = launch_force_t<float, true, true, true>(d, accumulate, st);
         else if (test) e = launch_force_t<float, true, true, false>(d, accumulate, st);

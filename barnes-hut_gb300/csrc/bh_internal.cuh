@@ -41,9 +41,9 @@ constexpr int FORCE_R = 4;                                   // targets per thre
 constexpr int TARGET_CHUNK = FORCE_THREADS * FORCE_R;        // targets per work item
 // FP64 pairs cost 16 FP32 ones or more, so their items are small: a CTA's share of the FP64 pipe
 // turns an item of 512 targets of a dense box into tens of milliseconds (65,536 clustered particles
-// on 32 x 32 boxes, the step: 512 targets 32.9 ms, 64: 8.1, 32: 7.1, 16: 6.6)
+// on 32 x 32 boxes, the step: 512 targets 32.9 ms, 64: 8.1, 32: 7.1, 16: 6.6; other seeds of that
+// input 21 to 32 ms with 512 targets, 4.6 to 5.4 with 16)
 constexpr int TARGET_CHUNK64 = 16;
-constexpr long long SPLIT_FORCE_MIN = 8192;  // particles from which FP64 near pairs run in split floats
 constexpr int FRONTIER_CAP = 512;                            // traversal frontier per level
 constexpr int SCAN_TILE = 4096;   // counts per tile of the single-pass scans (256 threads x 16)
 constexpr int MAX_TG = 8;          // largest target group (boxes per side)
@@ -118,7 +118,6 @@ struct DevPlan {
     SysDyn *dyn;
     Globals *glob;
     Split64 *split;  // the direct-sum sampler's
-    Split64 *fsplit;  // per system, for FP64 forces
     const long long *poff_tab;  // nsys + 1 particle offsets
     const long long *boff_tab;  // nsys + 1 box offsets
     const long long *coff_tab;  // nsys + 1 cell offsets
@@ -435,7 +434,6 @@ cudaError_t launch_lists(const DevPlan &d, cudaStream_t st);
 int list_kernels(long long items_max);  // kernels launch_lists launches for a plan of at most so many items
 cudaError_t launch_fstream(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
                            const cudaEvent_t *ev = nullptr);
-bool force_splits(long long n_total);  // FP64 forces launch two kernels more (launch_force64)
 cudaError_t fstream_init();
 cudaError_t force_init();
 cudaError_t launch_tick(const DevPlan &d, cudaStream_t st, bool keep_acc = false);
