@@ -30,7 +30,7 @@ struct bh_plan {
     long long org_total = 0;  // entries of the box-origin tables (2 G per system)
     // workspace layout (byte offsets)
     size_t ws_bytes = 0;
-    size_t o_sys, o_dyn, o_glob, o_split, o_poff, o_boff, o_coff, o_goff, o_toff, o_lvl;
+    size_t o_sys, o_dyn, o_glob, o_poff, o_boff, o_coff, o_goff, o_toff, o_lvl;
     size_t o_X[2], o_Y[2], o_VX[2], o_VY[2], o_M[2], o_PID[2];
     size_t o_AX, o_AY, o_key, o_slot, o_skey, o_bstart, o_sst, o_leafpart, o_perm, o_bigseg, o_icnt, o_ioff, o_igrp, o_mom, o_rec, o_PD,
         o_rec2, o_org, o_lfar, o_lnear, o_lcnt, o_iord, o_icost, o_ibkt, o_sicnt, o_sioff, o_sigrp, o_sisub, o_sichk, o_qcnt;
@@ -256,7 +256,6 @@ extern "C" int bh_plan_create(bh_plan **out, int nsys, const long long *n, const
     p->o_sys = take(sizeof(SysDesc) * nsys);
     p->o_dyn = take(sizeof(SysDyn) * nsys);
     p->o_glob = take(sizeof(Globals));
-    p->o_split = take(sizeof(Split64));
     p->o_poff = take(sizeof(long long) * (nsys + 1));
     p->o_boff = take(sizeof(long long) * (nsys + 1));
     p->o_coff = take(sizeof(long long) * (nsys + 1));
@@ -346,7 +345,6 @@ static void fill_dev(bh_plan *p) {
     d.sys = (const SysDesc *)(w + p->o_sys);
     d.dyn = (SysDyn *)(w + p->o_dyn);
     d.glob = (Globals *)(w + p->o_glob);
-    d.split = (Split64 *)(w + p->o_split);
     d.poff_tab = (const long long *)(w + p->o_poff);
     d.boff_tab = (const long long *)(w + p->o_boff);
     d.coff_tab = (const long long *)(w + p->o_coff);
@@ -445,13 +443,6 @@ extern "C" int bh_bind(bh_plan *p, void *workspace, size_t bytes, void *stream) 
     CK(p, cudaMemcpyAsync(w + p->o_lvl, p->lvl.data(), 8 * p->lvl.size(), cudaMemcpyHostToDevice, st), "upload lvl");
     CK(p, cudaMemsetAsync(w + p->o_dyn, 0, sizeof(SysDyn) * p->nsys, st), "zero dyn");
     CK(p, cudaMemsetAsync(w + p->o_glob, 0, sizeof(Globals), st), "zero globals");
-    {  // the sampler's extents start empty
-        Split64 s0;
-        memset(&s0, 0, sizeof(s0));
-        s0.ext[0] = s0.ext[1] = ~0ull;
-        CK(p, cudaMemcpyAsync(w + p->o_split, &s0, sizeof(s0), cudaMemcpyHostToDevice, st), "split frame");
-        CK(p, cudaStreamSynchronize(st), "split frame");  // (s0 leaves scope)
-    }
     {  // scan generations start at 1 over zeroed tile states
         const unsigned one[3] = {1u, 1u, 1u};
         CK(p, cudaMemcpyAsync(w + p->o_glob + offsetof(Globals, scan_gen), one, sizeof(one),

@@ -84,16 +84,6 @@ struct SysDyn {
     float key_tol;                // bound on |float quotient - exact quotient| (box edges)
 };
 
-// A system's frame for pairs in split floats (bh_split64.cuh): coordinates (x - cx) * scale lie in
-// [-1, 1], scale a power of two.
-struct Split64 {
-    double cx, cy, scale, inv_scale;
-    float eh, el;                    // softening^2 * scale^2 as two floats
-    int usable;                      // 0: FP64 arithmetic throughout
-    unsigned done;                   // blocks of k_direct_prep finished (the last one resets it)
-    unsigned long long ext[4];       // ordered bits of min x, min y, max x, max y (reset with done)
-};
-
 struct Globals {
     unsigned int epoch;
     unsigned int err;
@@ -117,7 +107,6 @@ struct DevPlan {
     const SysDesc *sys;
     SysDyn *dyn;
     Globals *glob;
-    Split64 *split;  // the direct-sum sampler's
     const long long *poff_tab;  // nsys + 1 particle offsets
     const long long *boff_tab;  // nsys + 1 box offsets
     const long long *coff_tab;  // nsys + 1 cell offsets

@@ -1,6 +1,6 @@
 // bh_misc.cu -- state upload / download, unfused tick, FP64 direct-sum sampler, diagnostics.
 #include "bh_internal.cuh"
-#include "bh_split64.cuh"
+#include "bh_pairs.cuh"
 
 namespace bh {
 
@@ -128,12 +128,6 @@ __global__ void k_inverse_pid(DevPlan d, long long i0, long long n) {
 // Partial sums of chunk c, target k: px, py[c * nt + k] (the state buffer that is not current, free
 // between steps), added in chunk order by k_direct_sum; a single chunk writes the result itself.
 constexpr int DT = 128, DR = 4, DRUN = 16;  // threads, targets per thread, sources per run
-// k_direct_split from 2^19 sources on: relative error of the sums against quadruple precision, over
-// uniform, clustered, generated and far-off systems, softened and not, FP64 kernel / split floats:
-// 65,536 sources 0.8-1.1e-16 / 1.6-3.2e-16, 262,144: 1.0-1.2 / 1.0-1.2, 524,288: 1.1-1.5 / 0.8-1.0,
-// 1,048,576: 1.3-1.9 / 0.7-1.0, 2,000,000: 1.3-2.3 / 0.7-1.1; and from 2^23 pairs on (two passes over
-// the particles first)
-constexpr long long SPLIT_MIN_N = 1 << 19, SPLIT_MIN_PAIRS = 1 << 23;
 
 __global__ void __launch_bounds__(DT) k_direct(DevPlan d, int sys, const long long *targets, long long nt, int T,
                                                int nchunk, double *oax, double *oay) {
@@ -214,168 +208,9 @@ __global__ void __launch_bounds__(DT) k_direct(DevPlan d, int sys, const long lo
     }
 }
 
-// ---- the same on the FP32 pipe (bh_split64.cuh), for long sums
-// Inverse permutation and extents of the system's particles; the last block sets up the frame.
-__global__ void __launch_bounds__(MT) k_direct_prep(DevPlan d, long long i0, long long n) {
-    const int b = (d.glob->epoch + 1) & 1;
-    const double *X = d.X[b], *Y = d.Y[b];
-    unsigned long long e[4] = {~0ull, ~0ull, 0ull, 0ull};
-    for (long long i = (long long)blockIdx.x * MT + threadIdx.x; i < n; i += (long long)gridDim.x * MT) {
-        d.key[d.PID[b][i0 + i]] = (int)(i0 + i);
-        const unsigned long long x = ord_bits(X[i0 + i]), y = ord_bits(Y[i0 + i]);
-        e[0] = x < e[0] ? x : e[0];
-        e[1] = y < e[1] ? y : e[1];
-        e[2] = x > e[2] ? x : e[2];
-        e[3] = y > e[3] ? y : e[3];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, e[q], o);
-            e[q] = q < 2 ? (v < e[q] ? v : e[q]) : (v > e[q] ? v : e[q]);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            if (q < 2) atomicMin(&d.split->ext[q], e[q]);
-            else atomicMax(&d.split->ext[q], e[q]);
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&d.split->done, 1u) == gridDim.x - 1) {
-        __threadfence();
-        Split64 &s = *d.split;
-        double v[4];
-        for (int q = 0; q < 4; q++) {
-            v[q] = unord_bits(__ldcg(&s.ext[q]));
-            s.ext[q] = q < 2 ? ~0ull : 0ull;
-        }
-        s.done = 0u;
-        split_setup(s, v[0], v[2], v[1], v[3], d.eps2);
-    }
-}
-
-// The particles as split floats, into the state buffer that is not current: (a, b) of x and of y, both
-// c, the mass.
-__global__ void __launch_bounds__(MT) k_direct_convert(DevPlan d, long long i0, long long n) {
-    const int b = (d.glob->epoch + 1) & 1;
-    const double cx = d.split->cx, cy = d.split->cy, scale = d.split->scale;
-    float2 *AX = reinterpret_cast<float2 *>(d.X[b ^ 1]), *AY = reinterpret_cast<float2 *>(d.Y[b ^ 1]);
-    float2 *C = reinterpret_cast<float2 *>(d.VX[b ^ 1]), *MM = reinterpret_cast<float2 *>(d.M[b ^ 1]);
-    for (long long i = i0 + (long long)blockIdx.x * MT + threadIdx.x; i < i0 + n; i += (long long)gridDim.x * MT) {
-        float xa, xb, xc, ya, yb, yc, mh, ml;
-        split3((d.X[b][i] - cx) * scale, xa, xb, xc);
-        split3((d.Y[b][i] - cy) * scale, ya, yb, yc);
-        if (!split_mass(d.M[b][i], mh, ml)) d.split->usable = 0;
-        AX[i] = make_float2(xa, xb);
-        AY[i] = make_float2(ya, yb);
-        C[i] = make_float2(xc, yc);
-        MM[i] = make_float2(mh, ml);
-    }
-}
-
-// As k_direct, with DT sources staged at a time; partial sums interleaved in VY of the other buffer.
-// 1,000 targets of 1,048,576: 21.9 ms in FP64 -> 3.3 ms, 100 targets 0.9 ms.
-template <bool EPS>
-__global__ void __launch_bounds__(DT, 4) k_direct_split(DevPlan d, int sys, const long long *targets, long long nt,
-                                                        int T, int nchunk, double *oax, double *oay) {
-    __shared__ __align__(16) Src64 src[DT];
-    __shared__ double red[2 * DT * DR];
-    const int b = (d.glob->epoch + 1) & 1;
-    const SysDesc &sd = d.sys[sys];
-    const Split64 &fr = *d.split;
-    const bool usable = fr.usable != 0;
-    const double *X = d.X[b], *Y = d.Y[b], *M = d.M[b];
-    const float2 *AX = reinterpret_cast<const float2 *>(d.X[b ^ 1]), *AY = reinterpret_cast<const float2 *>(d.Y[b ^ 1]);
-    const float2 *C = reinterpret_cast<const float2 *>(d.VX[b ^ 1]), *MM = reinterpret_cast<const float2 *>(d.M[b ^ 1]);
-    const int nthr = T / DR, nslice = DT / nthr, slice = threadIdx.x / nthr, tl = threadIdx.x - slice * nthr;
-    const long long tile = blockIdx.x / nchunk;
-    const int chunk = blockIdx.x - (int)(tile * nchunk);
-    const long long k0 = tile * T + (long long)tl * DR;
-    int ti[DR];
-    double sx[DR], sy[DR];
-    Tgt64 tg[DR / 2];
-    Sum64 sum[DR / 2];
-#pragma unroll
-    for (int r = 0; r < DR; r++) {
-        const long long t = k0 + r < nt ? targets[k0 + r] : -1;
-        ti[r] = t >= sd.poff && t < sd.poff + sd.n ? d.key[t] : -1;  // a particle of this system
-        sx[r] = sy[r] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < DR / 2; k++) {
-        const int i0 = ti[2 * k] < 0 ? (int)sd.poff : ti[2 * k], i1 = ti[2 * k + 1] < 0 ? (int)sd.poff : ti[2 * k + 1];
-        const float2 x0 = AX[i0], x1 = AX[i1], y0 = AY[i0], y1 = AY[i1], c0 = C[i0], c1 = C[i1];
-        tg[k].ax = f2_pack(x0.x, x1.x);
-        tg[k].bx = f2_pack(x0.y, x1.y);
-        tg[k].cx = f2_pack(c0.x, c1.x);
-        tg[k].ay = f2_pack(y0.x, y1.x);
-        tg[k].by = f2_pack(y0.y, y1.y);
-        tg[k].cy = f2_pack(c0.y, c1.y);
-        sum64_zero(sum[k]);
-    }
-    const f2_t eh = f2_dup(fr.eh), el = f2_dup(fr.el);
-    // one pair in FP64 (close ones, and every one of a system that does not fit the floats), into the
-    // sums' scaled units
-    auto pair_fp64 = [&](int r, long long j) {
-        if (ti[r] < 0 || j == ti[r]) return;
-        const double dx = X[j] - X[ti[r]], dy = Y[j] - Y[ti[r]];
-        const double w = M[j] * rcp64(dx * dx + (dy * dy + d.eps2)) * fr.inv_scale;
-        sx[r] += w * dx;
-        sy[r] += w * dy;
-    };
-    const long long j0 = sd.poff + (sd.n * chunk) / nchunk, j1 = sd.poff + (sd.n * (chunk + 1)) / nchunk;
-    for (long long p = j0; p < j1; p += DT) {
-        const int ns = (int)(j1 - p < DT ? j1 - p : DT);
-        __syncthreads();  // the previous stage has been swept
-        if (threadIdx.x < ns) {
-            const long long j = p + threadIdx.x;
-            const float2 ax = AX[j], ay = AY[j], c = C[j], m = MM[j];
-            src64_make(src[threadIdx.x], make_float4(ax.x, ax.y, c.x, m.x), make_float4(ay.x, ay.y, c.y, m.y));
-        }
-        __syncthreads();
-        if (usable) {
-            for (int q0 = slice; q0 < ns; q0 += SPLIT_RUN * nslice) {
-#pragma unroll 1
-                for (int u = 0; u < SPLIT_RUN; u++) {
-                    const int q = q0 + u * nslice;
-                    if (q >= ns) break;
-                    const Src64 s = src[q];
-#pragma unroll
-                    for (int k = 0; k < DR / 2; k++)
-                        pair64<EPS>(s, tg[k], eh, el, SPLIT_LIM, sum[k],
-                                    [&](int half, float) { pair_fp64(2 * k + half, p + q); });
-                }
-#pragma unroll
-                for (int k = 0; k < DR / 2; k++)
-                    sum64_flush(sum[k], sx[2 * k], sx[2 * k + 1], sy[2 * k], sy[2 * k + 1]);
-            }
-        } else {
-            for (int q = slice; q < ns; q += nslice)
-                for (int r = 0; r < DR; r++) pair_fp64(r, p + q);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < DR; r++) {
-        red[2 * (threadIdx.x * DR + r)] = sx[r];
-        red[2 * (threadIdx.x * DR + r) + 1] = sy[r];
-    }
-    __syncthreads();
-    double2 *part = reinterpret_cast<double2 *>(d.VY[b ^ 1]);
-    for (int v = threadIdx.x; v < T && tile * T + v < nt; v += DT) {
-        double ax = 0.0, ay = 0.0;
-        for (int s = 0; s < nslice; s++) {
-            ax += red[2 * (s * T + v)];
-            ay += red[2 * (s * T + v) + 1];
-        }
-        part[chunk * nt + tile * T + v] = make_double2(ax * fr.scale, ay * fr.scale);
-    }
-}
-
 // a warp per target: the chunks' partial sums, lane-strided, then a fixed tree
-// (pairs: the partial sums as pairs in VY, else x in VX and y in VY)
 __global__ void __launch_bounds__(MT) k_direct_sum(DevPlan d, int sys, const long long *targets, long long nt, int nchunk,
-                                                   int pairs, double *oax, double *oay) {
+                                                   double *oax, double *oay) {
     const int b = (d.glob->epoch + 1) & 1, lane = threadIdx.x & 31;
     const SysDesc &sd = d.sys[sys];
     const long long k = ((long long)blockIdx.x * MT + threadIdx.x) >> 5;
@@ -383,14 +218,8 @@ __global__ void __launch_bounds__(MT) k_direct_sum(DevPlan d, int sys, const lon
     const double *px = d.VX[b ^ 1], *py = d.VY[b ^ 1];
     double ax = 0.0, ay = 0.0;
     for (int c = lane; c < nchunk; c += 32) {
-        if (pairs) {
-            const double2 v = reinterpret_cast<const double2 *>(py)[c * nt + k];
-            ax += v.x;
-            ay += v.y;
-        } else {
-            ax += px[c * nt + k];
-            ay += py[c * nt + k];
-        }
+        ax += px[c * nt + k];
+        ay += py[c * nt + k];
     }
     for (int o = 16; o; o >>= 1) {
         ax += __shfl_xor_sync(0xffffffffu, ax, o);
@@ -493,16 +322,8 @@ cudaError_t launch_tick(const DevPlan &d, cudaStream_t st, bool keep_acc) {
 cudaError_t launch_direct(const DevPlan &d, int sys, long long poff, long long n, const long long *targets,
                           long long nt, double *ax, double *ay, cudaStream_t st) {
     if (d.n_total == 0 || nt == 0) return cudaSuccess;
-    // split floats: long sums (their accuracy rests on averaging), enough of them to pay for two
-    // passes over the particles, and room for the partial sums
-    const bool split = n >= SPLIT_MIN_N && nt * n >= SPLIT_MIN_PAIRS && 2 * nt <= d.n_total;
-    const long long cap = split ? d.n_total / (2 * nt) : d.n_total / nt;  // chunks the scratch holds
-    if (split) {
-        k_direct_prep<<<grid_of(n, MT * 4, d.nsm), MT, 0, st>>>(d, poff, n);
-        k_direct_convert<<<grid_of(n, MT, d.nsm), MT, 0, st>>>(d, poff, n);
-    } else if (n > 0) {
-        k_inverse_pid<<<grid_of(n, MT, d.nsm), MT, 0, st>>>(d, poff, n);
-    }
+    const long long cap = d.n_total / nt;  // chunks the scratch holds
+    if (n > 0) k_inverse_pid<<<grid_of(n, MT, d.nsm), MT, 0, st>>>(d, poff, n);
     // The largest tile that leaves at most 1/16 of its targets idle (else the one that leaves least),
     // while tiles x chunks fill the chip: the scratch holds n_total / nt chunks, so many targets of
     // few sources need small tiles.  A small tile costs nothing but its slices' longer reduction.
@@ -527,16 +348,9 @@ cudaError_t launch_direct(const DevPlan &d, int sys, long long poff, long long n
         nchunk = nchunk < most ? nchunk : most;
         nchunk = nchunk < cap ? nchunk : cap;
         if (nchunk < 1) nchunk = 1;
-        if (split) {
-            auto k = d.eps2 > 0.0 ? k_direct_split<true> : k_direct_split<false>;
-            k<<<(unsigned)(tiles * nchunk), DT, 0, st>>>(d, sys, targets + t0, c, T, (int)nchunk, ax + t0, ay + t0);
-            k_direct_sum<<<(unsigned)((c + MT / 32 - 1) / (MT / 32)), MT, 0, st>>>(d, sys, targets + t0, c, (int)nchunk, 1,
-                                                                                 ax + t0, ay + t0);
-            continue;
-        }
         k_direct<<<(unsigned)(tiles * nchunk), DT, 0, st>>>(d, sys, targets + t0, c, T, (int)nchunk, ax + t0, ay + t0);
         if (nchunk > 1)
-            k_direct_sum<<<(unsigned)((c + MT / 32 - 1) / (MT / 32)), MT, 0, st>>>(d, sys, targets + t0, c, (int)nchunk, 0,
+            k_direct_sum<<<(unsigned)((c + MT / 32 - 1) / (MT / 32)), MT, 0, st>>>(d, sys, targets + t0, c, (int)nchunk,
                                                                                  ax + t0, ay + t0);
     }
     return cudaGetLastError();

@@ -66,3 +66,41 @@ def test_fp64_forces_of_small_systems(n, systems, theta, eps, heavy):
         ref, size = direct_sums(xy[s, 0], xy[s, 1], m[s], eps, range(n))
         err = np.sqrt((((got[:, s] - ref) / size) ** 2).sum(0))
         assert float(err.max()) <= bound, float(err.max()) / EPS
+
+
+# The sampler over half a million sources and more of which eight have mass, or one has 1e9 times the
+# others': its result is an FP64 sum also where no errors average out.  A pair has 8.1 roundings of at most
+# 2^-53 (two differences, two of r^2's own and their two in it, reciprocal, weight and product).  Eight
+# terms: seven additions more, at most.  A heavy one: every addition after it rounds the whole sum; at most
+# 96 of them in a row (runs of 16, a thread's runs, slices, chunks), whose errors, 2^-53 at most and
+# independent, add up as a random walk.
+@pytest.mark.parametrize("nt", [16, 37])
+@pytest.mark.parametrize("eps", [0.0, 1e-3])
+@pytest.mark.parametrize("heavy", [False, True])
+def test_direct_sample_of_few_masses(nt, eps, heavy):
+    from barneshut.gb300 import native
+
+    n = (1 << 19) + 77
+    rng = np.random.default_rng(nt)
+    x, y = rng.random((2, n))
+    if heavy:
+        m = rng.uniform(0.5, 1.0, n)
+        m[n // 3] = 1e9
+    else:
+        m = np.zeros(n)
+        m[rng.choice(n, 8, replace=False)] = rng.uniform(0.5, 1.0, 8)
+    z = np.zeros(n)
+    plan = native.Plan([n], [64], native.make_params(1.0, 1e-5, eps, 0.0, 0.5))
+    plan.load(x, y, m, z, z)
+    t = rng.choice(n, nt, replace=False)
+    ax, ay = plan.direct_sample(t)
+    got = np.stack([ax.cpu().numpy(), ay.cpu().numpy()])
+    if heavy:  # (half a million terms a target in extended precision)
+        t, got = t[:8], got[:, :8]
+    used = np.unique(np.r_[np.flatnonzero(m), t])
+    ref, size = direct_sums(x[used], y[used], m[used], eps, np.searchsorted(used, t))
+    err = np.sqrt((((got - ref) / size) ** 2).sum(0))
+    if heavy:
+        assert float(np.sqrt(np.mean(err ** 2))) <= np.sqrt(8.1 + 96) * EPS
+    else:
+        assert float(err.max()) <= (8.1 + 7) * EPS
