@@ -393,6 +393,22 @@ inline cudaError_t launch_step(void (*k)(P...), unsigned grid, unsigned block, s
     return cudaLaunchKernelEx(&c, k, a...);
 }
 
+// Barrier over the CTAs of a cluster; shared-memory writes before it are visible to all of them after it.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    cluster_arrive();
+    cluster_wait();
+}
+// a 64-bit value in another CTA's shared memory
+__device__ __forceinline__ unsigned long long ld_cluster(const unsigned long long *p, unsigned rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    unsigned long long v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(r) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void raise_err(Globals *g, unsigned f) {
     if ((atomicOr(&g->err, 0u) & f) == 0) atomicOr(&g->err, f);
 }

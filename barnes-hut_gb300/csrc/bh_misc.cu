@@ -119,25 +119,27 @@ __global__ void k_inverse_pid(DevPlan d, long long i0, long long n) {
 }
 
 // FP64 direct sum (base.py:16-32; the target itself is skipped by index).  A CTA serves a tile of T
-// targets (T a power of two, 4 .. 64) over one chunk of the sources: T / 4 threads per slice of the
-// chunk, four targets each, so a source is loaded once per four pairs.  Bound: the FP64 pipe (2
-// operations per clock and SM on GB300; 10 per pair, with rcp64 in place of the division's 8), so
-// the split over chunks only has to fill it: few targets over many sources run on the whole chip
-// (before: one CTA per target, 16.5 operations per pair).  1,500 targets of 400,000: 16.2 ->
-// 13.4 ms; 100 of 200,000: 938 -> 536 us; 10 of 100,000: 494 -> 93 us.
-// Partial sums of chunk c, target k: px, py[c * nt + k] (the state buffer that is not current, free
-// between steps), added in chunk order by k_direct_sum; a single chunk writes the result itself.
-constexpr int DT = 128, DR = 4, DRUN = 16;  // threads, targets per thread, sources per run
+// targets (a power of two) over one chunk of the sources: T / DR threads per slice of the chunk, DR
+// targets each, so a source is loaded once per DR pairs; the chunks of a tile are the CTAs of one
+// cluster, whose sums meet in its first CTA, in chunk order.  Nothing is left in the workspace but
+// the inverse permutation, the same from every call: samplers on several streams may overlap, with
+// each other and with an evaluation.  Bound: the FP64 pipe (2 operations per clock and SM on GB300;
+// 10 per pair, with rcp64 in place of the division's 8), so the split only has to fill it.  One CTA
+// per target and the division, then this: 1,000 targets of 1,048,576 29.6 -> 23.4 ms, 100 of them 4.7
+// -> 2.2, 10 of them 4.7 -> 0.62; 1,500 of 400,000 16.2 -> 13.4; 10 of 100,000 0.50 -> 0.10.
+constexpr int DT = 128, DRUN = 16;  // threads, sources per run
+constexpr int DCL = 8;              // most chunks of a tile (the portable cluster size)
 
+template <int DR>
 __global__ void __launch_bounds__(DT) k_direct(DevPlan d, int sys, const long long *targets, long long nt, int T,
                                                int nchunk, double *oax, double *oay) {
     const int b = (d.glob->epoch + 1) & 1;
     const SysDesc &sd = d.sys[sys];
     const double *X = d.X[b], *Y = d.Y[b], *M = d.M[b];
-    __shared__ double red[2 * DT * DR];
+    __shared__ double red[2 * DT * DR], part[DT], sum[DT];  // (T <= DT / 2)
     const int nthr = T / DR, nslice = DT / nthr, slice = threadIdx.x / nthr, tl = threadIdx.x - slice * nthr;
     const long long tile = blockIdx.x / nchunk;
-    const int chunk = blockIdx.x - (int)(tile * nchunk);
+    const int chunk = blockIdx.x - (int)(tile * nchunk);  // (its rank in the cluster)
     const long long k0 = tile * T + (long long)tl * DR;
     long long ti[DR];
     double xt[DR], yt[DR], sx[DR], sy[DR];
@@ -183,49 +185,39 @@ __global__ void __launch_bounds__(DT) k_direct(DevPlan d, int sys, const long lo
         red[2 * (threadIdx.x * DR + r) + 1] = sy[r];
     }
     __syncthreads();
-    double *px = d.VX[b ^ 1], *py = d.VY[b ^ 1];
-    for (int v = threadIdx.x; v < T && tile * T + v < nt; v += DT) {
-        double ax = 0.0, ay = 0.0;
-        for (int s0 = 0; s0 < nslice; s0 += DRUN) {
-            double rx = 0.0, ry = 0.0;
-            for (int s = s0; s < s0 + DRUN && s < nslice; s++) {
-                rx += red[2 * (s * T + v)];
-                ry += red[2 * (s * T + v) + 1];
-            }
-            ax += rx;
-            ay += ry;
+    // the slices' sums, again in runs of DRUN, then the runs'; T x runs <= DT / 2 for every T
+    for (int e = threadIdx.x; e < T * ((nslice + DRUN - 1) / DRUN); e += DT) {
+        const int v = e % T, s0 = e / T * DRUN;
+        double rx = 0.0, ry = 0.0;
+        for (int s = s0; s < s0 + DRUN && s < nslice; s++) {
+            rx += red[2 * (s * T + v)];
+            ry += red[2 * (s * T + v) + 1];
         }
-        const long long k = tile * T + v;
-        if (nchunk > 1) {
-            px[chunk * nt + k] = ax;
-            py[chunk * nt + k] = ay;
-        } else {
-            const bool in = targets[k] >= sd.poff && targets[k] < sd.poff + sd.n;
-            const double nan = __longlong_as_double(0x7ff8000000000000ll);
-            oax[k] = in ? d.gconst * ax : nan;
-            oay[k] = in ? d.gconst * ay : nan;
-        }
+        part[2 * e] = rx;
+        part[2 * e + 1] = ry;
     }
-}
-
-// a warp per target: the chunks' partial sums, lane-strided, then a fixed tree
-__global__ void __launch_bounds__(MT) k_direct_sum(DevPlan d, int sys, const long long *targets, long long nt, int nchunk,
-                                                   double *oax, double *oay) {
-    const int b = (d.glob->epoch + 1) & 1, lane = threadIdx.x & 31;
-    const SysDesc &sd = d.sys[sys];
-    const long long k = ((long long)blockIdx.x * MT + threadIdx.x) >> 5;
-    if (k >= nt) return;
-    const double *px = d.VX[b ^ 1], *py = d.VY[b ^ 1];
+    __syncthreads();
+    const int v = threadIdx.x;
     double ax = 0.0, ay = 0.0;
-    for (int c = lane; c < nchunk; c += 32) {
-        ax += px[c * nt + k];
-        ay += py[c * nt + k];
+    if (v < T) {
+        for (int s0 = 0; s0 < nslice; s0 += DRUN) {
+            ax += part[2 * (s0 / DRUN * T + v)];
+            ay += part[2 * (s0 / DRUN * T + v) + 1];
+        }
+        sum[2 * v] = ax;
+        sum[2 * v + 1] = ay;
     }
-    for (int o = 16; o; o >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, o);
-        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+    if (nchunk > 1) {
+        cluster_sync();
+        if (chunk == 0 && v < T)
+            for (int c = 1; c < nchunk; c++) {
+                ax += __longlong_as_double(ld_cluster(reinterpret_cast<unsigned long long *>(sum) + 2 * v, c));
+                ay += __longlong_as_double(ld_cluster(reinterpret_cast<unsigned long long *>(sum) + 2 * v + 1, c));
+            }
+        cluster_sync();  // (the sums have been read)
     }
-    if (lane == 0) {
+    const long long k = tile * T + v;
+    if (chunk == 0 && v < T && k < nt) {
         const bool in = targets[k] >= sd.poff && targets[k] < sd.poff + sd.n;
         const double nan = __longlong_as_double(0x7ff8000000000000ll);
         oax[k] = in ? d.gconst * ax : nan;
@@ -322,36 +314,33 @@ cudaError_t launch_tick(const DevPlan &d, cudaStream_t st, bool keep_acc) {
 cudaError_t launch_direct(const DevPlan &d, int sys, long long poff, long long n, const long long *targets,
                           long long nt, double *ax, double *ay, cudaStream_t st) {
     if (d.n_total == 0 || nt == 0) return cudaSuccess;
-    const long long cap = d.n_total / nt;  // chunks the scratch holds
     if (n > 0) k_inverse_pid<<<grid_of(n, MT, d.nsm), MT, 0, st>>>(d, poff, n);
-    // The largest tile that leaves at most 1/16 of its targets idle (else the one that leaves least),
-    // while tiles x chunks fill the chip: the scratch holds n_total / nt chunks, so many targets of
-    // few sources need small tiles.  A small tile costs nothing but its slices' longer reduction.
-    const long long fill = (long long)d.nsm * 4;
-    int T = 64;
-    long long least = 0;
-    for (int c = 64; c >= DR; c >>= 1) {
-        const long long pad = (nt + c - 1) / c * c, room = cap > 1 ? cap : 1;
-        if (c == 64 || pad < least || (nt + T - 1) / T * room < fill) {
-            least = pad;
-            T = c;
-        }
-        if (16 * pad <= 17 * nt && (nt + T - 1) / T * room >= fill) break;
-    }
-    for (long long t0 = 0; t0 < nt; t0 += (1LL << 28)) {
-        const long long c = nt - t0 < (1LL << 28) ? nt - t0 : (1LL << 28), tiles = (c + T - 1) / T;
-        // chunks: 16 CTAs per SM (an SM with one more than another is then a sixteenth behind: 1,500
-        // targets of 400,000 15.5 -> 13.4 ms against four), at least two sources for every slice, within
-        // the scratch
-        long long nchunk = (4 * fill + tiles - 1) / tiles;
-        const long long most = n / (2LL * (DT * DR / T));
-        nchunk = nchunk < most ? nchunk : most;
-        nchunk = nchunk < cap ? nchunk : cap;
-        if (nchunk < 1) nchunk = 1;
-        k_direct<<<(unsigned)(tiles * nchunk), DT, 0, st>>>(d, sys, targets + t0, c, T, (int)nchunk, ax + t0, ay + t0);
-        if (nchunk > 1)
-            k_direct_sum<<<(unsigned)((c + MT / 32 - 1) / (MT / 32)), MT, 0, st>>>(d, sys, targets + t0, c, (int)nchunk,
-                                                                                 ax + t0, ay + t0);
+    // Four targets a thread where their tiles, in DCL chunks each, give every SM four CTAs, in the largest
+    // tile that leaves at most 1/16 of its targets idle and the chip filled; else one target a thread.
+    // Chunks: a power of two of them, 16 CTAs per SM (an SM with one more than another is then a
+    // sixteenth behind), two sources or more for every slice.
+    const long long fill = (long long)d.nsm * 16;
+    const bool four = (nt + 3) / 4 * DCL >= (long long)d.nsm * 4;
+    int T = four ? 64 : 1;
+    while (T > 4 && (16 * ((nt + T - 1) / T * T) > 17 * nt || (nt + T - 1) / T * DCL < fill)) T >>= 1;
+    for (long long t0 = 0; t0 < nt; t0 += (1LL << 26)) {
+        const long long c = nt - t0 < (1LL << 26) ? nt - t0 : (1LL << 26), tiles = (c + T - 1) / T;
+        const long long most = n / (2LL * (DT * (four ? 4 : 1) / T));
+        int nchunk = 1;
+        while (nchunk < DCL && tiles * nchunk < fill && 2 * nchunk <= most) nchunk *= 2;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = nchunk;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cf = {};
+        cf.gridDim = dim3((unsigned)(tiles * nchunk));
+        cf.blockDim = dim3(DT);
+        cf.stream = st;
+        cf.attrs = &at;
+        cf.numAttrs = 1;
+        cudaError_t e = cudaLaunchKernelEx(&cf, four ? k_direct<4> : k_direct<1>, d, sys, targets + t0, c, T, nchunk, ax + t0,
+                                           ay + t0);
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }

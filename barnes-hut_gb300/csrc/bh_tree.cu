@@ -1433,21 +1433,6 @@ struct ClusterSmem {
 };
 static_assert(4 * CL_MAX_BOXES <= 2048 * 8 && CL_MAX_SIDE * CL_MAX_SIDE == CL_MAX_BOXES, "eight CTAs or more: 2,048 quadrants each at most");
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync() {
-    cluster_arrive();
-    cluster_wait();
-}
-// a 64-bit value in another CTA's shared memory
-__device__ __forceinline__ unsigned long long ld_cluster(const unsigned long long *p, unsigned rank) {
-    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
-    unsigned long long v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(r) : "memory");
-    return v;
-}
-
 // Work items of the groups [g0, g1) by one CTA, from item `base` on; returns their number.  WRITE:
 // write them (the number alone needs no base).
 // Walking plan: k_group_items, its scan and k_fill_items.

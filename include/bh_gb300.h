@@ -233,7 +233,9 @@ int bh_force_kernel_ms(bh_plan *plan, float *ms);
 /* FP64 direct sum on the device for nt targets (indices into the
  * concatenated pid order, device array) of system `sys`, no cutoff, the
  * plan's softening: a_t = G sum_{j != t} m_j (x_j - x_t) / (r^2 + eps^2).
- * Outputs ax, ay (device, nt doubles).  Replaces nsquared_acc_check
+ * Outputs ax, ay (device, nt doubles).  Keeps no scratch in the plan: calls on
+ * several streams may overlap, with one another and with bh_evaluate.
+ * Replaces nsquared_acc_check
  * (base.py:16-32) of the --check accuracy sampler (base.py:149-205). */
 int bh_direct_sample(bh_plan *plan, int sys, const long long *targets, long long nt,
                      double *ax, double *ay, void *stream);

@@ -104,3 +104,64 @@ def test_direct_sample_of_few_masses(nt, eps, heavy):
         assert float(np.sqrt(np.mean(err ** 2))) <= np.sqrt(8.1 + 96) * EPS
     else:
         assert float(err.max()) <= (8.1 + 7) * EPS
+
+
+# Samplers on several streams of one plan, of the same system and of two, beside each other and beside an
+# FP64 evaluation: each gives what it gives alone, bit for bit, and so does the evaluation.
+def test_overlapping_samplers_and_evaluation():
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(3)
+    sizes = [60000, 90000]
+    n = sum(sizes)
+    x, y, m = rng.random(n), rng.random(n), rng.uniform(0.5, 1.0, n)
+    z = np.zeros(n)
+    plan = native.Plan(sizes, [64, 64], native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.6, 2, native.BH_PREC_FP64))
+    plan.load(x, y, m, z, z)
+    plan.create_tree()
+    plan.summarize()
+    calls = [(rng.choice(sizes[s], k, replace=False) + s * sizes[0], s) for s, k in ((0, 9), (1, 300), (1, 50), (0, 1200))]
+    alone = [torch.stack(plan.direct_sample(t, sys=s)) for t, s in calls]
+    plan.evaluate()
+    want = [plan.store()[k] for k in ("ax", "ay")]
+    streams = [torch.cuda.Stream() for _ in calls]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        plan.create_tree()
+        plan.summarize()
+        got = []
+        for st in streams:
+            st.wait_stream(torch.cuda.current_stream())
+        plan.evaluate()
+        for st, (t, s) in zip(streams, calls):
+            with torch.cuda.stream(st):
+                got.append(torch.stack(plan.direct_sample(t, sys=s)))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(alone, got))
+        out = plan.store()
+        assert torch.equal(out["ax"], want[0]) and torch.equal(out["ay"], want[1])
+    assert plan.error_flags() == 0
+
+
+# Target and source counts at the edges of the sampler's tiles, chunks and thread layouts: one target a
+# thread and four, tiles of 4 to 64 with idle targets, one chunk to eight, against extended precision.
+# 32 + 16 + 8 + 8 additions of a sum's roundings beside a pair's 8.1, of the terms' magnitudes.
+@pytest.mark.parametrize("n,nt", [(2, 1), (255, 7), (257, 75), (511, 76), (2049, 303), (2048, 304), (4097, 305), (3001, 2433),
+                                  (1500, 1216), (70001, 5), (300, 1000)])
+def test_direct_sample_layouts(n, nt):
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(n + nt)
+    x, y, m = rng.random(n), rng.random(n), rng.uniform(0.5, 1.0, n)
+    z = np.zeros(n)
+    plan = native.Plan([n], [2], native.make_params(1.0, 1e-5, 1e-3, 0.0, 0.5))
+    plan.load(x, y, m, z, z)
+    t = np.resize(rng.permutation(n), nt)  # (targets may repeat)
+    ax, ay = plan.direct_sample(t)
+    got = np.stack([ax.cpu().numpy(), ay.cpu().numpy()])
+    some = np.unique(np.r_[np.arange(min(nt, 12)), rng.choice(nt, min(nt, 12), replace=False), nt - 1])
+    ref, size = direct_sums(x, y, m, 1e-3, t[some])
+    err = np.sqrt((((got[:, some] - ref) / size) ** 2).sum(0))
+    assert float(err.max()) <= (8.1 + 64) * EPS
+    for i in set(t.tolist()) if nt > n else ():
+        assert len(np.unique(got[0, t == i])) == 1
