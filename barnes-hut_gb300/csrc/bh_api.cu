@@ -32,10 +32,10 @@ struct bh_plan {
     size_t ws_bytes = 0;
     size_t o_sys, o_dyn, o_glob, o_poff, o_boff, o_coff, o_goff, o_toff, o_lvl;
     size_t o_X[2], o_Y[2], o_VX[2], o_VY[2], o_M[2], o_PID[2];
-    size_t o_AX, o_AY, o_key, o_slot, o_skey, o_bstart, o_sst, o_leafpart, o_perm, o_bigseg, o_icnt, o_ioff, o_igrp, o_mom, o_rec, o_PD,
+    size_t o_AX, o_AY, o_key, o_slot, o_skey, o_bstart, o_sst, o_leafpart, o_perm, o_bigseg, o_icnt, o_ioff, o_igrp, o_picnt, o_pioff, o_pigrp, o_mom, o_rec, o_PD,
         o_rec2, o_org, o_lfar, o_lnear, o_lcnt, o_iord, o_icost, o_ibkt, o_sicnt, o_sioff, o_sigrp, o_sisub, o_sichk, o_qcnt;
     bool stream = false;  // theta-mode interaction lists built once per group and streamed
-    int chunk = TARGET_CHUNK;
+    int chunk = TARGET_CHUNK, pchunk = TARGET_CHUNK;
     int dense_min = BH_STREAM_DENSE_MIN;
     int quad_min = BH_STREAM_QUAD_MIN;
     void *ws = nullptr;
@@ -206,7 +206,8 @@ extern "C" int bh_plan_create(bh_plan **out, int nsys, const long long *n, const
     for (int s = 0; s < nsys; s++) maxG = std::max(maxG, p->sys[s].G);
     p->stream = !flat && pr.precision != BH_PREC_FP64 && pr.cutoff_r2 == 0.0 && pr.softening > 0.0 &&
                 !(pr.flags & BH_FLAG_WALK) && maxG <= LIST_MAX_G;
-    p->chunk = p->stream ? STREAM_CHUNK : pr.precision == BH_PREC_FP64 ? TARGET_CHUNK64 : TARGET_CHUNK;
+    p->pchunk = p->stream ? STREAM_CHUNK : TARGET_CHUNK;
+    p->chunk = pr.precision == BH_PREC_FP64 ? TARGET_CHUNK64 : p->pchunk;
     if (pr.dense_min < 0) return bad("dense_min < 0");
     p->dense_min = pr.dense_min > 0 ? pr.dense_min : BH_STREAM_DENSE_MIN;
     p->quad_min = pr.quad_min > 0 ? pr.quad_min : (pr.quad_min == 0 ? BH_STREAM_QUAD_MIN : 0);
@@ -285,6 +286,14 @@ extern "C" int bh_plan_create(bh_plan **out, int nsys, const long long *n, const
     p->o_icnt = take(4 * (size_t)p->NG_total);
     p->o_ioff = take(4 * ((size_t)p->NG_total + 1));
     p->o_igrp = take(4 * ((size_t)p->NG_total + N / p->chunk + 1));
+    p->o_picnt = p->o_icnt;
+    p->o_pioff = p->o_ioff;
+    p->o_pigrp = p->o_igrp;
+    if (p->pchunk != p->chunk) {
+        p->o_picnt = take(4 * (size_t)p->NG_total);
+        p->o_pioff = take(4 * ((size_t)p->NG_total + 1));
+        p->o_pigrp = take(4 * ((size_t)p->NG_total + N / p->pchunk + 1));
+    }
     p->o_lfar = take(16 * (size_t)lf_total);
     p->o_lnear = take(16 * (size_t)ln_total);
     p->o_lcnt = take(p->stream ? 8 * (size_t)p->NG_total : 0);
@@ -378,6 +387,9 @@ static void fill_dev(bh_plan *p) {
     d.item_cnt = (int *)(w + p->o_icnt);
     d.item_off = (int *)(w + p->o_ioff);
     d.item_group = (int *)(w + p->o_igrp);
+    d.pitem_cnt = (int *)(w + p->o_picnt);
+    d.pitem_off = (int *)(w + p->o_pioff);
+    d.pitem_group = (int *)(w + p->o_pigrp);
     d.mom = (double *)(w + p->o_mom);
     d.leafpart = (float *)(w + p->o_leafpart);
     d.upcnt = (unsigned *)(w + p->o_upcnt);
@@ -401,6 +413,7 @@ static void fill_dev(bh_plan *p) {
     d.cl_ctas = p->cl_ctas;
     d.stream = p->stream ? 1 : 0;
     d.chunk = p->chunk;
+    d.pchunk = p->pchunk;
     const bh_params &pr = p->params;
     d.gconst = pr.grav_constant;
     d.dt = pr.tick_seconds;
@@ -688,11 +701,12 @@ extern "C" int bh_kernels_per_step(const bh_plan *p, int *count) {
     // place, the scatter's four kernels (permutation, quadrant sort, long quadrants, gather with
     // the leaf sums), force (and before it, when streaming, the list build and the two kernels of
     // the heaviest-first item order); work items: count, scan, fill for the walk or the learned
-    // correction, one kernel for list streaming
-    const bool walk_items = !p->stream || (p->params.flags & BH_FLAG_LEARNED);
+    // correction (and again where the pair generator's items differ), one kernel for list streaming
+    const bool learned = p->params.flags & BH_FLAG_LEARNED;
+    const int walk_items = !p->stream || learned ? (learned && p->pchunk != p->chunk ? 6 : 3) : 0;
     // (a walking plan's tick is a kernel of its own: the walk reads the state the tick writes)
     // A small system's tree, work items and summarize are one kernel (cluster_tree).
-    const int tree = cluster_tree(p) ? 1 : 1 + 1 + (walk_items ? 3 : 0) + 1 + (p->n_total > 0 ? 6 : 0) + (p->stream ? 1 : 0);
+    const int tree = cluster_tree(p) ? 1 : 1 + 1 + walk_items + 1 + (p->n_total > 0 ? 6 : 0) + (p->stream ? 1 : 0);
     const long long items_max = p->NG_total + p->n_total / p->dense_min +
                                 (p->quad_min > 0 ? 4 * (p->n_total / p->quad_min) : 0) + p->n_total / STREAM_ITEM_DIV + 1;
     *count = tree + (p->n_total > 0 ? 1 : 0) + (p->stream && p->n_total > 0 ? list_kernels(items_max) : 0) + (!p->stream && p->n_total > 0 ? 1 : 0);
@@ -909,10 +923,11 @@ extern "C" int bh_learned_pairs(bh_plan *p, double theta_hi, double theta_lo, in
         tpi < 1 || capacity < 0 || !feats || !targets || !counter)
         return fail(p, BH_ERR_INVALID, "bad learned_pairs arguments");
     // a plan without the learned correction builds neither the pyramid's second moments nor
-    // (when streaming) the walk items in its step: rebuild the pyramid above the summed leaves
-    // with them (the same centres of mass and masses)
+    // (when streaming, or with FP64 pairs) the generator's items in the step: rebuild the pyramid above the
+    // summed leaves with them (the same centres of mass and masses)
     if (!p->dev.learned) CK(p, launch_pyramid(p->dev, (cudaStream_t)stream, true), "second moments");
-    if (p->dev.stream && !p->dev.learned) CK(p, launch_walk_items(p->dev, (cudaStream_t)stream), "work items");
+    if (!p->dev.learned && (p->stream || p->pchunk != p->chunk))
+        CK(p, launch_walk_items(pair_items(p->dev), (cudaStream_t)stream), "work items");
     CK(p, launch_learned_pairs(p->dev, theta_hi, theta_lo, max_level, item_offset, item_stride, tpi,
                                feats, targets, counter, capacity, (cudaStream_t)stream),
        "learned pairs");

@@ -132,6 +132,8 @@ struct DevPlan {
     int *qcounts;  // per box, particles in each quadrant (x half * 2 + y half); a box's particles
                    // are stored quadrant by quadrant
     int *item_cnt, *item_off, *item_group;  // force work items (group, target chunk)
+    int *pitem_cnt, *pitem_off, *pitem_group;  // the pair generator's (pair_items): the force's own
+                                               // except with FP64 pairs
     double *org;  // per system: box origins mn + k step along x (k < G), then along y, FP64
     double *mom;
     unsigned *upcnt;  // per pyramid cell above the summarize tiles (levels >= 5): children done
@@ -165,6 +167,7 @@ struct DevPlan {
     int cl_ctas;  // CTAs of a small system's tree kernel (tree_init)
     int stream;  // 1: lists are built by k_lists and streamed by k_fstream
     int chunk;   // targets per work item (TARGET_CHUNK, TARGET_CHUNK64, or STREAM_CHUNK when stream)
+    int pchunk;  // ... of the pair generator's items (TARGET_CHUNK, or STREAM_CHUNK when stream)
     // parameters
     double gconst, dt, eps2, cutoff;
     float theta2_f, eps2_f, cut_f;
@@ -417,6 +420,17 @@ __device__ __forceinline__ void raise_err(Globals *g, unsigned f) {
 
 // kernel launch wrappers (bh_tree.cu, bh_force.cu, bh_misc.cu)
 namespace bh {
+// The plan as the generator of training pairs sees it: its work items in the place of the force's.
+// FP64 forces take items of 16 targets, while the generator's item_stride and targets_per_item count
+// items of TARGET_CHUNK.  (The correction takes the force's: see launch_learned_correct.)
+inline DevPlan pair_items(const DevPlan &d) {
+    DevPlan l = d;
+    l.item_cnt = d.pitem_cnt;
+    l.item_off = d.pitem_off;
+    l.item_group = d.pitem_group;
+    l.chunk = d.pchunk;
+    return l;
+}
 cudaError_t tree_init(int *ctas);  // *ctas: the cluster's size on this device
 // create_tree of a small system (and its summarize) as one kernel
 cudaError_t launch_tree_cluster(const DevPlan &d, bool summary, cudaStream_t st);

@@ -599,6 +599,10 @@ cudaError_t learned_init() {
                                 PSmem::TOTAL + 16);
 }
 
+// The correction takes the force's items, also the small ones of an FP64 plan, which spread over the chip
+// (4,096 particles on 16 x 16 boxes, theta 0.8 corrected below 0.5, the FP64 step: 245 us against 859
+// with items of up to 512 targets; 65,536 on 128 x 128 1,743 and 1,893; 262,144 20.1 ms and 19.4: there
+// the repeated band walks cost more).
 cudaError_t launch_learned_correct(const DevPlan &d, double theta_lo, const uint8_t *img,
                                    const float *params, bool tick, cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
@@ -626,7 +630,7 @@ cudaError_t launch_learned_pairs(const DevPlan &d, double theta_hi, double theta
                                  cudaStream_t st) {
     if (d.n_total == 0) return cudaSuccess;
     k_learned_pairs<<<d.nsm * 4, LT, PSmem::TOTAL + 16, st>>>(
-        d, (float)(theta_hi * theta_hi), (float)(theta_lo * theta_lo), max_level, item_offset,
+        pair_items(d), (float)(theta_hi * theta_hi), (float)(theta_lo * theta_lo), max_level, item_offset,
         item_stride, tpi, feats, targets, counter, capacity);
     return cudaGetLastError();
 }

@@ -517,7 +517,7 @@ static cudaError_t scan_excl(const int *in, int *out, long long n, unsigned long
 
 // ---------------------------------------------------------------- work items
 // Force work items: a target group with nt targets is split into
-// ceil(nt / TARGET_CHUNK) items so that dense groups spread over many CTAs.
+// ceil(nt / chunk) items so that dense groups spread over many CTAs.
 __global__ void __launch_bounds__(TPB) k_group_items(DevPlan d) {
     step_enter();
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -1761,7 +1761,7 @@ cudaError_t launch_place(const DevPlan &d, cudaStream_t st) {
 cudaError_t launch_scan(const DevPlan &d, cudaStream_t st) {
     return scan_excl(d.qcounts, d.box_start, d.B_total, d.sst_box, d.glob, 0, st, true);
 }
-// Work items of the walk kernel and of the learned correction (group, target chunk).
+// Work items of the walk kernel and the learned correction, or of the pair generator (group, target chunk).
 cudaError_t launch_walk_items(const DevPlan &d, cudaStream_t st) {
     unsigned g = grid_for(d.NG_total, TPB, d.nsm * 8LL);
     k_group_items<<<g, TPB, 0, st>>>(d);
@@ -1772,11 +1772,13 @@ cudaError_t launch_walk_items(const DevPlan &d, cudaStream_t st) {
 }
 // The step's work items: the walk items where the walk or the learned correction runs, the
 // list-streaming items where the lists are streamed (a streaming plan builds walk items only
-// with the learned correction, or on demand for bh_learned_pairs).
+// with the learned correction, or on demand for bh_learned_pairs; so does a plan with FP64 pairs
+// the generator's).
 cudaError_t launch_items(const DevPlan &d, cudaStream_t st) {
     cudaError_t e;
     if (!d.stream || d.learned) {
         e = launch_walk_items(d, st);
+        if (e == cudaSuccess && d.learned && d.pchunk != d.chunk) e = launch_walk_items(pair_items(d), st);
         if (e != cudaSuccess) return e;
     }
     if (d.stream && d.NG_total > 0) {

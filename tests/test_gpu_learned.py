@@ -90,3 +90,42 @@ def test_learned_correction_gain():
     # (the step-time side of the comparison is the benchmark's learned Pareto)
     assert matched is not None and matched <= 0.7, (plain, el)
     assert el > e05, (e05, el)
+
+
+# A plan with FP64 pairs, whose force items are small: the generator's item_stride and targets_per_item count
+# items of up to 512 targets as in the walking FP32 plan, which has the same tree: the same rows (in any
+# order).  The correction is the FP32 plan's, read off as the difference of two accelerations some ten times
+# larger (FP32 sums of some hundred terms: 1e-4 relative RMS); and the step launches the kernels it says.
+@pytest.mark.parametrize("n,grid,group", [(700, 4, 1), (5003, 8, 2), (20011, 24, 8)])
+def test_fp64_plans_keep_the_generators_items(n, grid, group):
+    from barneshut.gb300 import learned, native, workloads
+
+    s = workloads.cluster_mixture(n, seed=n)
+    mlp = learned.LearnedCorrection(params=learned.init_params(23))
+    rows, corr = [], []
+    for prec, flags in ((native.BH_PREC_FP64, 0), (native.BH_PREC_FP32, native.BH_FLAG_WALK)):
+        acc = []
+        for flag in (0, native.BH_FLAG_LEARNED):
+            prm = native.make_params(1.0, 1e-5, 1e-4, 0.0, 0.8, group, prec, flags | flag, correction_theta=0.5)
+            plan = native.Plan([n], [grid], prm)
+            if flag:
+                plan.set_correction(mlp)
+            plan.load(*s)
+            plan.create_tree()
+            plan.summarize()
+            plan.evaluate()
+            out = plan.store()
+            acc.append(torch.stack([out["ax"], out["ay"]]).cpu().numpy())
+            f, t, c = plan.learned_pairs(0.8, 0.5, 1 << 18, item_offset=1, item_stride=3, targets_per_item=40)
+            k = int(c.item())
+            assert 0 < k < 1 << 18
+            r = torch.cat([f[:k], t[:k]], 1).cpu().numpy()
+            rows.append(r[np.lexsort(r.T)])
+            if flag:
+                plan.step_graph(1)
+                assert plan.graph_kernel_nodes() == plan.kernels_per_step()
+            assert plan.error_flags() == 0
+        corr.append(acc[1] - acc[0])
+    assert all(np.array_equal(r, rows[0]) for r in rows)
+    assert np.abs(corr[1]).max() > 0
+    assert np.sqrt(((corr[0] - corr[1]) ** 2).sum() / (corr[1] ** 2).sum()) < 1e-4
