@@ -544,9 +544,8 @@ static int enqueue_tree(bh_plan *p, bool summary, cudaStream_t st) {
     CK(p, cudaStreamWaitEvent(p->side, p->fork_ev, 0), "fork wait");
     CK(p, launch_items(p->dev, p->side), "work items");
     CK(p, cudaEventRecord(p->join_ev, p->side), "join");
-    CK(p, launch_scatter(p->dev, st), "scatter");  // (and the leaf sums)
+    CK(p, launch_scatter(p->dev, p->join_ev, st), "scatter");  // (and the leaf sums; joins)
     p->leaves_stale = false;
-    CK(p, cudaStreamWaitEvent(st, p->join_ev, 0), "join wait");
     if (summary) CK(p, launch_summarize(p->dev, false, st), "summarize");
     return BH_OK;
 }

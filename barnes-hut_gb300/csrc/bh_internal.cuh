@@ -379,7 +379,8 @@ __device__ __forceinline__ void sitem_range(int nt, int k, int *c0, int *T) {
 // 131,071 502 -> 474, four of 1,048,576 3,731 -> 3,697.  Letting the successor in earlier, when the last
 // block has started, loses: its waiting blocks take places, and the streaming force kernel, launched so,
 // was dealt unevenly to the SMs (131,071 particles 870 us; launched plainly behind kernels that do so 479).
-// A kernel that waits for another stream as well is launched plainly.
+// A kernel that a call has wait for another stream as well is launched plainly (k_gather, k_group_items and
+// k_sitems), and no tree of particles leaves its stream waiting for another: its last work is the gather.
 __device__ __forceinline__ void step_enter() { cudaGridDependencySynchronize(); }
 template <typename... P, typename... A>
 inline cudaError_t launch_step(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... a) {
@@ -440,7 +441,7 @@ cudaError_t launch_place(const DevPlan &d, cudaStream_t st);
 cudaError_t launch_scan(const DevPlan &d, cudaStream_t st);
 cudaError_t launch_items(const DevPlan &d, cudaStream_t st);
 cudaError_t launch_walk_items(const DevPlan &d, cudaStream_t st);
-cudaError_t launch_scatter(const DevPlan &d, cudaStream_t st);
+cudaError_t launch_scatter(const DevPlan &d, cudaEvent_t join, cudaStream_t st);
 cudaError_t launch_summarize(const DevPlan &d, bool leaves, cudaStream_t st);
 // the pyramid levels above the leaves and the cell records, from the leaf moments
 // second: also the second moments and their records (always with the learned correction; a plan

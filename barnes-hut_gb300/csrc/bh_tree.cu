@@ -1786,13 +1786,17 @@ cudaError_t launch_items(const DevPlan &d, cudaStream_t st) {
     }
     return cudaGetLastError();
 }
-cudaError_t launch_scatter(const DevPlan &d, cudaStream_t st) {
-    if (d.n_total == 0) return cudaSuccess;
+// The stream waits for `join` (the work items, on another stream) before the gather, so that whatever
+// follows the tree waits for one kernel; the gather itself, which waits for two, is launched plainly.
+cudaError_t launch_scatter(const DevPlan &d, cudaEvent_t join, cudaStream_t st) {
+    if (d.n_total == 0) return cudaStreamWaitEvent(st, join, 0);
     launch_step(k_perm, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
     launch_step(k_segsort, grid_for(4 * d.B_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
     launch_step(k_segsort_big, (unsigned)(d.nsm * 4), TPB, 0, st, d);
-    if (d.learned) launch_step(k_gather<true>, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
-    else launch_step(k_gather<false>, grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st, d);
+    const cudaError_t e = cudaStreamWaitEvent(st, join, 0);
+    if (e != cudaSuccess) return e;
+    if (d.learned) k_gather<true><<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
+    else k_gather<false><<<grid_for(d.n_total, TPB, d.nsm * 8LL), TPB, 0, st>>>(d);
     return cudaGetLastError();
 }
 // leaves: the leaf sums of k_gather were overwritten since (bh_set_leaf_moments): redo them
@@ -1804,8 +1808,9 @@ cudaError_t launch_summarize(const DevPlan &d, bool leaves, cudaStream_t st) {
     }
     // the second moments of the pyramid cells feed only the learned correction
     const unsigned g = grid_for(d.T_total, 1, d.nsm * 8LL);
-    if (d.learned) k_summarize<true><<<g, SUM_THREADS, 0, st>>>(d, 0);
-    else k_summarize<false><<<g, SUM_THREADS, 0, st>>>(d, 0);
+    auto k = d.learned ? k_summarize<true> : k_summarize<false>;
+    if (d.n_total > 0) launch_step(k, g, SUM_THREADS, 0, st, d, 0);
+    else k<<<g, SUM_THREADS, 0, st>>>(d, 0);  // (a tree without particles ends on the join)
     return cudaGetLastError();
 }
 cudaError_t launch_pyramid(const DevPlan &d, cudaStream_t st, bool second) {
