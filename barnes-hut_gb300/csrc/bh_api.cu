@@ -341,6 +341,25 @@ extern "C" int bh_workspace_size(const bh_plan *p, size_t *bytes) {
     return BH_OK;
 }
 
+static void fill_params(const bh_plan *p, DevPlan &d) {
+    const bh_params &pr = p->params;
+    d.stream = p->stream ? 1 : 0;
+    d.chunk = p->chunk;
+    d.pchunk = p->pchunk;
+    d.gconst = pr.grav_constant;
+    d.dt = pr.tick_seconds;
+    d.eps2 = pr.softening * pr.softening;
+    d.cutoff = pr.cutoff_r2;
+    d.theta2_f = (float)(pr.theta * pr.theta);
+    d.eps2_f = (float)d.eps2;
+    d.cut_f = (float)d.cutoff;
+    d.flat = pr.theta > 0.0 ? 0 : 1;
+    d.prec = pr.precision;
+    d.learned = (pr.flags & BH_FLAG_LEARNED) ? 1 : 0;
+    d.tune = pr.tune;
+    d.correction_theta = pr.correction_theta;
+}
+
 static void fill_dev(bh_plan *p) {
     char *w = (char *)p->ws;
     DevPlan &d = p->dev;
@@ -411,22 +430,13 @@ static void fill_dev(bh_plan *p) {
     d.item_cost = (unsigned char *)(w + p->o_icost);
     d.nsm = p->nsm;
     d.cl_ctas = p->cl_ctas;
-    d.stream = p->stream ? 1 : 0;
-    d.chunk = p->chunk;
-    d.pchunk = p->pchunk;
-    const bh_params &pr = p->params;
-    d.gconst = pr.grav_constant;
-    d.dt = pr.tick_seconds;
-    d.eps2 = pr.softening * pr.softening;
-    d.cutoff = pr.cutoff_r2;
-    d.theta2_f = (float)(pr.theta * pr.theta);
-    d.eps2_f = (float)d.eps2;
-    d.cut_f = (float)d.cutoff;
-    d.flat = pr.theta > 0.0 ? 0 : 1;
-    d.prec = pr.precision;
-    d.learned = (pr.flags & BH_FLAG_LEARNED) ? 1 : 0;
-    d.tune = pr.tune;
-    d.correction_theta = pr.correction_theta;
+    fill_params(p, d);
+}
+
+// One small system without the learned correction: its tree is one kernel's work.
+static bool cluster_tree(const bh_plan *p) {
+    return p->nsys == 1 && !(p->params.flags & BH_FLAG_LEARNED) && p->n_total > 0 && p->n_total <= CL_MAX_N &&
+           p->B_total <= CL_MAX_BOXES;
 }
 
 extern "C" int bh_bind(bh_plan *p, void *workspace, size_t bytes, void *stream) {
@@ -438,9 +448,13 @@ extern "C" int bh_bind(bh_plan *p, void *workspace, size_t bytes, void *stream) 
     CK(p, cudaGetDevice(&p->device), "cudaGetDevice");
     CK(p, cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device), "SM count");
     if (p->nsm < 1) p->nsm = 1;
-    CK(p, force_init(), "force kernel attributes");
-    CK(p, learned_init(), "learned kernel attributes");
-    CK(p, tree_init(&p->cl_ctas), "tree kernel attributes");
+    // attributes of the kernels that this plan launches, the large part of a bind's time
+    DevPlan d;
+    memset(&d, 0, sizeof(d));
+    fill_params(p, d);
+    CK(p, force_init(d), "force kernel attributes");
+    if (d.learned) CK(p, learned_init(), "learned kernel attributes");
+    if (cluster_tree(p)) CK(p, tree_init(&p->cl_ctas), "tree kernel attributes");
     if (!p->side) CK(p, cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking), "side stream");
     if (!p->fork_ev) CK(p, cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming), "fork event");
     if (!p->join_ev) CK(p, cudaEventCreateWithFlags(&p->join_ev, cudaEventDisableTiming), "join event");
@@ -520,12 +534,6 @@ extern "C" int bh_store(bh_plan *p, double *x, double *y, double *vx, double *vy
     CK(p, launch_store(p->dev, p->has_tree ? 1 : 0, p->acc_valid, nullptr, x, y, vx, vy, ax, ay, (cudaStream_t)stream),
        "store");
     return BH_OK;
-}
-
-// One small system without the learned correction: its tree is one kernel's work.
-static bool cluster_tree(const bh_plan *p) {
-    return p->nsys == 1 && !(p->params.flags & BH_FLAG_LEARNED) && p->n_total > 0 && p->n_total <= CL_MAX_N &&
-           p->B_total <= CL_MAX_BOXES;
 }
 
 // summary: the summarize phase too (launched by the caller where the tree is not one kernel's work)

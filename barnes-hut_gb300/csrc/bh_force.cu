@@ -719,39 +719,43 @@ static cudaError_t launch_force_nr(const DevPlan &d, bool accumulate, cudaStream
 // (five of the half ones): 200,000 particles on 24 x 24 boxes 917 us, with six, which spill, 1,135.
 template <bool TEST, int MINB> constexpr int HALF_MINB = TEST ? MINB + 1 : MINB;
 template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 4 : 8)>
-static cudaError_t launch_force_t(const DevPlan &d, bool accumulate, cudaStream_t st) {
-    const long long items_max = d.NG_total + d.n_total / d.chunk + 1;
-    if constexpr (sizeof(R) == 4)
-        if (2 * items_max <= (long long)d.nsm * HALF_MINB<TEST, MINB>)
-            return launch_force_nr<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>(d, accumulate, st, items_max);
-    return launch_force_nr<R, FORCE_R, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);
+struct ForceForm {  // the builds of one plan's walk
+    static cudaError_t launch(const DevPlan &d, bool accumulate, cudaStream_t st) {
+        const long long items_max = d.NG_total + d.n_total / d.chunk + 1;
+        if constexpr (sizeof(R) == 4)
+            if (2 * items_max <= (long long)d.nsm * HALF_MINB<TEST, MINB>)
+                return launch_force_nr<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>(d, accumulate, st, items_max);
+        return launch_force_nr<R, FORCE_R, KAHAN, TEST, EXACT, MINB>(d, accumulate, st, items_max);
+    }
+    static cudaError_t init() {
+        const int sm = (int)force_smem<R>();
+        if constexpr (sizeof(R) == 4) {
+            cudaError_t e = cudaFuncSetAttribute(k_force<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaFuncSetAttribute(k_force<R, FORCE_R, KAHAN, TEST, EXACT, MINB>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    }
+};
+
+// f(the plan's form)
+template <bool KAHAN, typename F> static cudaError_t with_form32(const DevPlan &d, F f) {
+    if (d.cutoff > 0.0) return f(ForceForm<float, KAHAN, true, true>());
+    if (d.eps2 == 0.0) return f(ForceForm<float, KAHAN, true, false>());
+    if (d.tune == 1) return f(ForceForm<float, KAHAN, false, false, 6>());
+    return f(ForceForm<float, KAHAN, false, false>());
+}
+template <typename F> static cudaError_t with_form(const DevPlan &d, F f) {
+    if (d.prec != 2) return d.prec == 1 ? with_form32<true>(d, f) : with_form32<false>(d, f);
+    if (d.cutoff > 0.0 || d.eps2 == 0.0) return f(ForceForm<double, false, true, false>());
+    return f(ForceForm<double, false, false, false>());
 }
 
-template <typename R, bool KAHAN, bool TEST, bool EXACT, int MINB = (sizeof(R) == 8 ? 4 : TEST ? 4 : 8)>
-static cudaError_t init_force_t() {
-    const int sm = (int)force_smem<R>();
-    cudaError_t e = cudaFuncSetAttribute(k_force<R, FORCE_R, KAHAN, TEST, EXACT, MINB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e != cudaSuccess || sizeof(R) == 8) return e;
-    return cudaFuncSetAttribute(k_force<R, 2, KAHAN, TEST, EXACT, HALF_MINB<TEST, MINB>>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-}
-
-// Raise the dynamic shared-memory limit of every instantiation once (outside
-// any stream capture).
-cudaError_t force_init() {
-    cudaError_t e;
-    if ((e = fstream_init()) != cudaSuccess) return e;
-    if ((e = init_force_t<double, false, true, false>()) != cudaSuccess) return e;
-    if ((e = init_force_t<double, false, false, false>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, true, true, true>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, true, true, false>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, true, false, false>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, false, true, true>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, false, true, false>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, true, false, false, 6>()) != cudaSuccess) return e;
-    if ((e = init_force_t<float, false, false, false, 6>()) != cudaSuccess) return e;
-    return init_force_t<float, false, false, false>();
+// Raise the dynamic shared-memory limit of the builds the plan launches (outside any stream capture).
+cudaError_t force_init(const DevPlan &d) {
+    if (d.stream) return fstream_init(d);
+    return with_form(d, [](auto form) { return form.init(); });
 }
 
 cudaError_t launch_force(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
@@ -766,22 +770,7 @@ cudaError_t launch_force(const DevPlan &d, bool tick, bool accumulate, cudaStrea
     // place while other CTAs still read them, so here the tick runs as its own kernel.
     cudaError_t e = cudaSuccess;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
-    const bool test = d.cutoff > 0.0 || d.eps2 == 0.0;
-    const bool exact = d.cutoff > 0.0;
-    if (d.prec == 2) {
-        e = test ? launch_force_t<double, false, true, false>(d, accumulate, st)
-                 : launch_force_t<double, false, false, false>(d, accumulate, st);
-    } else if (d.prec == 1) {
-        if (exact) e = launch_force_t<float, true, true, true>(d, accumulate, st);
-        else if (test) e = launch_force_t<float, true, true, false>(d, accumulate, st);
-        else if (d.tune == 1) e = launch_force_t<float, true, false, false, 6>(d, accumulate, st);
-        else e = launch_force_t<float, true, false, false>(d, accumulate, st);
-    } else {
-        if (exact) e = launch_force_t<float, false, true, true>(d, accumulate, st);
-        else if (test) e = launch_force_t<float, false, true, false>(d, accumulate, st);
-        else if (d.tune == 1) e = launch_force_t<float, false, false, false, 6>(d, accumulate, st);
-        else e = launch_force_t<float, false, false, false>(d, accumulate, st);
-    }
+    e = with_form(d, [&](auto form) { return form.launch(d, accumulate, st); });
     if (e != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;
     return tick ? launch_tick(d, st, true) : cudaSuccess;

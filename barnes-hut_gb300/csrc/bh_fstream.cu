@@ -723,12 +723,9 @@ static cudaError_t init_fstream_t() {
     return cudaFuncSetAttribute(k_fstream<KAHAN, MINB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
-cudaError_t fstream_init() {
-    cudaError_t e;
-    if ((e = init_fstream_t<true, 8>()) != cudaSuccess) return e;
-    if ((e = init_fstream_t<true, 6>()) != cudaSuccess) return e;
-    if ((e = init_fstream_t<false, 8>()) != cudaSuccess) return e;
-    return init_fstream_t<false, 6>();
+cudaError_t fstream_init(const DevPlan &d) {
+    if (d.prec == 1) return d.tune == 1 ? init_fstream_t<true, 8>() : init_fstream_t<true, 6>();
+    return d.tune == 1 ? init_fstream_t<false, 8>() : init_fstream_t<false, 6>();
 }
 
 cudaError_t launch_fstream(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,

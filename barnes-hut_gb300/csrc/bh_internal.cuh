@@ -432,7 +432,7 @@ inline DevPlan pair_items(const DevPlan &d) {
     l.chunk = d.pchunk;
     return l;
 }
-cudaError_t tree_init(int *ctas);  // *ctas: the cluster's size on this device
+cudaError_t tree_init(int *ctas);  // for k_tree_cluster; *ctas: the cluster's size on this device
 // create_tree of a small system (and its summarize) as one kernel
 cudaError_t launch_tree_cluster(const DevPlan &d, bool summary, cudaStream_t st);
 cudaError_t launch_prologue(const DevPlan &d, cudaStream_t st);
@@ -454,8 +454,8 @@ cudaError_t launch_lists(const DevPlan &d, cudaStream_t st);
 int list_kernels(long long items_max);  // kernels launch_lists launches for a plan of at most so many items
 cudaError_t launch_fstream(const DevPlan &d, bool tick, bool accumulate, cudaStream_t st,
                            const cudaEvent_t *ev = nullptr);
-cudaError_t fstream_init();
-cudaError_t force_init();
+cudaError_t fstream_init(const DevPlan &d);
+cudaError_t force_init(const DevPlan &d);
 cudaError_t launch_tick(const DevPlan &d, cudaStream_t st, bool keep_acc = false);
 cudaError_t launch_load(const DevPlan &d, const double *x, const double *y, const double *m,
                         const double *vx, const double *vy, long long rec_stride,

@@ -422,6 +422,7 @@ struct PSmem {
     static constexpr int BAND = 0;
     static constexpr int FR = BAND_CAP * 32;
     static constexpr int TOTAL = FR + 2 * FRONTIER_CAP * 4;
+    static_assert(TOTAL + 16 <= 46 * 1024, "within the limit that needs no attribute");
 };
 
 // For items item_offset + k * item_stride: band cells at levels <= max_level, up to tpi targets
@@ -518,11 +519,7 @@ __global__ void __launch_bounds__(LT) k_learned_pairs(DevPlan d, float th2_hi, f
 
 // ------------------------------------------------------------------------ launches
 cudaError_t learned_init() {
-    cudaError_t e = cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         LSmem::TOTAL);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_learned_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                PSmem::TOTAL + 16);
+    return cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize, LSmem::TOTAL);
 }
 
 // The correction takes the force's items, also the small ones of an FP64 plan, which spread over the chip
