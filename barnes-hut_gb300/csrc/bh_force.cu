@@ -1,20 +1,21 @@
-// bh_force.cu -- box-tiled force evaluation with the tick fused into its epilogue.
+// bh_force.cu -- box-tiled force evaluation by a walk of the cell pyramid per work item.
 //
 // Replaces g_evaluate_boxes (python-bh/barneshut/kernels/grid_decomposition/gpu/grid.py:116-157,
-// with d_self_self_grav / d_self_other_grav / d_self_COM_grav at :211-268) and, when the tick is
-// fused, g_tick_particles (gpu/grid.py:159-174).  The interaction semantics follow the reference
-// CPU path (kernels/grid_decomposition/sequential/evaluation.py:73-109 with
+// with d_self_self_grav / d_self_other_grav / d_self_COM_grav at :211-268); the tick
+// (g_tick_particles, gpu/grid.py:159-174) is a kernel of its own here (launch_force).  The
+// interaction semantics follow the reference CPU path
+// (kernels/grid_decomposition/sequential/evaluation.py:73-109 with
 // kernels/gravity/cpu_numba.py:30-92) in flat mode, and this project's opening-angle rule in
 // theta mode.
 //
 // Work decomposition: a target group is TG x TG leaf boxes; its nt targets are split into work
-// items of at most TARGET_CHUNK targets (built after the box scan), which CTAs pull from a device
-// queue, so dense groups spread over many SMs.  Per item the CTA walks the cell pyramid level by
-// level (every thread tests one frontier cell; accepted cells, rejected leaves and children are
-// compacted with a block scan, so list order is deterministic), stages far entries (centre of
-// mass in the group frame, mass) and near-box particles (float4 shifted into the group frame) in
-// shared memory, and evaluates them: each thread owns R targets in registers and sweeps a slice of
-// the staged entries (one shared-memory load feeds R pair interactions).  Lists that outgrow
+// items of at most TARGET_CHUNK targets (TARGET_CHUNK64 with FP64 pairs; built after the box scan),
+// which CTAs pull from a device queue, so dense groups spread over many SMs.  Per item the CTA walks
+// the cell pyramid level by level (every thread tests one frontier cell; accepted cells, rejected
+// leaves and children are compacted with a block scan, so list order is deterministic), stages far
+// entries (centre of mass in the group frame, mass) and near-box particles (shifted into the group
+// frame) in shared memory, and evaluates them: each thread owns R targets in registers and sweeps a
+// slice of the staged entries (one shared-memory load feeds R pair interactions).  Lists that outgrow
 // shared memory are evaluated and emptied on the fly; slice partials are reduced in shared memory.
 //
 // Pair arithmetic: a += m_j (x_j - x_t) * rcp(r^2 + eps^2) in FP32 (rcp.approx), far-field
@@ -54,7 +55,7 @@ template <typename R> __host__ __device__ constexpr int src_bytes() {
 // NR = 2 (launch_force).
 template <typename R, int NR, bool KAHAN, bool TEST, bool EXACT, int MINB>
 __global__ void __launch_bounds__(FT, MINB)
-k_force(DevPlan d, int tick, int accumulate) {
+k_force(DevPlan d, int accumulate) {
     step_enter();
     using S = typename Src<R>::T;
     constexpr bool F32 = sizeof(R) == 4;
@@ -672,13 +673,6 @@ k_force(DevPlan d, int tick, int accumulate) {
                 }
                 d.AX[t] = ax;
                 d.AY[t] = ay;
-                if (tick) {
-                    double vx = d.VX[nxt][t] + ax * d.dt, vy = d.VY[nxt][t] + ay * d.dt;
-                    d.VX[nxt][t] = vx;
-                    d.VY[nxt][t] = vy;
-                    d.X[nxt][t] = Xs[t] + vx * d.dt;
-                    d.Y[nxt][t] = Ys[t] + vy * d.dt;
-                }
             }
         }
         __syncthreads();  // red and s_item are reused by the next item
@@ -708,7 +702,7 @@ static cudaError_t launch_force_nr(const DevPlan &d, bool accumulate, cudaStream
     static_assert(FT * FORCE_R >= TARGET_CHUNK, "a CTA's quads must cover every target of a work item");
     auto k = k_force<R, NR, KAHAN, TEST, EXACT, MINB>;
     const long long slots = (long long)d.nsm * MINB, grid = items_max * (FORCE_R / NR);
-    launch_step(k, (unsigned)(grid < slots ? grid : slots), FT, force_smem<R>(), st, d, 0, accumulate ? 1 : 0);
+    launch_step(k, (unsigned)(grid < slots ? grid : slots), FT, force_smem<R>(), st, d, accumulate ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -766,7 +760,7 @@ cudaError_t launch_force(const DevPlan &d, bool tick, bool accumulate, cudaStrea
         if (e != cudaSuccess) return e;
         return launch_fstream(d, tick, accumulate, st, ev);
     }
-    // The walk reads source positions from the FP64 state that the fused tick would update in
+    // The walk reads source positions from the FP64 state that a fused tick would update in
     // place while other CTAs still read them, so here the tick runs as its own kernel.
     cudaError_t e = cudaSuccess;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
