@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(DT) k_direct(DevPlan d, int sys, const long lo
 #pragma unroll
             for (int r = 0; r < DR; r++) {
                 const double dx = x - xt[r], dy = y - yt[r];
-                const double w = m * rcp64(dx * dx + (dy * dy + d.eps2));
+                const double w = quot64(m, dx * dx + (dy * dy + d.eps2));
                 if (j != ti[r]) {
                     rx[r] += w * dx;
                     ry[r] += w * dy;

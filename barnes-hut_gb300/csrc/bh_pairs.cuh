@@ -17,19 +17,24 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
-// 1 / x in FP64: the hardware's approximation and one step of the cubic iteration y + y (e + e^2),
-// e = 1 - x y (Householder's method of order 2), 3 FP64 operations; the last is a fused one, so the
-// result is within rounding of the quotient.  Arguments near the ends of the exponent range, zeros,
-// infinities and NaN take the division.
-__device__ __forceinline__ double rcp64(double x) {
-    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
-    if (e - 24u > 2000u) return 1.0 / x;
+// 1 / x in FP64: the hardware's approximation (2^-20 or better) and one step of the cubic iteration y +
+// y (e + e^2), e = 1 - x y (Householder's method of order 2), 3 FP64 operations: the iteration leaves
+// 2^-60, its last operation is fused, so the result is within one unit in the last place of the rounded
+// quotient.  Arguments near the ends of the exponent range (rcp64_usual), zeros, infinities and NaN take
+// the division.
+__device__ __forceinline__ bool rcp64_usual(double x) {
+    return (((unsigned)__double2hiint(x) >> 20) & 0x7FFu) - 24u <= 2000u;
+}
+__device__ __forceinline__ double rcp64_step(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     double r = __fma_rn(-x, y, 1.0);
     r = __fma_rn(r, r, r);
     return __fma_rn(y, r, y);
 }
+__device__ __forceinline__ double rcp64(double x) { return rcp64_usual(x) ? rcp64_step(x) : 1.0 / x; }
+// m / x: outside the usual range too, where 1 / x overflows or loses bits that the quotient has
+__device__ __forceinline__ double quot64(double m, double x) { return rcp64_usual(x) ? m * rcp64_step(x) : m / x; }
 
 // Packed FP32 pairs (sm_100-family f32x2 instructions): two lanes of work per instruction.
 typedef unsigned long long f2_t;

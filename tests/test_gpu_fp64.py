@@ -165,3 +165,61 @@ def test_direct_sample_layouts(n, nt):
     assert float(err.max()) <= (8.1 + 64) * EPS
     for i in set(t.tolist()) if nt > n else ():
         assert len(np.unique(got[0, t == i])) == 1
+
+
+# The FP64 pairs' reciprocal against the division, element by element, through the sampler: a source of mass
+# m at the origin and a target at (-2^k, -y) give m / s * 2^k with s = 2^2k + y^2 (y^2 rounded, then the sum),
+# an exact multiple of the weight.  Within one unit in the last place of the rounded quotient, and equal to
+# it where the division is taken.
+def reciprocal_case(e, rng, mantissa=None):
+    """(k, y, s) of an r^2 near 2^e."""
+    y = np.ldexp(np.sqrt(rng.uniform(1.0, 4.0) if mantissa is None else mantissa), e // 2)
+    k = e // 2 - 1
+    s = np.float64(np.longdouble(np.ldexp(1.0, 2 * k)) + np.longdouble(y * y))
+    return k, y, s
+
+
+def test_reciprocal_random_mantissas():
+    from barneshut.gb300 import native
+
+    n = 40000
+    rng = np.random.default_rng(77)
+    e = rng.integers(-300, 300, n)
+    k, y, s = (np.array(v) for v in zip(*(reciprocal_case(int(v), rng) for v in e)))
+    x = -np.ldexp(1.0, k)
+    m = np.zeros(n)
+    x[0], y[0], m[0] = 0.0, 0.0, 1.0
+    plan = native.Plan([n], [4], native.make_params(1.0, 1e-5, 0.0, 0.0, 0.5))
+    plan.load(x, -y, m, np.zeros(n), np.zeros(n))
+    ax, _ = plan.direct_sample(np.arange(1, n))
+    got, want = np.ldexp(ax.cpu().numpy(), -k[1:]), 1.0 / s[1:]
+    assert np.abs((got - want) / np.spacing(want)).max() <= 1.0
+    assert (got == want).mean() > 0.9  # (half a unit and 2^-7 of one: nearly always the rounded quotient)
+
+
+def test_reciprocal_every_exponent():
+    from barneshut.gb300 import native
+
+    rng = np.random.default_rng(78)
+    cases = []
+    for e in list(range(-1074, 1024)) + 4 * [-1000, -999, -998, 1001, 1002, 1003]:
+        cases.append(reciprocal_case(e, rng) + (1.0,))
+        if not -990 < e < 990:  # a mass whose quotient is in range where the reciprocal is not
+            cases.append(reciprocal_case(e, rng) + (float(np.ldexp(rng.uniform(1.0, 2.0), np.clip(e, -1000, 1000))),))
+    cases += [(-10, 1e200, np.inf, 1.0), (0, np.inf, np.inf, 1.0), (0, np.nan, np.nan, 1.0), (0, 0.0, 1.0, np.inf)]
+    S = len(cases)
+    xy, m = np.zeros((2, 2 * S)), np.zeros(2 * S)
+    for c, (k, y, s, mass) in enumerate(cases):
+        xy[:, 2 * c + 1] = -np.ldexp(1.0, k), -y
+        m[2 * c] = mass
+    plan = native.Plan([2] * S, [1] * S, native.make_params(1.0, 1e-5, 0.0, 0.0, 0.5))
+    plan.load(xy[0], xy[1], m, np.zeros(2 * S), np.zeros(2 * S))
+    got = torch.cat([plan.direct_sample([2 * c + 1], sys=c)[0] for c in range(S)]).cpu().numpy()
+    for (k, y, s, mass), a in zip(cases, got):
+        with np.errstate(all="ignore"):
+            want = np.float64(mass) / s * np.ldexp(1.0, k)
+        usual = np.isfinite(s) and s > 0 and 24 <= np.frexp(s)[1] + 1022 <= 2024
+        if not usual or np.isinf(want):
+            assert a == want or (np.isnan(a) and np.isnan(want)), (k, y, s, mass, a, want)
+        else:
+            assert abs(a - want) <= np.spacing(abs(want)), (k, y, s, mass, a, want)
