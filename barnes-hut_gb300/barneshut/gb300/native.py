@@ -169,11 +169,15 @@ def _ptr(t):
 
 def current_stream_ptr(device):
     """The cudaStream_t (an int) of torch's current stream on a device: without the stream object,
-    whose construction costs more host time than a launch."""
+    whose construction costs more host time than a launch, where torch has the call for it (not a
+    public one)."""
     import torch
 
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream(device).cuda_stream
     i = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
+    return raw(torch.cuda.current_device() if i is None else i)
 
 
 class Plan:

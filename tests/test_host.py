@@ -81,3 +81,19 @@ def test_timer_median():
     assert Timer.medians()["evaluation"] == 2.0
     Timer.reset()
     Timer.verbose = True
+
+
+def test_current_stream_with_and_without_the_raw_call(monkeypatch):
+    import types
+
+    import torch
+
+    from barneshut.gb300 import native
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: types.SimpleNamespace(cuda_stream=("stream", d.index)))
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda i: ("raw", i), raising=False)
+    assert native.current_stream_ptr(torch.device("cuda:1")) == ("raw", 1)
+    assert native.current_stream_ptr(torch.device("cuda")) == ("raw", 3)
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    assert native.current_stream_ptr(torch.device("cuda:1")) == ("stream", 1)
