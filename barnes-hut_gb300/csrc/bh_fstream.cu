@@ -81,11 +81,11 @@ __device__ __forceinline__ void pair1(float x, float y, float m, float ntx, floa
 
 // How many of the heaviest items run as four warps' work (.x) and how many of the next as two (.y),
 // from the cost histogram (bucket b: costs in [2^b, 2^(b+1))).  A warp alone takes about 70 cycles
-// per source of a full item where a busy scheduler takes 40, so an item of more than 1/1,000 of the
-// whole cost outlasts everything else on 608 schedulers; a part of it holds half or a quarter of the
-// targets of every quad, with the same slices and order of sources (the same bits), and sweeps with
-// that much less work and more sources in flight.  The parts repeat the item's staging, so items
-// below the line stay whole.
+// per source of a full item where a busy scheduler takes 40, so an item of about a thousandth of the
+// whole cost outlasts everything else on 608 schedulers: items above 1 / SPLIT2 of it are halved, above
+// 1 / SPLIT4 quartered.  A part holds half or a quarter of the targets of every quad, with the same slices
+// and order of sources (the same bits), and sweeps with that much less work and more sources in flight.
+// The parts repeat the item's staging, so items below the line stay whole.
 __device__ __forceinline__ int2 stream_split(const int *hist) {
     const int lane = threadIdx.x & 31;
     const int h = hist[lane];  // ITEM_BUCKETS == 32

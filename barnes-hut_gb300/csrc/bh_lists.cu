@@ -25,7 +25,7 @@
 namespace bh {
 
 constexpr int LW = 4;  // warps per list-building CTA; one warp walks one group
-// CTAs per SM (64 registers): the walk is bound by its instructions and their latency together.  1,048,576
+// CTAs per SM (56 registers): the walk is bound by its instructions and their latency together.  1,048,576
 // particles, four steps: 3,773 us with twelve (40 registers, which spill), 3,749 with ten, 3,717 with eight
 constexpr int LISTS_MINB = 8;
 

@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(TPB) k_gather(DevPlan d) {
     const int lane = threadIdx.x & 31;
     // SU particles per thread per round, each stage's loads issued for all of them before the
     // next stage uses them; the loop runs per warp (its first lane's index), for the scans.
-    // Two per round keep the kernel at 58 registers, 4 CTAs per SM (four: 93, 2 CTAs, 9% slower)
+    // Two per round keep the kernel at 64 registers, 4 CTAs per SM (four: 93, 2 CTAs, 9% slower)
     constexpr int SU = 2;
     const long long n = d.n_total, stride = (long long)gridDim.x * blockDim.x;
     // one system (the common case): its grid constants once, no search per particle

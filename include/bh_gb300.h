@@ -79,9 +79,12 @@ typedef struct bh_params {
     int precision;        /* BH_PREC_* */
     int flags;            /* BH_FLAG_* */
     int tune;             /* force-kernel build, picked by the autotuner: 0 the path's
-                             default (list streaming: 6 CTAs per SM, 80 registers; walk:
-                             8 CTAs per SM), 1 the other (list streaming: 8 CTAs per SM,
-                             64 registers; walk: 6 CTAs per SM) */
+                             default (list streaming: 80 registers, up to 6 CTAs per SM;
+                             walk: 64 registers, 8 CTAs per SM), 1 the other (list
+                             streaming: 64 registers, up to 8 CTAs per SM; walk: 80
+                             registers, 6 CTAs per SM).  Streaming plans of few items run
+                             2 to 5 CTAs per SM with either; the walk with a cutoff or
+                             without softening (4 or 5) and FP64 pairs (4) have one build. */
     double correction_theta; /* with BH_FLAG_LEARNED: cells accepted at theta but
                                 not at correction_theta get the learned correction */
     int dense_min;        /* list streaming: boxes with at least this many particles get

@@ -28,7 +28,7 @@ def network_rows(n, seed, width=8):
 
 
 # Forward: BF16 operands at the oracle's rounding points, so 2e-2 as in the network's own tests.
-# 152 SMs x 4 CTAs x 2 tiles of 128 rows in flight: 155,649 rows leave a second round of one row.
+# 152 SMs x 8 tiles of 128 rows in flight: 155,649 rows leave a second round of one row.
 @pytest.mark.parametrize("n,width", [(1, 6), (127, 7), (128, 8), (129, 9), (257, 12), (155649, 6)])
 def test_network_forward_rows_and_strides(n, width):
     from barneshut.gb300.learned import LearnedCorrection
@@ -353,8 +353,8 @@ def test_adam_with_images_is_adam_then_pack():
     assert torch.allclose(a.grad, b.grad, rtol=1e-4, atol=1e-6)  # (FP32 additions in another order)
 
 
-# Long direct sums in split floats, with what they leave to FP64: coincident and very close pairs, a
-# system whose masses leave the floats' range, one far from the origin; and a target of another system.
+# Long direct sums: coincident and very close pairs, one mass far above the others, a system far from the
+# origin; and a target of another system.
 @pytest.mark.parametrize("kind", ["plain", "close", "heavy", "offset"])
 @pytest.mark.parametrize("eps", [0.0, 1e-3])
 def test_direct_sample_long_sums(kind, eps):
@@ -387,9 +387,8 @@ def test_direct_sample_long_sums(kind, eps):
         assert np.linalg.norm(got[:, k] - ref) <= 1e-12 * np.linalg.norm(ref)
 
 
-# FP64 forces whose near pairs run in split floats (from 8,192 particles on), every pair near: close and
-# coincident pairs, pairs at the cutoff, a mass out of the floats' range, a system far off, another in
-# the batch.  FP64 sums of 8,000 terms: 1e-12.
+# FP64 forces with every pair near (8,200 particles): close and coincident pairs, pairs at the cutoff, a mass
+# far above the others, a system far off, another in the batch.  FP64 sums of 8,000 terms: 1e-12.
 @pytest.mark.parametrize("kind", ["plain", "close", "cutoff", "heavy", "offset"])
 @pytest.mark.parametrize("theta,eps,cutoff", [(0.0, 0.0, 1e-5), (0.0, 0.0, 0.0), (0.5, 1e-3, 0.0), (0.0, 1e-2, 1e-4)])
 def test_fp64_forces_in_split_floats(kind, theta, eps, cutoff):
