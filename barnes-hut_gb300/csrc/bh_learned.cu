@@ -244,19 +244,17 @@ struct LSmem {
     static constexpr int TPOS = BAND + BAND_CAP * 32;  // LTMAX float2
     static constexpr int CORR = TPOS + LTMAX * 8;    // LTMAX float2
     static constexpr int BIAS = CORR + LTMAX * 8;    // 208 floats
-    static constexpr int OUT = BIAS + 208 * 4;       // per group: 128 float2
-    static constexpr int TOTAL = OUT + LG * 1024;
+    static constexpr int TOTAL = BIAS + 208 * 4;
     static_assert(LC_CTAS * (TOTAL + 1280) <= 228 * 1024, "LC_CTAS must fit in the SM's shared memory");
     static_assert(LC_CTAS * 256 <= 512 && LG * 64 <= 256, "and in its tensor memory");
 };
 
 // One work item per CTA at a time: the band walk, then its (target, band cell) pairs in tiles of
-// 128, a group of 128 threads per tile.  Bound like the network's forward pass (mlp_group_forward).
-// The pairs run cell by cell, so a warp's lanes read few cells' records at a time, and a thread per
-// target adds the target's outputs in the order of its cells, the groups' sums then in their order: the
-// same sums in every run.  262,144 clustered particles, 128 x 128 boxes, theta 0.8 corrected below 0.5,
-// the step: 1,495 us, with shared-memory FP32 atomics, whose order changes from run to run, 1,460;
-// 4,096 on 16 x 16 164 us, in CTAs of one tile at a time 235.
+// 128, a group of 128 threads per tile.  Bound like the network's forward pass (mlp_group_forward);
+// the pairs are laid out cell by cell, so a warp's lanes read one cell's record at a time and add
+// their outputs to 32 different targets.  262,144 clustered particles, 128 x 128 boxes, theta 0.8
+// corrected below 0.5: 3,895 us -> 1,230 us (1,678 with single bf16 conversions; before: 8 warps per
+// SM in target-major order, whose shared-memory FP32 atomics met on one target).
 __global__ void __launch_bounds__(128 * LG, LC_CTAS)
 k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *params, int tick) {
     constexpr int NT = 128 * LG;
@@ -271,7 +269,6 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
     float *bias = reinterpret_cast<float *>(sm + LSmem::BIAS);
     const int tid = threadIdx.x, grp = tid >> 7, r = tid & 127;
     uint8_t *ACT = sm + LSmem::ACT + 16384 * grp;
-    float2 *out0 = reinterpret_cast<float2 *>(sm + LSmem::OUT), *out = out0 + 128 * grp;  // a tile's outputs
     copy_bytes(sm + LSmem::W, img, I_FWD);
     for (int i = tid; i < 64; i += NT) {
         bias[i] = params[P_B1 + i];
@@ -324,14 +321,9 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
             corr[v] = make_float2(0.f, 0.f);
         }
         __syncthreads();
-        // up to 128 targets: the tiles go round the groups, each with sums of its own; more: a group has a
-        // third of the targets and all of their tiles to itself
-        const bool shared = ig.T <= 128;
-        const unsigned t0 = shared ? 0u : ig.T * grp / LG, T = shared ? (unsigned)ig.T : ig.T * (grp + 1) / LG - t0;
-        const unsigned npairs = T * (unsigned)nb;  // (at most LTMAX x BAND_CAP)
-        if (tid == 0) atomicAdd(&d.glob->corr_pairs, (unsigned long long)ig.T * nb);
-        float2 sum = make_float2(0.f, 0.f);  // of target t0 + r (T <= 128)
-        for (unsigned p0 = shared ? 128u * grp : 0u; p0 < npairs; p0 += shared ? NT : 128) {
+        const unsigned T = (unsigned)ig.T, npairs = T * (unsigned)nb;  // (at most LTMAX x BAND_CAP)
+        if (tid == 0) atomicAdd(&d.glob->corr_pairs, (unsigned long long)npairs);
+        for (unsigned p0 = 128u * grp; p0 < npairs; p0 += NT) {
             const unsigned p = p0 + r;
             float f[16];
 #pragma unroll
@@ -339,63 +331,23 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
             unsigned t = 0, k = 0;
             if (p < npairs) {
                 k = p / T;
-                t = t0 + p - k * T;
+                t = p - k * T;
                 band_features(band[k], band[k].s, tpos[t].x, tpos[t].y, f);
             }
             store_row16(ACT, r, f);
             float y[2];
             if (!mlp_group_forward(sW, ACT, bias, tmem, &mbars[grp], phase, 1 + grp, ok, y)) break;
-            const float scale = p < npairs ? band[k].M : 0.f;
-            if (T < 128) {
-                out[r] = make_float2(scale * y[0], scale * y[1]);
-                group_sync(1 + grp, 128);
-                if (r < T) {
-                    // the tile's pairs of target t0 + r, one cell after another (the next tile's outputs come
-                    // after the barriers of its forward pass)
-                    const unsigned off = p0 % T, n = min(128u, npairs - p0);
-                    for (unsigned j = r >= off ? r - off : r + T - off; j < n; j += 4 * T) {
-                        float2 v[4];
-#pragma unroll
-                        for (int u = 0; u < 4; u++) v[u] = j + u * T < n ? out[j + u * T] : make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            sum.x += v[u].x;
-                            sum.y += v[u].y;
-                        }
-                    }
-                }
-            } else if (p < npairs) {  // one pair a target in a tile
-                if (T == 128) {
-                    sum.x += scale * y[0];
-                    sum.y += scale * y[1];
-                } else {
-                    corr[t].x += scale * y[0];
-                    corr[t].y += scale * y[1];
-                }
-            }
-        }
-        if (T <= 128) {
-            if (shared) {
-                group_sync(1 + grp, 128);  // (the last tile's outputs have been added)
-                out[r] = sum;
-            } else if (r < T) {
-                corr[t0 + r] = sum;
+            if (p < npairs && ok) {
+                const float scale = band[k].M;
+                atomicAdd(&corr[t].x, scale * y[0]);
+                atomicAdd(&corr[t].y, scale * y[1]);
             }
         }
         if (!__syncthreads_and(ok ? 1 : 0)) break;
         for (int v = tid; v < ig.T; v += NT) {
             int ti = item_target(ig, s_col0, s_colpre, v);
-            float2 c = corr[v];
-            if (shared) {
-                c = out0[v];
-#pragma unroll
-                for (int g = 1; g < LG; g++) {
-                    c.x += out0[128 * g + v].x;
-                    c.y += out0[128 * g + v].y;
-                }
-            }
-            const double ax = d.AX[ti] + d.gconst * (double)c.x;
-            const double ay = d.AY[ti] + d.gconst * (double)c.y;
+            double ax = d.AX[ti] + d.gconst * (double)corr[v].x;
+            double ay = d.AY[ti] + d.gconst * (double)corr[v].y;
             d.AX[ti] = ax;
             d.AY[ti] = ay;
             if (tick) {
@@ -415,6 +367,125 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
     tc::fence_before();
     __syncthreads();
     if (tid < 32) tc::tmem_dealloc(tslot, 256);
+}
+
+// The same for a plan of few items: a CTA of 128 threads, one tile at a time in target-major order.
+// With an SM to itself a CTA meets the additions to a target's sums in the same order in every run,
+// so a small system's step is the same bits each time, which the tiles in flight of the form above
+// give up (launch_learned_correct).
+struct LSmemFew {
+    static constexpr int W = 0;                      // forward images
+    static constexpr int A0 = I_FWD;                 // 128 x 16 BF16
+    static constexpr int ACT = A0 + 4096;            // 128 x 64 BF16
+    static constexpr int BAND = ACT + 16384;         // BAND_CAP x 32 B
+    static constexpr int TPOS = BAND + BAND_CAP * 32;  // LTMAX float2
+    static constexpr int CORR = TPOS + LTMAX * 8;    // LTMAX float2
+    static constexpr int FR = CORR + LTMAX * 8;      // 2 x FRONTIER_CAP int
+    static constexpr int BIAS = FR + 2 * FRONTIER_CAP * 4;  // 208 floats
+    static constexpr int TOTAL = BIAS + 208 * 4;
+};
+
+__global__ void __launch_bounds__(LT) k_learned_correct_few(DevPlan d, float th2_lo, const uint8_t *img,
+                                                        const float *params, int tick) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    __shared__ uint64_t mbar;
+    __shared__ uint32_t tslot;
+    __shared__ int sh_scan[32], s_item, s_col0[9], s_colpre[9];
+    BandCell *band = reinterpret_cast<BandCell *>(sm + LSmemFew::BAND);
+    float2 *tpos = reinterpret_cast<float2 *>(sm + LSmemFew::TPOS);
+    float2 *corr = reinterpret_cast<float2 *>(sm + LSmemFew::CORR);
+    int *fr0 = reinterpret_cast<int *>(sm + LSmemFew::FR), *fr1 = fr0 + FRONTIER_CAP;
+    float *bias = reinterpret_cast<float *>(sm + LSmemFew::BIAS);
+    const int tid = threadIdx.x;
+    copy_bytes(sm + LSmemFew::W, img, I_FWD);
+    for (int i = tid; i < 64; i += LT) {
+        bias[i] = params[P_B1 + i];
+        bias[64 + i] = params[P_B2 + i];
+        bias[128 + i] = params[P_B3 + i];
+    }
+    if (tid < 16) bias[192 + tid] = params[P_B4 + tid];
+    if (tid < 32) {
+        tc::tmem_alloc(&tslot, 64);
+        tc::tmem_relinquish();
+    }
+    if (tid == 0) {
+        tc::mbar_init(&mbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = tslot, sW = tc::smem_u32(sm + LSmemFew::W), sA0 = tc::smem_u32(sm + LSmemFew::A0);
+    uint32_t phase = 0;
+    bool ok = true;
+    const int nxt = (d.glob->epoch + 1) & 1;
+    const long long nitems = d.item_off[d.NG_total];
+    for (;;) {
+        if (tid == 0) s_item = (int)atomicAdd(&d.glob->item_next2, 1u);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= nitems || !ok) break;
+        const long long g = d.item_group[item];
+        ItemGeom ig;
+        item_geom(d, g, item - d.item_off[g], s_col0, s_colpre, ig);
+        const SysDyn &dy = d.dyn[ig.s];
+        const float step_f = __double2float_rn(dy.step);
+        bool of;
+        const int nb = band_walk<LT>(d, ig, d.theta2_f, th2_lo, 64, band, fr0, fr1, sh_scan, &of);
+        if (of && tid == 0) raise_err(d.glob, 2u /*BH_DEV_LIST_OVERFLOW*/);
+        for (int v = tid; v < ig.T; v += LT) {
+            int ti = item_target(ig, s_col0, s_colpre, v);
+            const float4 p = d.PD[2 * (long long)ti];  // (x, x, y, y) box-relative
+            int lb = d.skey[ti] - (int)d.sys[ig.s].boff;
+            int kx = lb / ig.G, ky = lb - kx * ig.G;
+            tpos[v] = make_float2(__fadd_rn(__fmul_rn((float)(kx - ig.gx0), step_f), p.x),
+                                  __fadd_rn(__fmul_rn((float)(ky - ig.gy0), step_f), p.z));
+            corr[v] = make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+        const long long npairs = (long long)ig.T * nb;
+        if (tid == 0) atomicAdd(&d.glob->corr_pairs, (unsigned long long)npairs);
+        for (long long p0 = 0; p0 < npairs && ok; p0 += 128) {
+            const long long p = p0 + tid;
+            float f[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) f[k] = 0.f;
+            int t = 0, k = 0;
+            if (p < npairs) {
+                t = (int)(p / nb);
+                k = (int)(p - (long long)t * nb);
+                band_features(band[k], 1.f / band[k].s, tpos[t].x, tpos[t].y, f);
+            }
+            store_row16(sm + LSmemFew::A0, tid, f);
+            float y[2];
+            ok = mlp_tile_forward(sW, sA0, sm + LSmemFew::ACT, bias, tmem, &mbar, phase, y);
+            if (ok && p < npairs) {
+                float scale = band[k].M / band[k].s;
+                atomicAdd(&corr[t].x, scale * y[0]);
+                atomicAdd(&corr[t].y, scale * y[1]);
+            }
+        }
+        __syncthreads();
+        for (int v = tid; v < ig.T && ok; v += LT) {
+            int ti = item_target(ig, s_col0, s_colpre, v);
+            double ax = d.AX[ti] + d.gconst * (double)corr[v].x;
+            double ay = d.AY[ti] + d.gconst * (double)corr[v].y;
+            d.AX[ti] = ax;
+            d.AY[ti] = ay;
+            if (tick) {
+                double vx = d.VX[nxt][ti] + ax * d.dt, vy = d.VY[nxt][ti] + ay * d.dt;
+                d.VX[nxt][ti] = vx;
+                d.VY[nxt][ti] = vy;
+                d.X[nxt][ti] = d.X[nxt][ti] + vx * d.dt;
+                d.Y[nxt][ti] = d.Y[nxt][ti] + vy * d.dt;
+            }
+        }
+        __syncthreads();
+    }
+    if (!ok && tid == 0) raise_err(d.glob, 8u /*BH_DEV_WAIT_TIMEOUT*/);
+    tc::fence_before();
+    __syncthreads();
+    if (tid < 32) tc::tmem_dealloc(tmem, 64);
 }
 
 // ------------------------------------------------------------------- training pairs
@@ -519,7 +590,11 @@ __global__ void __launch_bounds__(LT) k_learned_pairs(DevPlan d, float th2_hi, f
 
 // ------------------------------------------------------------------------ launches
 cudaError_t learned_init() {
-    return cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize, LSmem::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         LSmem::TOTAL);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_learned_correct_few, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                LSmemFew::TOTAL + 1024);
 }
 
 // The correction takes the force's items, also the small ones of an FP64 plan, which spread over the chip
@@ -533,9 +608,17 @@ cudaError_t launch_learned_correct(const DevPlan &d, double theta_lo, const uint
     if (e != cudaSuccess) return e;
     long long items_max = d.NG_total + d.n_total / d.chunk + 1;
     long long grid = (long long)d.nsm * LC_CTAS;
+    // up to two rounds of items over the chip: the reproducible form (4,096 particles, theta 0.8: 401
+    // us a step, bit for bit the same each time); beyond that CTAs share SMs and no form keeps its
+    // order (40,000 particles, theta 0.6: 450 -> 399 us)
+    const bool few = items_max <= 2 * grid;
     if (grid > items_max) grid = items_max;
-    k_learned_correct<<<(unsigned)grid, 128 * LG, LSmem::TOTAL, st>>>(d, (float)(theta_lo * theta_lo), img, params,
-                                                                    tick ? 1 : 0);
+    if (few)
+        k_learned_correct_few<<<(unsigned)grid, LT, LSmemFew::TOTAL + 1024, st>>>(
+            d, (float)(theta_lo * theta_lo), img, params, tick ? 1 : 0);
+    else
+        k_learned_correct<<<(unsigned)grid, 128 * LG, LSmem::TOTAL, st>>>(
+            d, (float)(theta_lo * theta_lo), img, params, tick ? 1 : 0);
     return cudaGetLastError();
 }
 

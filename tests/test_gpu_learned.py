@@ -129,29 +129,3 @@ def test_fp64_plans_keep_the_generators_items(n, grid, group):
     assert all(np.array_equal(r, rows[0]) for r in rows)
     assert np.abs(corr[1]).max() > 0
     assert np.sqrt(((corr[0] - corr[1]) ** 2).sum() / (corr[1] ** 2).sum()) < 1e-4
-
-
-# The correction's sums are added in the order of the cells, by one thread per target: the same bits in every
-# run, with items below and above 128 targets a group of threads, on plans from less than a CTA per SM to
-# several rounds (and on two of one group, which have no cells in the band).
-@pytest.mark.parametrize("n,grid,group,walk,band", [(300, 4, 1, 0, True), (4096, 16, 0, 1, True), (6000, 4, 4, 1, False),
-                                                    (10000, 25, 0, 0, True), (20011, 8, 8, 1, False), (30011, 16, 2, 1, True),
-                                                    (60000, 61, 0, 0, True)])
-def test_learned_steps_repeat_bit_for_bit(n, grid, group, walk, band):
-    from barneshut.gb300 import learned, native, workloads
-
-    s = workloads.cluster_mixture(n, seed=n)
-    mlp = learned.LearnedCorrection(params=learned.init_params(23))
-    prm = native.make_params(1.0, 1e-5, 1e-4, 0.0, 0.8, group, native.BH_PREC_FP32_KAHAN,
-                             native.BH_FLAG_LEARNED | walk * native.BH_FLAG_WALK, correction_theta=0.5)
-    plan = native.Plan([n], [grid], prm)
-    plan.set_correction(mlp)
-    first = None
-    for _ in range(20):
-        plan.load(*s)
-        plan.step(1)
-        out = plan.store()
-        acc = torch.stack([out["ax"], out["ay"]])
-        first = acc if first is None else first
-        assert torch.equal(acc, first)
-    assert (plan.corrected_pairs() > 0) == band and plan.error_flags() == 0
