@@ -369,10 +369,10 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
     if (tid < 32) tc::tmem_dealloc(tslot, 256);
 }
 
-// The same for a plan of few items: a CTA of 128 threads, one tile at a time in target-major order.
-// With an SM to itself a CTA meets the additions to a target's sums in the same order in every run,
-// so a small system's step is the same bits each time, which the tiles in flight of the form above
-// give up (launch_learned_correct).
+// The same for a plan of few items: a CTA of 128 threads, one tile at a time in target-major order, so
+// that a target's sum meets its terms nearly in the order of its cells.  No order is guaranteed (FP32
+// shared-memory atomics from up to four warps): twenty steps of a system of 300 to 6,000 particles were
+// mostly the same bits, of 10,000 and more nearly never (1e-9 to 2e-8 of an acceleration apart).
 struct LSmemFew {
     static constexpr int W = 0;                      // forward images
     static constexpr int A0 = I_FWD;                 // 128 x 16 BF16
@@ -608,9 +608,11 @@ cudaError_t launch_learned_correct(const DevPlan &d, double theta_lo, const uint
     if (e != cudaSuccess) return e;
     long long items_max = d.NG_total + d.n_total / d.chunk + 1;
     long long grid = (long long)d.nsm * LC_CTAS;
-    // up to two rounds of items over the chip: the reproducible form (4,096 particles, theta 0.8: 401
-    // us a step, bit for bit the same each time); beyond that CTAs share SMs and no form keeps its
-    // order (40,000 particles, theta 0.6: 450 -> 399 us)
+    // Up to two rounds of items over the chip the tile-at-a-time form stays, for its results: three tiles in
+    // flight add in another order, 1e-9 to 3e-8 of an acceleration away, where this form's runs agree (up to
+    // some 150 items) or are 1e-8 apart themselves (beyond).  It is the slower one: 4,096 particles on 16 x
+    // 16 boxes, theta 0.8, a step 314 us against 159, 20,000 on 35 x 35 504 against 251; above the line,
+    // 40,000 on 50 x 50, theta 0.6, 319 against 273, 262,144 on 128 x 128, theta 0.8, 2,430 against 1,460.
     const bool few = items_max <= 2 * grid;
     if (grid > items_max) grid = items_max;
     if (few)

@@ -206,9 +206,9 @@ __device__ __forceinline__ bool mma_round(uint64_t *mbar, uint32_t &phase, F iss
 }
 
 // Forward of one 128-row tile by a CTA of 128 threads, whose input rows are already in A0 (K-major
-// 128 x 16): the tile-at-a-time form for a few items (k_learned_correct_few).  Thread t owns row t and receives the two outputs in y[0..1].  W = forward images in shared
-// memory, bias = 208 floats (b1, b2, b3, b4) in shared memory, ACT = 128 x 64 scratch tile,
-// tmem = 64 allocated columns.  Returns false if a tensor-core wait timed out.
+// 128 x 16): the tile-at-a-time form for a few items (k_learned_correct_few).  Thread t owns row t and
+// receives the two outputs in y[0..1].  W = forward images in shared memory, bias = 208 floats (b1, b2,
+// b3, b4) in shared memory, ACT = 128 x 64 scratch tile, tmem = 64 allocated columns.  Returns false if a tensor-core wait timed out.
 __device__ __forceinline__ bool mlp_tile_forward(uint32_t sW, uint32_t sA0, uint8_t *ACT,
                                                  const float *bias, uint32_t tmem, uint64_t *mbar,
                                                  uint32_t &phase, float *y) {
