@@ -226,7 +226,7 @@ k_force(DevPlan d, int accumulate) {
             if (active && F32) {
                 const ulonglong2 *fp = reinterpret_cast<const ulonglong2 *>(far);
                 const f2_t *fm = reinterpret_cast<const f2_t *>(farm);
-#pragma unroll 2
+#pragma unroll 4
                 for (int k = slice; k < nf; k += nslice) {
                     const ulonglong2 rxy = fp[k];  // (rx, rx), (ry, ry)
                     const f2_t mm = fm[k];         // (M, M)
@@ -451,7 +451,7 @@ k_force(DevPlan d, int accumulate) {
 #pragma unroll 1
                         for (; j < ns; j += nslice) sweep1(j);
                     } else {
-#pragma unroll 16 / NR
+#pragma unroll 8 / NR
                         for (int j = slice; j < ns; j += nslice) sweep1(j);
                     }
                 } else if (active) {
@@ -655,11 +655,15 @@ k_force(DevPlan d, int accumulate) {
             }
         }
         __syncthreads();
+        // (the sweeps' and this loop's unrolling: 100,003 particles on 12 x 12 boxes, no cutoff, the round 384 us,
+        // with far entries by two and near ones by sixteen 397; 200,000 on 24 x 24 with the cutoff 593, with
+        // four targets here at once 601)
         if (active && slice == 0) {
-#pragma unroll
+#pragma unroll NR == 4 && EXACT ? 1 : NR
             for (int r = 0; r < NR; r++) {
                 if (!tv[r]) continue;
                 R sx = 0, sy = 0;
+#pragma unroll 4
                 for (int k = 0; k < nslice; k++) {
                     const R *o = red + 2 * ((k * nthr + tl) * NR + r);
                     sx += o[0];
