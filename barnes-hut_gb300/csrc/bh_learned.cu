@@ -371,7 +371,7 @@ k_learned_correct(DevPlan d, float th2_lo, const uint8_t *img, const float *para
 
 // The same for a plan of few items: a CTA of 128 threads, one tile at a time in target-major order, so
 // that a target's sum meets its terms nearly in the order of its cells.  No order is guaranteed (FP32
-// shared-memory atomics from up to four warps): twenty steps of a system of 300 to 6,000 particles were
+// shared-memory atomics from up to four warps): forty steps of a system of 300 to 6,000 particles were
 // mostly the same bits, of 10,000 and more nearly never (1e-9 to 2e-8 of an acceleration apart).
 struct LSmemFew {
     static constexpr int W = 0;                      // forward images
